@@ -674,7 +674,7 @@ __device__ __forceinline__ void issue_tile(R* B0, const CUtensorMap* tm_phi, con
 template <int NT>
 struct StageShared {
   double red[NT / 32];
-  double sh_s[NT], sh_c[NT];
+  double sh_s[NT / 32], sh_c[NT / 32];
   uint64_t bar;
   int am_last;
 };
@@ -916,7 +916,7 @@ __global__ void __launch_bounds__(NT, (pipe_ctas<TH, MODE>())) flow_kernel_pipe(
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* ring = reinterpret_cast<R*>(smem_raw);
   __shared__ double red[NT / 32];
-  __shared__ double sh_s[NT], sh_c[NT];
+  __shared__ double sh_s[NT / 32], sh_c[NT / 32];
   __shared__ int am_last;
   __shared__ int timed_out;
   __shared__ __align__(8) uint64_t full[STAGES];
@@ -1122,7 +1122,7 @@ __global__ void __launch_bounds__(NT)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* tile = reinterpret_cast<R*>(smem_raw);
   __shared__ double red[NT / 32];
-  __shared__ double sh_s[NT], sh_c[NT];
+  __shared__ double sh_s[NT / 32], sh_c[NT / 32];
   __shared__ int am_last;
   const int tiles_y = (G.Y + TY - 1) / TY;
   const int x0 = (blockIdx.x / tiles_y) * TX;
