@@ -37,10 +37,9 @@ XLEN = YLEN = 4096
 XSIZE = 128.0
 METRIC = "Mpoint-updates/s per flow step at dE/E<=1e-6 vs plain FP64; achieved HBM GB/s"
 UNIT = "Mpoint-updates/s"
-# words of nf components moved per site and step: S1 2 (phi in, l1 out), S2 3, S3 7
-# (phi, V, l1, l2 in; T4, cV, cP out), S4 5 (T4, cP, cV in; phi', V' out) as four
-# kernels; S1 2, S2+S3 fused 6, S4 5 when stages 2 and 3 run as one kernel
-WORDS_SEPARATE, WORDS_FUSED = 17, 13
+# words of nf components moved per site and step: phase A 4 (phi, V in; l1, l2 out), phase B 6
+# (phi, V, l1, l2 in; phi', V' out)
+WORDS = 10
 # end to end: one host->device load of the field and velocity, E2E_CALLS one-step
 # Simulation.step calls (each returns E and err to the host), one device->host read-back
 E2E_CALLS = 100
@@ -321,10 +320,10 @@ def gpu_arm(args, rank, world, local_rank):
     ms = max_over_ranks(ev0.elapsed_time(ev1))
     ms_step = ms / K
     value = world * N * K / (ms / 1e3) / 1e6
-    # stage launches per step, then the call's trailing energy pass and finish kernel
-    launches = (3 if (s.tma_enabled and s._lib.ss_get_variant(s._h, 6) == 1) else 4) * K + 2
+    # two launches per step, then the call's trailing energy pass and finish kernel
+    launches = 2 * K + 2
 
-    # roofline of the stage kernels (3 launches per step with stages 2 and 3 fused, else 4)
+    # roofline of the step's two phase kernels
     from soliton_solver_b200._native import load as _load  # noqa: F401 (library loaded)
     peaks = {}
     try:
@@ -333,9 +332,7 @@ def gpu_arm(args, rank, world, local_rank):
         pass
     peak = float(peaks.get("hbm_gbs", 6650.0))
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
-    fused = s.tma_enabled and s._lib.ss_get_variant(s._h, 6) == 1
-    words = WORDS_FUSED if fused else WORDS_SEPARATE
-    bytes_step = words * 4 * 4 * N
+    bytes_step = WORDS * 4 * 4 * N
     achieved = bytes_step / (ms_step / 1e3) / 1e9
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "flow_kernel_traffic.json")
@@ -384,9 +381,8 @@ def gpu_arm(args, rank, world, local_rank):
                                   "global_sites": world * N}),
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
-                             "kernel": "flow_kernel<ChiralMagnet,float> stage launches (S1, S2+S3 fused, S4)"
-                                       if fused else "flow_kernel<ChiralMagnet,float> (4 stage launches per step)",
-                             "launches_per_step": 3 if fused else 4,
+                             "kernel": "step_kernel<ChiralMagnet,float> phases A (l1, l2) and B (l3, l4, update)",
+                             "launches_per_step": 2,
                              "algorithmic_bytes_per_step": bytes_step},
                 "cpu_baseline": cpu, "cpu_baseline_port": cpu_port,
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
@@ -394,10 +390,9 @@ def gpu_arm(args, rank, world, local_rank):
                         "note": f"pinned host field+velocity in once, {Ke} one-step calls each returning (E, err), "
                                 "field out once; wall clock, max over ranks"},
                 "gpu_launches": launches, "clocks": clk.summary(),
-                "autotune": {**{f"S{m}": {"tile_per_cta_ms": a, "pipelined_ms": b, "chosen": "pipelined" if c else
-                                          "tile_per_cta"} for m, (a, b, c) in tuning.items() if m != 6},
-                             "S2+S3": {"two_kernels_ms": tuning[6][0], "fused_ms": tuning[6][1],
-                                       "chosen": "fused" if tuning[6][2] else "two kernels"}}}
+                "autotune": {"A": {"tile_per_cta_ms": tuning[1][0]},
+                             "B": {"tile_per_cta_ms": tuning[4][0], "pipelined_ms": tuning[4][1],
+                                   "chosen": "pipelined" if tuning[4][2] else "tile_per_cta"}}}
         line.update(extra)
         print(json.dumps(line), flush=True)
     return 0
@@ -619,10 +614,10 @@ def batched_sweep(dev, steps=20, seed=4, reps=3):
     Eg, _ = b.trajectory()
     peak = float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))).get("hbm_gbs", 6650.0)) \
         if os.path.exists(os.path.join(ROOT, "MEASURED_PEAKS.json")) else 6650.0
-    gbs = sites * WORDS_FUSED * 3 * 4 / (ms / 1e3) / 1e9
+    gbs = sites * WORDS * 3 * 4 / (ms / 1e3) / 1e9
     return {"lattices": 256, "sites": sites, "steps_per_graph": steps, "replays": reps,
             "value": sites / (ms / 1e3) / 1e6, "unit": UNIT, "ms_per_step": ms,
-            "achieved_gbs": gbs, "frac_of_measured_hbm": gbs / peak, "bytes_per_point_update": WORDS_FUSED * 3 * 4,
+            "achieved_gbs": gbs, "frac_of_measured_hbm": gbs / peak, "bytes_per_point_update": WORDS * 3 * 4,
             "stream_value": sites * steps / dt_stream / 1e6, "stream_ms_per_step": dt_stream / steps * 1e3,
             "tma": b.tma_enabled, "finite": bool(np.isfinite(E).all() and np.isfinite(Eg).all()),
             "tile_shapes": {f"{k[0]}x{k[1]}": {"ms_16x64": v[0], "ms_8x32": v[1], "chosen": "8x32" if v[2] else "16x64"}
@@ -794,7 +789,7 @@ def fused_fp64(dev, F0, steps=50):
     e1.record()
     torch.cuda.synchronize(dev)
     ms = e0.elapsed_time(e1) / steps
-    words = WORDS_FUSED if (s.tma_enabled and s._lib.ss_get_variant(s._h, 6) == 1) else WORDS_SEPARATE
+    words = WORDS
     gbs = words * 4 * 8 * XLEN * YLEN / (ms / 1e3) / 1e9
     out = {"value": XLEN * YLEN / (ms / 1e3) / 1e6, "unit": UNIT, "ms_per_step": ms, "steps": steps,
            "achieved_gbs": gbs, "bytes_per_point_update": words * 4 * 8, "finite": bool(torch.isfinite(E).all()),

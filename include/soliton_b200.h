@@ -105,8 +105,8 @@ const char *ss_last_error(void);
 int ss_create(int theory, const int32_t *p_i, int n_i, const double *p_f, int n_f, int precision,
               ss_handle **out);
 int ss_destroy(ss_handle *h);
-/* Bytes of caller-owned device workspace ss_bind() needs (five field-sized flow
- * buffers: l1, l2, the stage-4 field T4 and stage 4's two accumulated inputs; reduction
+/* Bytes of caller-owned device workspace ss_bind() needs (four field-sized flow
+ * buffers: l1, l2 and the second field and velocity that steps alternate with; reduction
  * partials and the device-side step state). */
 int ss_workspace_bytes(const ss_handle *h, size_t *bytes);
 /* Bind the caller's Field and Velocity buffers, the workspace and the stream. */
@@ -134,22 +134,23 @@ int ss_check_status(ss_handle *h);
 /* 1 when the bound Field/Velocity/workspace buffers are staged by TMA tensor maps
  * (row pitch and base 16-byte aligned), 0 when the plain-load path is used. */
 int ss_tma_enabled(const ss_handle *h);
-/* Autotuner: times, on the bound buffers, the two TMA staging variants of each flow
- * stage (persistent CTAs walking tiles through a shared-memory ring, or one tile per
- * CTA) over `iters` launches and keeps the faster one, then times stages 2 and 3 fused
- * into one kernel (one staging of phi, V, l1) against the two chosen kernels.  Writes
- * only workspace scratch.  ms_out (nullable, 14 floats) receives [mode][variant]
- * times for modes 0..6 (mode 6: [two kernels, fused]). */
+/* Autotuner: times, on the bound buffers, the step's phase A (stages 1 and 2), the two
+ * variants of its phase B (stages 3 and 4) and of the gradient (persistent CTAs walking
+ * tiles through a shared-memory ring, or one tile per CTA) over `iters` launches and keeps
+ * the faster variants.  Writes only workspace scratch.  ms_out (nullable, 14 floats)
+ * receives [mode][variant] times: modes 1 and 2 phase A (one form), 3 and 4 phase B, 0 the
+ * gradient, 6 the two phases together. */
 int ss_autotune(ss_handle *h, int iters, float *ms_out);
-/* Variant chosen for a flow mode (0..5): 1 pipelined, 0 one tile per CTA; mode 6: 1 if
- * stages 2 and 3 run fused; -1 bad args. */
+/* Variant chosen or pinned for a mode (0 gradient, 1..4 the RK stages, 5 the energy): 1
+ * pipelined, 0 one tile per CTA; mode 6: the value pinned; -1 bad args. */
 int ss_get_variant(const ss_handle *h, int mode);
-/* Pin the staging variant of a flow mode instead of autotuning it: mode 0 (gradient)
- * or 1..4 (stages; stage 1 also sets the energy pass, whose per-CTA partials must
- * match it), variant 0 (one tile per CTA) or 1 (pipelined; needs TMA-staged bound
- * buffers and FP32 fields); mode 6: 1 runs stages 2 and 3 as one kernel (with TMA
- * staging), 0 as two.  For reproducible runs and for profiling a known kernel set.
- * No reference counterpart (tuning control). */
+/* Pin the staging variant of a mode instead of autotuning it: mode 0 (gradient) or 1..4
+ * (RK stages; stages 3 and 4 run as one kernel, pinned by mode 4; stages 1 and 2 run as
+ * one kernel with one form, so modes 1 and 2 are kept but change nothing, mode 1 sets the
+ * energy observable's variant as well), variant 0 (one tile per CTA) or 1 (pipelined;
+ * needs TMA-staged bound buffers and FP32 fields); mode 6 (0 or 1) is kept and changes
+ * nothing.  For reproducible runs and for profiling a known kernel set.  No reference
+ * counterpart (tuning control). */
 int ss_set_variant(ss_handle *h, int mode, int variant);
 /* Failure-detection hook.  Sets the bound (clock64 cycles, default 2e9) of every
  * device-side mbarrier wait of this handle's kernels; with inject != 0 the next

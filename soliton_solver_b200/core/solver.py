@@ -140,10 +140,11 @@ class Solver:
         return bool(self._lib.ss_tma_enabled(self._h))
 
     def autotune(self, iters: int = 5):
-        """Pick the faster TMA staging variant of each flow stage on the bound buffers.
+        """Pick the faster staging variants of the flow's kernels on the bound buffers.
 
-        Returns {stage: (ms one-tile-per-CTA, ms pipelined, chosen)} for stages 1-4 and
-        {6: (ms stages 2 and 3 as two kernels, ms fused, 1 if fused)}."""
+        Returns {stage: (ms one-tile-per-CTA, ms pipelined, chosen)} for stages 1-4 (1 and 2:
+        the step's first kernel, which has one form; 3 and 4: its second) and {6: (ms of both
+        kernels, the same, pinned value)}."""
         ms = np.zeros(14, dtype=np.float32)
         with torch.cuda.device(self.device):
             nat.check(self._lib.ss_autotune(self._h, int(iters), ms.ctypes.data))
@@ -171,8 +172,8 @@ class Solver:
                                                   int(vortex), float(rotation)))
 
     def set_variant(self, stage: int, variant: int):
-        """Pin the staging variant of flow mode `stage` (0 gradient, 1-4 stages):
-        0 one tile per CTA, 1 pipelined (see ss_set_variant)."""
+        """Pin the staging variant of mode `stage` (0 gradient, 1-4 RK stages): 0 one tile
+        per CTA, 1 pipelined (see ss_set_variant)."""
         nat.check(self._lib.ss_set_variant(self._h, int(stage), int(variant)))
 
     def debug_wait_timeout(self, wait_cycles: int, inject: bool):

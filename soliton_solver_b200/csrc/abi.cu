@@ -14,6 +14,7 @@
 #include "../../include/soliton_b200.h"
 #include "common.cuh"
 #include "flow.cuh"
+#include "rk.cuh"
 #include "plain.cuh"
 #include "batch.cuh"
 #include "render.cuh"
@@ -30,9 +31,9 @@ namespace {
 constexpr int TX = 16, TY = 64, NT = 256;  // fused tile: 16 x 64 sites, 256 threads
 constexpr int TRAJ_CAP = 1024;              // device trajectory slots used by ss_step
 constexpr size_t ALIGN = 256;
-// TMA maps of a bound handle: halo boxes of the field, the velocity, l1 and T4 (l[2]),
-// and centre boxes of cP and cV
-enum { TM_FIELD = 0, TM_VEL = 1, TM_L1 = 2, TM_T4 = 3, TM_CP = 4, TM_CV = 5, TM_COUNT = 6 };
+// Tensor maps of a bound handle (halo boxes): phi and V of the caller's buffers and of the
+// workspace's pair in the tile shapes of phases A and B, l1 and l2 in phase B's
+enum { TM_A = 0, TM_B = 4, TM_L = 8, TM_COUNT = 10 };  // TM_A + 2 * pair + (0 phi, 1 V); TM_L + (0 l1, 1 l2)
 
 thread_local char g_err[512] = "";
 
@@ -93,7 +94,7 @@ struct ss_handle {
   Grid G{};
   Phys P{};
   size_t elem = 8;
-  int nblocks = 0;        // fused tiles
+  int nblocks = 0;        // 16 x 64 tiles (gradient, energy, densities)
   int plain_sum_blocks = 0, plain_max_blocks = 0;
   // bound buffers
   void* field = nullptr;
@@ -106,11 +107,10 @@ struct ss_handle {
   double* partial = nullptr;
   double* traj_E = nullptr;
   double* traj_err = nullptr;
-  // fused flow buffers: l1, l2 (four-kernel steps only), T4; then cP and cV (stage 4's
-  // inputs besides T4: phi + dt V + dt (l1 + l2 + l3)/6 and V + (l1 + 2 l2 + 2 l3)/6)
+  // fused flow buffers: l1, l2 and the second phi, V that steps alternate with
   void* l[4] = {nullptr, nullptr, nullptr, nullptr};
-  void* cp_buf = nullptr;
-  void* cv_buf = nullptr;
+  void* phi2 = nullptr;
+  void* vel2 = nullptr;
   // plain extras
   void* k[4] = {nullptr, nullptr, nullptr, nullptr};
   void* temp = nullptr;
@@ -125,7 +125,8 @@ struct ss_handle {
   CUtensorMap tm[TM_COUNT];
   bool tma = false;
   int num_sms = 148;
-  // per flow mode: 1 = persistent pipelined kernel, 0 = one tile per CTA (autotuned)
+  // per flow mode: 1 = persistent pipelined kernel, 0 = one tile per CTA (autotuned).  The
+  // gradient's (0) and phase B's (3, 4) are read; 1, 2, 5 and fuse23 are kept as pinned
   int use_pipe[N_FLOW_MODES] = {1, 1, 1, 1, 1, 1, 0};
   float tune_ms[N_FLOW_MODES][2] = {};
   int fuse23 = 1;  // stages 2 and 3 in one kernel (TMA staging only)
@@ -158,7 +159,8 @@ size_t layout(ss_handle* h, char* base) {
   };
   const size_t field_bytes = h->elem * (size_t)h->nf * (size_t)h->G.N;
   h->st = (StepState*)take(sizeof(StepState));
-  const size_t np = (size_t)std::max(h->nblocks, std::max(h->plain_sum_blocks, h->plain_max_blocks));
+  // energy partials: one per tile of 16 rows, or of 8 in the step's phases
+  const size_t np = (size_t)std::max(2 * h->nblocks, std::max(h->plain_sum_blocks, h->plain_max_blocks));
   h->partial = (double*)take(np * sizeof(double));
   h->traj_E = (double*)take(TRAJ_CAP * sizeof(double));
   h->traj_err = (double*)take(TRAJ_CAP * sizeof(double));
@@ -172,10 +174,10 @@ size_t layout(ss_handle* h, char* base) {
     h->en = (double*)take((size_t)h->G.N * sizeof(double));
     h->entmp = (double*)take((size_t)h->G.N * sizeof(double));
   } else {
-    for (int i = 0; i < 3; ++i) h->l[i] = take(field_bytes);
-    h->l[3] = nullptr;
-    h->cp_buf = take(field_bytes);
-    h->cv_buf = take(field_bytes);
+    for (int i = 0; i < 2; ++i) h->l[i] = take(field_bytes);
+    h->l[2] = h->l[3] = nullptr;
+    h->phi2 = take(field_bytes);
+    h->vel2 = take(field_bytes);
   }
   return off;
 }
@@ -330,73 +332,29 @@ struct Fused {
   // tma: use the TMA-staged instantiation (A.tm_* must describe A's buffers)
   static inline unsigned long long smem_done[2][N_FLOW_MODES] = {};
 
-  // dynamic shared memory of flow_kernel: the staged buffers
-  template <bool TMA_, int MODE>
-  static constexpr size_t flow_smem() {
-    return TMA_ ? flow_buffers(MODE) * BUF : BUF;
-  }
-
-  // threads of a one-tile CTA: 512 where the staged buffers leave room for only one CTA
-  // per SM (above 113 KB: FP64 stages 3 and 2+3, and stage 2 of the six-component s+id
-  // in FP64), else 256
-  template <bool TMA_, int MODE>
-  static constexpr int flow_threads() {
-    return flow_smem<TMA_, MODE>() > 113 * 1024 ? 2 * NT : NT;
-  }
-
   template <bool TMA_, int MODE>
   static int launch_mode(const ss_handle* h, const FlowArgs<R>& A) {
-    constexpr int NTM = flow_threads<TMA_, MODE>();
-    auto k = flow_kernel<TH, R, TX, TY, NTM, TMA_, MODE>;
-    const size_t smem = flow_smem<TMA_, MODE>();
-    set_smem(k, smem, smem_done[TMA_ ? 1 : 0][MODE]);
-    k<<<h->nblocks, NTM, smem, h->stream>>>(A);
+    auto k = flow_kernel<TH, R, TX, TY, NT, TMA_, MODE>;
+    set_smem(k, BUF, smem_done[TMA_ ? 1 : 0][MODE]);
+    k<<<h->nblocks, NT, BUF, h->stream>>>(A);
     CK(cudaGetLastError());
     return SS_OK;
   }
 
   template <bool TMA_>
   static int launch_tma(const ss_handle* h, const FlowArgs<R>& A) {
-    switch (A.mode) {
-      case M_GRAD: return launch_mode<TMA_, M_GRAD>(h, A);
-      case M_S1: return launch_mode<TMA_, M_S1>(h, A);
-      case M_S2: return launch_mode<TMA_, M_S2>(h, A);
-      case M_S3: return launch_mode<TMA_, M_S3>(h, A);
-      case M_S4: return launch_mode<TMA_, M_S4>(h, A);
-      case M_ENERGY: return launch_mode<TMA_, M_ENERGY>(h, A);
-      case M_S23:
-        if constexpr (TMA_) return launch_mode<TMA_, M_S23>(h, A);
-        else return fail(SS_ERR_ARG, "the fused stages 2+3 need TMA staging");
-    }
-    return fail(SS_ERR_ARG, "bad flow mode");
+    return A.mode == M_GRAD ? launch_mode<TMA_, M_GRAD>(h, A) : launch_mode<TMA_, M_ENERGY>(h, A);
   }
 
-  // persistent TMA-pipelined variant: FP32 fields and at least two ring slots; threads
-  // and resident CTAs per SM from pipe_threads / pipe_ctas
-  template <int MODE>
-  static constexpr int pipe_stages() {
-    const size_t slot = pipe_slot_bytes<R, TH::NF, TX, TY, MODE>();
-    // dynamic shared memory left next to the static reduction arrays, per resident CTA
-    const size_t budget = pipe_ctas<TH, MODE>() == 4 ? 50 * 1024 : 212 * 1024;
-    const int n = (int)(budget / slot);
-    return n > 4 ? 4 : n;
-  }
-  template <int MODE>
-  static constexpr bool pipe_ok() {
-    return sizeof(R) == 4 && pipe_stages<MODE>() >= 2;
-  }
+  // persistent TMA-pipelined variant: FP32 fields
+  static constexpr int PIPE_STAGES = 212 * 1024 / BUF > 4 ? 4 : (int)(212 * 1024 / BUF);
   static inline unsigned long long smem_done_pipe[N_FLOW_MODES] = {};
-
   template <int MODE>
   static int launch_pipe(const ss_handle* h, const FlowArgs<R>& A) {
-    if constexpr (pipe_ok<MODE>()) {
-      constexpr int S = pipe_stages<MODE>();
-      constexpr int NTP = pipe_threads<TH, MODE>();
-      auto k = flow_kernel_pipe<TH, R, TX, TY, NTP, MODE, S>;
-      const size_t smem = S * pipe_slot_bytes<R, TH::NF, TX, TY, MODE>();
-      set_smem(k, smem, smem_done_pipe[MODE]);
-      const int grid = std::min(h->nblocks, pipe_ctas<TH, MODE>() * h->num_sms);
-      k<<<grid, NTP, smem, h->stream>>>(A);
+    if constexpr (sizeof(R) == 4) {
+      auto k = flow_kernel_pipe<TH, R, TX, TY, 2 * NT, MODE, PIPE_STAGES>;
+      set_smem(k, PIPE_STAGES * BUF, smem_done_pipe[MODE]);
+      k<<<std::min(h->nblocks, h->num_sms), 2 * NT, PIPE_STAGES * BUF, h->stream>>>(A);
       CK(cudaGetLastError());
       return SS_OK;
     } else {
@@ -404,19 +362,10 @@ struct Fused {
     }
   }
 
-  static bool uses_pipe(int mode) {
-    switch (mode) {
-      case M_GRAD: return pipe_ok<M_GRAD>();
-      case M_S1: return pipe_ok<M_S1>();
-      case M_S2: return pipe_ok<M_S2>();
-      case M_S3: return pipe_ok<M_S3>();
-      case M_S4: return pipe_ok<M_S4>();
-      case M_ENERGY: return pipe_ok<M_ENERGY>();
-    }
-    return false;
-  }
+  // whether a mode has a pipelined variant (phase A's, M_S1 and M_S2, is accepted and ignored)
+  static bool uses_pipe(int) { return sizeof(R) == 4; }
 
-  // tma: use the TMA-staged instantiations (A.tm_* must describe A's buffers)
+  // tma: use the TMA-staged instantiations (A.tm_phi must describe A.phi)
   static int launch(const ss_handle* h, const FlowArgs<R>& A0, bool tma) {
     FlowArgs<R> A = A0;
     if (h->inject_timeout && tma) {
@@ -424,19 +373,9 @@ struct Fused {
       h->inject_timeout = 0;
     }
     if (!tma) return launch_tma<false>(h, A);
-    // exact FP64 energies (observables) run one tile per CTA: the pipelined energy pass
-    // of the packed-energy theories is built for the flow energy only
-    if (!h->use_pipe[A.mode] || (A.mode == M_ENERGY && A.exact_energy && pipe_ctas<TH, M_ENERGY>() == 4))
-      return launch_tma<true>(h, A);
-    switch (A.mode) {
-      case M_GRAD: return launch_pipe<M_GRAD>(h, A);
-      case M_S1: return launch_pipe<M_S1>(h, A);
-      case M_S2: return launch_pipe<M_S2>(h, A);
-      case M_S3: return launch_pipe<M_S3>(h, A);
-      case M_S4: return launch_pipe<M_S4>(h, A);
-      case M_ENERGY: return launch_pipe<M_ENERGY>(h, A);
-    }
-    return fail(SS_ERR_ARG, "bad flow mode");
+    // the chiral magnet's exact energy is better one tile per CTA
+    if (!h->use_pipe[A.mode] || (A.mode == M_ENERGY && TH::S1_CTAS == 4)) return launch_tma<true>(h, A);
+    return A.mode == M_GRAD ? launch_pipe<M_GRAD>(h, A) : launch_pipe<M_ENERGY>(h, A);
   }
 
   static FlowArgs<R> base_args(const ss_handle* h) {
@@ -447,134 +386,133 @@ struct Fused {
     A.P = h->P;
     A.st = h->st;
     A.partial = h->partial;
+    return A;
+  }
+
+  // ---- the RK4 step (rk.cuh) ------------------------------------------------
+  static constexpr int TXA = StepShape<TH, R, PH_A>::TX;
+
+  // tensor maps of a phase's inputs (phi and V of the pair that A.phi belongs to)
+  static StepMaps phase_maps(const ss_handle* h, const StepArgs<R>& A, int maps) {
+    const int pair = (const void*)A.phi == h->phi2 ? 1 : 0;
+    return StepMaps{h->tm[maps + 2 * pair], h->tm[maps + 2 * pair + 1], h->tm[TM_L], h->tm[TM_L + 1]};
+  }
+  template <bool TMA_, int PH>
+  static int launch_phase(const ss_handle* h, StepArgs<R>& A, const StepMaps* M = nullptr) {
+    constexpr int NTP = StepShape<TH, R, PH>::NT;
+    constexpr size_t smem = step_smem<TH, R, PH, TMA_>();
+    auto k = step_kernel<TH, R, TMA_, PH>;
+    static unsigned long long done = 0;  // one per instantiation
+    set_smem(k, smem, done);
+    A.tx_extra = 0;
+    if (TMA_ && h->inject_timeout) {
+      A.tx_extra = 16;
+      h->inject_timeout = 0;
+    }
+    constexpr int TXP = StepShape<TH, R, PH>::TX;
+    const int tiles = ((h->G.X + TXP - 1) / TXP) * ((h->G.Y + TY - 1) / TY);
+    k<<<tiles, NTP, smem, h->stream>>>(M ? *M : phase_maps(h, A, PH == PH_B ? TM_B : TM_A), A);
+    CK(cudaGetLastError());
+    return SS_OK;
+  }
+  static int launch_phase_pipe(const ss_handle* h, StepArgs<R>& A) {
+    using SH = PipeShape<TH, R>;
+    if constexpr (SH::OK) {
+      auto k = step_kernel_pipe<TH, R>;
+      static unsigned long long done = 0;
+      set_smem(k, SH::SLOTS * SH::SLOT, done);
+      A.tx_extra = 0;
+      if (h->inject_timeout) {
+        A.tx_extra = 16;
+        h->inject_timeout = 0;
+      }
+      const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + SH::TY - 1) / SH::TY);
+      k<<<std::min(tiles, h->num_sms), SH::NT, SH::SLOTS * SH::SLOT, h->stream>>>(phase_maps(h, A, TM_B), A);
+      CK(cudaGetLastError());
+      return SS_OK;
+    } else {
+      return launch_phase<true, PH_B>(h, A);
+    }
+  }
+  template <int PH>
+  static int launch_phase(const ss_handle* h, StepArgs<R>& A) {
+    if (!h->tma) return launch_phase<false, PH>(h, A);
+    if (PH == PH_B && h->use_pipe[M_S4]) return launch_phase_pipe(h, A);
+    return launch_phase<true, PH>(h, A);
+  }
+
+  static StepArgs<R> step_args(const ss_handle* h) {
+    StepArgs<R> A;
+    memset(&A, 0, sizeof(A));
+    A.wait_cycles = h->wait_cycles;
+    A.G = h->G;
+    A.P = h->P;
+    A.st = h->st;
+    A.partial = h->partial;
     A.force = h->force;
+    A.l1 = A.out_l1 = (R*)h->l[0];
+    A.l2 = A.out_l2 = (R*)h->l[1];
     A.E_idx = -1;
     A.err_idx = -1;
     A.prev_energy = NAN;
     return A;
+  }
+  // phi and V of buffer pair `pair` (0: the caller's, 1: the workspace's) as a phase's inputs
+  static void set_input(const ss_handle* h, StepArgs<R>& A, int pair) {
+    A.phi = (const R*)(pair ? h->phi2 : h->field);
+    A.vel = (const R*)(pair ? h->vel2 : h->vel);
   }
 
   // n flow steps of the bound buffers, in place; trajectories to device arrays (nullable)
   // status_out (nullable, device-visible): the finish kernel copies the call's status there
   static int step(ss_handle* h, int n, double prev, double* E_dev, double* err_dev, int* status_out = nullptr) {
     if (n <= 0) return SS_OK;
-    R* field = (R*)h->field;
-    R* vel = (R*)h->vel;
-    R* l1 = (R*)h->l[0];
-    R* l2 = (R*)h->l[1];
-    R* t4 = (R*)h->l[2];
-    R* cp = (R*)h->cp_buf;
-    R* cv = (R*)h->cv_buf;
-    FlowArgs<R> A = base_args(h);
+    StepArgs<R> A = step_args(h);
     A.E_traj = E_dev;
     A.err_traj = err_dev;
-    const bool tma = h->tma;
-    const bool fused23 = tma && h->fuse23;
-    A.vel = vel;
-    A.la = l1;
-    A.lb = l2;
-    A.out_t4 = t4;
-    A.out_cp = cp;
-    A.out_cv = cv;
-    A.cp = cp;
-    A.cv = cv;
-    A.phi_out = field;
-    A.vel_out = vel;
-    if (tma) {
-      A.tm_vel = h->tm[TM_VEL];
-      A.tm_l = h->tm[TM_L1];
-      A.tm_cp = h->tm[TM_CP];
-      A.tm_cv = h->tm[TM_CV];
-    }
-    for (int s = 0; s < n; ++s) {
-      // S1: l1 = -dt G(phi); energy of phi (the previous step's result) + arrest test
-      A.mode = M_S1;
-      A.phi = field;
-      A.out_l = l1;
-      A.with_energy = s > 0;
-      A.arrest_update = s > 0;
+    int rc, cur = 0;
+    for (int s = 0; s < n; ++s, cur ^= 1) {
+      // A: l1, l2; energy of phi (the previous step's result) and its arrest test
+      A.with_energy = A.arrest_update = s > 0;
       A.E_idx = s - 1;
       A.init_state = s == 0;
       A.prev_energy = prev;
-      if (tma) A.tm_phi = h->tm[TM_FIELD];
-      int rc = launch(h, A, tma);
-      if (rc) return rc;
-      A.with_energy = 0;
-      A.arrest_update = 0;
+      set_input(h, A, cur);
+      if ((rc = launch_phase<PH_A>(h, A))) return rc;
       A.init_state = 0;
-      A.E_idx = -1;
-      // S2, S3 (one fused kernel on TMA-staged buffers: one staging of phi, V, l1):
-      // T4, cV, cP
-      if (fused23) {
-        A.mode = M_S23;
-        if ((rc = launch(h, A, tma))) return rc;
-      } else {
-        A.mode = M_S2;
-        A.out_l = l2;
-        if ((rc = launch(h, A, tma))) return rc;
-        A.mode = M_S3;
-        if ((rc = launch(h, A, tma))) return rc;
-      }
-      A.out_l = nullptr;
-      // S4: phi' and V' into the caller's buffers, err
-      A.mode = M_S4;
-      A.phi = t4;
+      // B: phi' and V' into the other pair, err
       A.err_idx = s;
-      if (tma) A.tm_phi = h->tm[TM_T4];
-      if ((rc = launch(h, A, tma))) return rc;
-      A.err_idx = -1;
+      A.phi_out = (R*)(cur ? h->field : h->phi2);
+      A.vel_out = (R*)(cur ? h->vel : h->vel2);
+      set_input(h, A, cur);
+      if ((rc = launch_phase<PH_B>(h, A))) return rc;
     }
-    // trailing energy of the final field + arrest test
-    A.phi = field;
-    A.mode = M_ENERGY;
-    A.with_energy = 1;
-    A.arrest_update = 1;
+    // trailing energy of the final field and its arrest test; phi back to the caller's buffer
+    A.with_energy = A.arrest_update = 1;
     A.E_idx = n - 1;
-    if (tma) A.tm_phi = h->tm[TM_FIELD];
-    int rc = launch(h, A, tma);
-    if (rc) return rc;
+    A.phi_out = cur ? (R*)h->field : nullptr;
+    set_input(h, A, cur);
+    if ((rc = launch_phase<PH_E>(h, A))) return rc;
     const long long nfN = (long long)h->nf * h->G.N;
-    finish_kernel<R><<<grid_1d(nfN), 256, 0, h->stream>>>(vel, nfN, h->st, status_out);
+    step_finish_kernel<R><<<grid_1d(nfN), 256, 0, h->stream>>>((R*)h->vel, cur ? (const R*)h->vel2 : nullptr, nfN,
+                                                               h->st, status_out);
     CK(cudaGetLastError());
     return SS_OK;
   }
 
-  // Time both staging variants of every stage on the bound buffers and keep the faster
-  // one.  Writes only workspace scratch: l1, l2, T4, cV, cP, and stage 4's phi' and V'
-  // into the l1 and l2 buffers (stage 4 reads neither); stage 1's energy reduction
-  // leaves the arrest state and the trajectories alone.
+  // Time the step's two phases and the two staging variants of the gradient on the bound
+  // buffers (the faster gradient variant is kept).  Writes only workspace scratch; the
+  // energy reduction leaves the arrest state and the trajectories alone.
   static int autotune(ss_handle* h, int iters) {
     if (!h->tma) return SS_OK;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    FlowArgs<R> A = base_args(h);
-    A.vel = (const R*)h->vel;
-    A.la = (const R*)h->l[0];
-    A.lb = (const R*)h->l[1];
-    A.out_t4 = (R*)h->l[2];
-    A.out_cp = (R*)h->cp_buf;
-    A.out_cv = (R*)h->cv_buf;
-    A.cp = (const R*)h->cp_buf;
-    A.cv = (const R*)h->cv_buf;
-    A.phi_out = (R*)h->l[0];
-    A.vel_out = (R*)h->l[1];
-    A.tm_vel = h->tm[TM_VEL];
-    A.tm_l = h->tm[TM_L1];
-    A.tm_cp = h->tm[TM_CP];
-    A.tm_cv = h->tm[TM_CV];
-    auto set_mode = [&](int m) {
-      A.mode = m;
-      A.phi = m == M_S4 ? (const R*)h->l[2] : (const R*)h->field;
-      A.tm_phi = h->tm[m == M_S4 ? TM_T4 : TM_FIELD];
-      A.out_l = m == M_S1 ? (R*)h->l[0] : m == M_S2 ? (R*)h->l[1] : nullptr;
-      A.with_energy = m == M_S1 ? 1 : 0;
-    };
-    auto time_mode = [&](float& out) -> int {
-      int rc = launch(h, A, true);  // warm-up
+    auto timed = [&](float& out, auto&& go) -> int {
+      int rc = go();  // warm-up
       if (rc) return rc;
       CK(cudaEventRecord(e0, h->stream));
-      for (int i = 0; i < iters && rc == SS_OK; ++i) rc = launch(h, A, true);
+      for (int i = 0; i < iters && rc == SS_OK; ++i) rc = go();
       CK(cudaEventRecord(e1, h->stream));
       CK(cudaEventSynchronize(e1));
       float ms = 0.f;
@@ -582,35 +520,36 @@ struct Fused {
       out = ms / iters;
       return rc;
     };
-    const int modes[4] = {M_S1, M_S2, M_S3, M_S4};
+    StepArgs<R> A = step_args(h);
+    A.with_energy = 1;
+    A.phi_out = (R*)h->phi2;
+    A.vel_out = (R*)h->vel2;
     int rc = SS_OK;
-    for (int mi = 0; mi < 4 && rc == SS_OK; ++mi) {
-      const int m = modes[mi];
-      if (m == M_S4) {  // stage 4's inputs from this field, whatever stage 3's variants
-        set_mode(M_S3);
-        if ((rc = launch(h, A, true))) break;
+    for (int m : {(int)M_S1, (int)M_S4}) {
+      const bool two = m == M_S4 && PipeShape<TH, R>::OK;
+      for (int v = 0; v < 2 && !rc; ++v) {
+        if (two) h->use_pipe[M_S3] = h->use_pipe[M_S4] = v;
+        set_input(h, A, 0);
+        if (v == 0 || two)
+          rc = timed(h->tune_ms[m][v], [&]() { return m == M_S1 ? launch_phase<PH_A>(h, A) : launch_phase<PH_B>(h, A); });
+        else
+          h->tune_ms[m][1] = h->tune_ms[m][0];
       }
-      set_mode(m);
-      // the one-tile-per-CTA variant always (its time enters the fusion decision below),
-      // the pipelined one where it exists
-      const bool pipe = uses_pipe(m);
-      for (int v = 0; v < (pipe ? 2 : 1) && rc == SS_OK; ++v) {
-        h->use_pipe[m] = v;
-        rc = time_mode(h->tune_ms[m][v]);
-      }
-      h->use_pipe[m] = (pipe && h->tune_ms[m][1] <= h->tune_ms[m][0]) ? 1 : 0;
+      if (two) h->use_pipe[M_S3] = h->use_pipe[M_S4] = h->tune_ms[m][1] <= h->tune_ms[m][0] ? 1 : 0;
+      for (int v = 0; v < 2; ++v) h->tune_ms[m == M_S1 ? M_S2 : M_S3][v] = h->tune_ms[m][v];
     }
-    // the energy-only pass must reduce exactly like stage 1 (same grid and tile order)
-    h->use_pipe[M_ENERGY] = h->use_pipe[M_S1];
-    h->use_pipe[M_GRAD] = h->use_pipe[M_S2];
-    // fused stages 2+3 against the two chosen stage kernels
-    if (rc == SS_OK) {
-      set_mode(M_S23);
-      rc = time_mode(h->tune_ms[M_S23][1]);
-      if (rc == SS_OK) {
-        h->tune_ms[M_S23][0] = h->tune_ms[M_S2][h->use_pipe[M_S2]] + h->tune_ms[M_S3][h->use_pipe[M_S3]];
-        h->fuse23 = h->tune_ms[M_S23][1] <= h->tune_ms[M_S23][0] ? 1 : 0;
+    for (int v = 0; v < 2; ++v) h->tune_ms[M_S23][v] = h->tune_ms[M_S1][0] + h->tune_ms[M_S4][h->use_pipe[M_S4]];
+    if (uses_pipe(M_GRAD)) {
+      FlowArgs<R> F = base_args(h);
+      F.mode = M_GRAD;
+      F.phi = (const R*)h->field;
+      F.out_l = (R*)h->l[0];
+      const bool tma = encode_tile_map(&F.tm_phi, F.phi, sizeof(R), h->G.X, h->G.Y, TH::NF);
+      for (int v = 0; v < 2 && tma && !rc; ++v) {
+        h->use_pipe[M_GRAD] = v;
+        rc = timed(h->tune_ms[M_GRAD][v], [&]() { return launch(h, F, true); });
       }
+      h->use_pipe[M_GRAD] = h->tune_ms[M_GRAD][1] <= h->tune_ms[M_GRAD][0] ? 1 : 0;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -645,11 +584,17 @@ struct Fused {
 
   // the observable: exact FP64 stencil of the stored values for every precision
   static int energy(ss_handle* h, const void* field) {
+    if constexpr (sizeof(R) == 8) {  // the flow's own energy pass: FP64 jets are the exact differences
+      StepArgs<R> S = step_args(h);
+      S.with_energy = 1;
+      S.phi = (const R*)field;
+      StepMaps M{};
+      const bool tma = encode_tile_map(&M.phi, field, sizeof(R), h->G.X, h->G.Y, TH::NF, false, TXA, TY);
+      return tma ? launch_phase<true, PH_E>(h, S, &M) : launch_phase<false, PH_E>(h, S);
+    }
     FlowArgs<R> A = base_args(h);
     A.mode = M_ENERGY;
-    A.exact_energy = 1;
     A.phi = (const R*)field;
-    A.with_energy = 1;
     const bool tma = encode_tile_map(&A.tm_phi, field, sizeof(R), h->G.X, h->G.Y, TH::NF);
     return launch(h, A, tma);
   }
@@ -789,6 +734,16 @@ int dispatch(const ss_handle* h, Fn&& fn) {
   return fail(SS_ERR_ARG, "bad theory");
 }
 
+// rows of the step's phase tiles
+void step_shape(const ss_handle* h, int& txa, int& txb) {
+  dispatch(h, [&](auto* tag) -> int {
+    using TH = std::remove_pointer_t<decltype(tag)>;
+    txa = h->precision == SS_FP32 ? StepShape<TH, float, PH_A>::TX : StepShape<TH, double, PH_A>::TX;
+    txb = h->precision == SS_FP32 ? StepShape<TH, float, PH_B>::TX : StepShape<TH, double, PH_B>::TX;
+    return SS_OK;
+  });
+}
+
 int read_state(ss_handle* h, StepState* out) {
   CK(cudaMemcpyAsync(out, h->st, sizeof(StepState), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -887,8 +842,9 @@ int ss_create(int theory, const int32_t* p_i, int n_i, const double* p_f, int n_
     return rc;
   }
   h->elem = precision == SS_FP32 ? 4 : 8;
+  // the step's phases tile at 8 rows where 16 do not fit: up to twice the tiles
   const long long tiles = (long long)((h->G.X + TX - 1) / TX) * ((h->G.Y + TY - 1) / TY);
-  if (tiles > 0x7fffffffLL) {
+  if (tiles > 0x3fffffffLL) {
     delete h;
     return fail(SS_ERR_ARG, "lattice too large");
   }
@@ -935,10 +891,15 @@ int ss_bind(ss_handle* h, void* field, void* velocity, void* workspace, size_t w
   h->E_last_host = NAN;
   h->tma = false;
   if (h->precision != SS_PLAIN_FP64 && field && velocity) {
-    const void* bufs[TM_COUNT] = {field, velocity, h->l[0], h->l[2], h->cp_buf, h->cv_buf};
+    const void* pairs[4] = {field, velocity, h->phi2, h->vel2};
+    int txa = 0, txb = 0;
+    step_shape(h, txa, txb);
     bool ok = true;
-    for (int i = 0; i < TM_COUNT && ok; ++i)
-      ok = encode_tile_map(&h->tm[i], bufs[i], h->elem, h->G.X, h->G.Y, h->nf, i >= TM_CP);
+    for (int i = 0; i < 4 && ok; ++i)
+      ok = encode_tile_map(&h->tm[TM_A + i], pairs[i], h->elem, h->G.X, h->G.Y, h->nf, false, txa, TY) &&
+           encode_tile_map(&h->tm[TM_B + i], pairs[i], h->elem, h->G.X, h->G.Y, h->nf, false, txb, TY);
+    for (int i = 0; i < 2 && ok; ++i)
+      ok = encode_tile_map(&h->tm[TM_L + i], h->l[i], h->elem, h->G.X, h->G.Y, h->nf, false, txb, TY);
     h->tma = ok;
   }
   int dev = 0, sms = 0;
@@ -1462,15 +1423,12 @@ extern "C" int ss_energy_noalloc(int theory, const int32_t* p_i, int n_i, const 
     if (precision == SS_FP32) {
       FlowArgs<float> A = Fused<TH, float>::base_args(&h);
       A.mode = M_ENERGY;
-      A.exact_energy = 1;
-      A.phi = (const float*)field;
-      A.with_energy = 1;
+        A.phi = (const float*)field;
       return Fused<TH, float>::template launch_mode<false, M_ENERGY>(&h, A);
     }
     FlowArgs<double> A = Fused<TH, double>::base_args(&h);
     A.mode = M_ENERGY;
     A.phi = (const double*)field;
-    A.with_energy = 1;
     return Fused<TH, double>::template launch_mode<false, M_ENERGY>(&h, A);
   });
   if (rc) return rc;
@@ -1486,11 +1444,9 @@ extern "C" int ss_energy_noalloc(int theory, const int32_t* p_i, int n_i, const 
 // ===========================================================================
 // Batched lattices: many independent relaxations of one theory per launch
 // ===========================================================================
-// Tile shapes of the batched stage kernels (x rows, y columns, threads): the
-// autotuner picks one per size class of lattices (ss_batch_autotune).  Shape 1 exists
-// for TMA-staged FP32 batches.
+// Tile shapes of the batched phase kernels (BatchShape): the autotuner picks one per size
+// class of lattices (ss_batch_autotune).  Shape 1 exists for TMA-staged FP32 batches.
 constexpr int N_BATCH_SHAPES = 2;
-constexpr int BSHAPE_TX[N_BATCH_SHAPES] = {16, 8};
 constexpr int BSHAPE_TY[N_BATCH_SHAPES] = {64, 32};
 
 struct ss_batch {
@@ -1500,13 +1456,13 @@ struct ss_batch {
   std::vector<int> shape;        // tile shape per lattice
   std::vector<int> max_tiles;    // tiles per lattice in its finest shape (partials are sized for it)
   int total_max = 0;             // sum of max_tiles: capacity of each tile list
-  int group_tiles[N_BATCH_SHAPES] = {0, 0};  // tiles of the lattices of each shape
+  int group_tiles[N_BATCH_SHAPES][2] = {};  // tiles of the lattices of each shape and phase
   bool tma = false;
   cudaStream_t stream = nullptr;
   char* ws = nullptr;
   BatchInst* d_insts = nullptr;
-  int* d_tile_inst[N_BATCH_SHAPES] = {nullptr, nullptr};  // lattice of each tile, per shape group
-  int* d_tune_tiles = nullptr;   // a single size class's tiles while the autotuner times it
+  // lattice of each tile, per shape group and phase (A and E, B)
+  int* d_tile_inst[N_BATCH_SHAPES][2] = {};
   float tune_ms[64][N_BATCH_SHAPES] = {};  // autotuner: per size class (first 64) and shape
   double* d_prev = nullptr;
   std::vector<BatchInst> h_insts;
@@ -1535,8 +1491,8 @@ size_t batch_layout(ss_batch* b, char* base) {
     return p;
   };
   b->d_insts = (BatchInst*)take(sizeof(BatchInst) * b->n);
-  for (int g = 0; g < N_BATCH_SHAPES; ++g) b->d_tile_inst[g] = (int*)take(sizeof(int) * b->total_max);
-  b->d_tune_tiles = (int*)take(sizeof(int) * b->total_max);
+  for (int g = 0; g < N_BATCH_SHAPES; ++g)
+    for (int p = 0; p < 2; ++p) b->d_tile_inst[g][p] = (int*)take(sizeof(int) * b->total_max);
   b->d_prev = (double*)take(sizeof(double) * b->n);
   b->d_st = (StepState*)take(sizeof(StepState) * b->n);
   b->d_E = (double*)take(sizeof(double) * TRAJ_CAP * b->n);
@@ -1549,97 +1505,10 @@ size_t batch_layout(ss_batch* b, char* base) {
     I.partial = (double*)take(sizeof(double) * b->max_tiles[i]);
     I.E_traj = b->d_E ? b->d_E + (size_t)i * TRAJ_CAP : nullptr;
     I.err_traj = b->d_err ? b->d_err + (size_t)i * TRAJ_CAP : nullptr;
-    for (int k = BB_CP; k < BB_COUNT; ++k) I.buf[k] = take(fb);
+    for (int k = BB_PHI2; k < BB_COUNT; ++k) I.buf[k] = take(fb);
   }
   return off;
 }
-
-template <class TH, typename R>
-struct Batched {
-  // one launch over the tiles of `tile_inst` (lattices of one tile shape)
-  template <int BTX, int BTY, int BNT, bool TMA_, int MODE>
-  static int launch_shape(const ss_batch* b, const BatchStep& B, const int* tile_inst, int ntiles) {
-    if (ntiles <= 0) return SS_OK;
-    constexpr size_t BUF = tile_buf_bytes<R, TH::NF, BTX, BTY>();
-    constexpr size_t smem = TMA_ ? flow_buffers(MODE) * BUF : BUF;
-    constexpr int NTM = smem > 113 * 1024 ? 2 * BNT : BNT;  // as Fused::flow_threads
-    auto k = batch_flow_kernel<TH, R, BTX, BTY, NTM, TMA_, MODE>;
-    static unsigned long long smem_done = 0;  // one per instantiation
-    set_smem(k, smem, smem_done);
-    k<<<ntiles, NTM, smem, b->stream>>>(b->d_insts, tile_inst, B);
-    CK(cudaGetLastError());
-    return SS_OK;
-  }
-  // a stage over every shape group (shape 1: TMA-staged FP32 batches only)
-  template <int MODE>
-  static int launch(const ss_batch* b, const BatchStep& B) {
-    int rc;
-    if constexpr (MODE == M_S23) {  // needs TMA staging
-      rc = launch_shape<16, 64, NT, true, MODE>(b, B, b->d_tile_inst[0], b->group_tiles[0]);
-    } else {
-      rc = b->tma ? launch_shape<16, 64, NT, true, MODE>(b, B, b->d_tile_inst[0], b->group_tiles[0])
-                  : launch_shape<16, 64, NT, false, MODE>(b, B, b->d_tile_inst[0], b->group_tiles[0]);
-    }
-    if (rc) return rc;
-    if constexpr (sizeof(R) == 4) {
-      if (b->tma && b->group_tiles[1] > 0)
-        rc = launch_shape<8, 32, 128, true, MODE>(b, B, b->d_tile_inst[1], b->group_tiles[1]);
-    }
-    return rc;
-  }
-
-  static int step(ss_batch* b, int n, bool use_prev) {
-    if (n <= 0) return SS_OK;
-    BatchStep B;
-    memset(&B, 0, sizeof(B));
-    B.wait_cycles = b->wait_cycles;
-    int rc;
-    for (int s = 0; s < n; ++s) {
-      B.with_energy = s > 0;
-      B.arrest_update = s > 0;
-      B.init_state = s == 0;
-      B.prev_energy = (s == 0 && use_prev) ? b->d_prev : nullptr;
-      B.E_idx = s - 1;
-      B.err_idx = -1;
-      if ((rc = launch<M_S1>(b, B))) return rc;
-      B.with_energy = B.arrest_update = B.init_state = 0;
-      B.prev_energy = nullptr;
-      B.E_idx = -1;
-      if (b->tma) {  // stages 2 and 3 fused (one staging of phi, V, l1)
-        if ((rc = launch<M_S23>(b, B))) return rc;
-      } else {
-        if ((rc = launch<M_S2>(b, B))) return rc;
-        if ((rc = launch<M_S3>(b, B))) return rc;
-      }
-      B.err_idx = s;
-      if ((rc = launch<M_S4>(b, B))) return rc;  // in place
-      B.err_idx = -1;
-    }
-    B.with_energy = B.arrest_update = 1;
-    B.E_idx = n - 1;
-    if ((rc = launch<M_ENERGY>(b, B))) return rc;
-    batch_finish_kernel<R, TH::NF><<<dim3(64, b->n), 256, 0, b->stream>>>(b->d_insts);
-    CK(cudaGetLastError());
-    return SS_OK;
-  }
-
-  // The stage launches of one step with every reduction, trajectory and arrest update
-  // off: reads the current fields, writes only workspace scratch (l1, l2, T4, cV, cP,
-  // and stage 4's phi' and V' into l1 and l2).
-  static int timing_step(ss_batch* b) {
-    BatchStep B;
-    memset(&B, 0, sizeof(B));
-    B.wait_cycles = b->wait_cycles;
-    B.E_idx = -1;
-    B.err_idx = -1;
-    int rc = launch<M_S1>(b, B);
-    if (!rc) rc = b->tma ? launch<M_S23>(b, B) : launch<M_S2>(b, B);
-    if (!rc && !b->tma) rc = launch<M_S3>(b, B);
-    B.scratch_out = 1;
-    if (!rc) rc = launch<M_S4>(b, B);
-    return rc;
-  }
-};
 
 template <class Fn>
 int batch_dispatch(const ss_batch* b, Fn&& fn) {
@@ -1652,9 +1521,91 @@ int batch_dispatch(const ss_batch* b, Fn&& fn) {
   return fail(SS_ERR_ARG, "bad theory");
 }
 
-// tiles of a lattice in tile shape `shape`
-long long batch_tiles(const Grid& G, int shape) {
-  return (long long)((G.X + BSHAPE_TX[shape] - 1) / BSHAPE_TX[shape]) * ((G.Y + BSHAPE_TY[shape] - 1) / BSHAPE_TY[shape]);
+template <class TH, typename R>
+struct Batched {
+  // one launch over the tiles of `tile_inst` (lattices of one tile shape)
+  template <bool SMALL, bool TMA_, int PH>
+  static int launch_shape(const ss_batch* b, const BatchStep& B, const int* tile_inst, int ntiles) {
+    if (ntiles <= 0) return SS_OK;
+    using SH = BatchShape<TH, R, PH, SMALL>;
+    constexpr size_t smem = step_buffers<PH, TMA_>() * tile_buf_bytes<R, TH::NF, SH::TX, SH::TY>();
+    auto k = batch_step_kernel<TH, R, SMALL, TMA_, PH>;
+    static unsigned long long smem_done = 0;  // one per instantiation
+    set_smem(k, smem, smem_done);
+    k<<<ntiles, SH::NT, smem, b->stream>>>(b->d_insts, tile_inst, B);
+    CK(cudaGetLastError());
+    return SS_OK;
+  }
+  // a phase over every shape group (shape 1: TMA-staged FP32 batches only)
+  template <int PH>
+  static int launch(const ss_batch* b, const BatchStep& B) {
+    constexpr int p = PH == PH_B ? 1 : 0;
+    int rc = b->tma ? launch_shape<false, true, PH>(b, B, b->d_tile_inst[0][p], b->group_tiles[0][p])
+                    : launch_shape<false, false, PH>(b, B, b->d_tile_inst[0][p], b->group_tiles[0][p]);
+    if constexpr (sizeof(R) == 4) {
+      if (!rc && b->tma) rc = launch_shape<true, true, PH>(b, B, b->d_tile_inst[1][p], b->group_tiles[1][p]);
+    }
+    return rc;
+  }
+
+  static int step(ss_batch* b, int n, bool use_prev) {
+    if (n <= 0) return SS_OK;
+    BatchStep B;
+    memset(&B, 0, sizeof(B));
+    B.wait_cycles = b->wait_cycles;
+    B.E_idx = B.err_idx = -1;
+    int rc;
+    for (int s = 0; s < n; ++s, B.cur ^= 1) {
+      B.with_energy = B.arrest_update = s > 0;
+      B.init_state = s == 0;
+      B.prev_energy = (s == 0 && use_prev) ? b->d_prev : nullptr;
+      B.E_idx = s - 1;
+      if ((rc = launch<PH_A>(b, B))) return rc;
+      B.init_state = 0;
+      B.prev_energy = nullptr;
+      B.err_idx = s;
+      if ((rc = launch<PH_B>(b, B))) return rc;
+    }
+    B.with_energy = B.arrest_update = 1;
+    B.E_idx = n - 1;
+    if ((rc = launch<PH_E>(b, B))) return rc;
+    batch_finish_kernel<R, TH::NF><<<dim3(64, b->n), 256, 0, b->stream>>>(b->d_insts, B.cur);
+    CK(cudaGetLastError());
+    return SS_OK;
+  }
+
+  // The launches of one step with every trajectory and arrest update off: reads the
+  // current fields, writes only workspace scratch (l1, l2 and the second pair).
+  static int timing_step(ss_batch* b) {
+    BatchStep B;
+    memset(&B, 0, sizeof(B));
+    B.wait_cycles = b->wait_cycles;
+    B.E_idx = -1;
+    B.err_idx = -1;
+    int rc = launch<PH_A>(b, B);
+    if (!rc) rc = launch<PH_B>(b, B);
+    return rc;
+  }
+};
+
+// rows of a tile of shape `shape` in phase p (0: A and E, 1: B)
+int batch_tx(const ss_batch* b, int shape, int p) {
+  int tx = 0;
+  batch_dispatch(b, [&](auto* tag) -> int {
+    using TH = std::remove_pointer_t<decltype(tag)>;
+    if (b->precision == SS_FP32)
+      tx = shape ? (p ? BatchShape<TH, float, PH_B, true>::TX : BatchShape<TH, float, PH_A, true>::TX)
+                 : (p ? BatchShape<TH, float, PH_B, false>::TX : BatchShape<TH, float, PH_A, false>::TX);
+    else
+      tx = p ? BatchShape<TH, double, PH_B, false>::TX : BatchShape<TH, double, PH_A, false>::TX;
+    return SS_OK;
+  });
+  return tx;
+}
+// tiles of a lattice in tile shape `shape`, phase p
+long long batch_tiles(const ss_batch* b, const Grid& G, int shape, int p) {
+  const int tx = batch_tx(b, shape, p), ty = BSHAPE_TY[shape];
+  return (long long)((G.X + tx - 1) / tx) * ((G.Y + ty - 1) / ty);
 }
 
 // TMA maps of lattice i for its current tile shape (buffers already set); false when
@@ -1664,32 +1615,32 @@ bool batch_encode(ss_batch* b, int i) {
   const int sh = b->shape[i];
   bool ok = true;
   for (int k = 0; k < BT_COUNT && ok; ++k)
-    ok = encode_tile_map(&I.tm[k], I.buf[BATCH_TM_BUF[k]], b->elem, I.G.X, I.G.Y, b->nf, false, BSHAPE_TX[sh],
-                         BSHAPE_TY[sh]);
+    ok = encode_tile_map(&I.tm[k], I.buf[BATCH_TM_BUF[k]], b->elem, I.G.X, I.G.Y, b->nf, false,
+                         batch_tx(b, sh, k >= BT_B ? 1 : 0), BSHAPE_TY[sh]);
   return ok;
 }
 
 // Rebuild the per-shape tile lists from the lattices with include[i] (all when null),
 // set each lattice's tile range and copy the descriptors and lists to the device.
 int batch_upload(ss_batch* b, const std::vector<char>* include) {
-  std::vector<int> lists[N_BATCH_SHAPES];
+  std::vector<int> lists[N_BATCH_SHAPES][2];
   for (int i = 0; i < b->n; ++i) {
     BatchInst& I = b->h_insts[i];
     const int sh = b->shape[i];
-    I.ntiles = (int)batch_tiles(I.G, sh);
-    if (include && !(*include)[i]) {
-      I.tile0 = 0;
-      continue;
+    for (int p = 0; p < 2; ++p) {
+      std::vector<int>& L = lists[sh][p];
+      I.ntiles[p] = (int)batch_tiles(b, I.G, sh, p);
+      I.tile0[p] = (int)L.size();
+      if (!include || (*include)[i]) L.insert(L.end(), (size_t)I.ntiles[p], i);
     }
-    I.tile0 = (int)lists[sh].size();
-    lists[sh].insert(lists[sh].end(), (size_t)I.ntiles, i);
   }
-  for (int g = 0; g < N_BATCH_SHAPES; ++g) {
-    b->group_tiles[g] = (int)lists[g].size();
-    if (!lists[g].empty())
-      CK(cudaMemcpyAsync(b->d_tile_inst[g], lists[g].data(), sizeof(int) * lists[g].size(), cudaMemcpyHostToDevice,
-                         b->stream));
-  }
+  for (int g = 0; g < N_BATCH_SHAPES; ++g)
+    for (int p = 0; p < 2; ++p) {
+      b->group_tiles[g][p] = (int)lists[g][p].size();
+      if (!lists[g][p].empty())
+        CK(cudaMemcpyAsync(b->d_tile_inst[g][p], lists[g][p].data(), sizeof(int) * lists[g][p].size(),
+                           cudaMemcpyHostToDevice, b->stream));
+    }
   CK(cudaMemcpyAsync(b->d_insts, b->h_insts.data(), sizeof(BatchInst) * b->n, cudaMemcpyHostToDevice, b->stream));
   CK(cudaStreamSynchronize(b->stream));
   return SS_OK;
@@ -1722,7 +1673,9 @@ int ss_batch_create(int theory, int n_lattices, const int32_t* p_i, int n_i, con
       return fail(rc, "lattice %d: %s", i, msg);
     }
     // partials and tile lists are sized for the finest shape the precision may use
-    const long long t = std::max(batch_tiles(h.G, 0), precision == SS_FP32 ? batch_tiles(h.G, 1) : 0LL);
+    long long t = 0;
+    for (int sh = 0; sh < (precision == SS_FP32 ? N_BATCH_SHAPES : 1); ++sh)
+      for (int p = 0; p < 2; ++p) t = std::max(t, batch_tiles(b, h.G, sh, p));
     b->max_tiles.push_back((int)std::min(t, 0x7fffffffLL));
     total += t;
   }

@@ -89,6 +89,15 @@ __device__ inline Dual<K>& operator-=(Dual<K>& a, const Dual<K>& b) { a = a - b;
 template <int K>
 __device__ inline Dual<K>& operator-=(Dual<K>& a, double s) { a.v -= s; return a; }
 
+template <int K>
+__device__ inline Dual<K> vfma(const Dual<K>& a, const Dual<K>& b, const Dual<K>& c) {
+  Dual<K> r;
+  r.v = fma(a.v, b.v, c.v);
+#pragma unroll
+  for (int k = 0; k < K; ++k) r.d[k] = fma(a.d[k], b.v, fma(a.v, b.d[k], c.d[k]));
+  return r;
+}
+
 // Pass 1: de/df_a into grad (nf planes of N) and mask x de/d(dx_a), mask x de/d(dy_a)
 // into q (2 nf planes of N: x planes, then y planes).  Jets: FP64 difference-form
 // stencils of the stored values (as the energy observable), masked like the reference.

@@ -1,28 +1,6 @@
-// flow.cuh -- fused single-pass-per-stage kernels of the arrested-Newton-flow step.
-//
-// One RK4 step of the reference (core/integrator.py:217-348) is
-//   k1 = dt V,            T1 = phi,           l1 = -dt G(T1)
-//   k2 = dt (V + l1/2),   T2 = phi + k1/2,    l2 = -dt G(T2)
-//   k3 = dt (V + l2/2),   T3 = phi + k2/2,    l3 = -dt G(T3)
-//   k4 = dt (V + l3),     T4 = phi + k3,      l4 = -dt G(T4)
-//   V' = V + (l1 + 2 l2 + 2 l3 + l4)/6,  phi' = phi + (k1 + 2 k2 + 2 k3 + k4)/6
-// followed by the unit-norm re-projection, the energy of phi', the arrest test
-// (E' > E -> V' = 0) and err = max G(T4).  The update is linear in V and the l_s, so
-// everything stage 4 needs besides l4 is known once l2 and l3 are:
-//   T4 = phi + dt (V + l2/2),  cV = V + (l1 + 2 l2 + 2 l3)/6,  cP = phi + dt V + dt (l1 + l2 + l3)/6
-//   V' = cV + l4/6,            phi' = cP (re-projected)
-// Stage s recomputes its T_s from (phi, V, l_s) while a tile is staged:
-//   S1  reads phi                        writes l1  (+ energy of phi, see below)
-//   S2  reads phi, V                     writes l2
-//   S3  reads phi, V, l1 (+ l2 centres)  writes T4, cV, cP
-//   S4  reads T4 (halo tile), cP, cV     writes phi', V', err
-// Stage 4 reads neither phi nor V, so it writes the caller's buffers in place (no
-// ping-pong copies).  The energy of a step's result is computed by the NEXT step's S1,
-// which stages exactly that field anyway, and the arrest decision is kept on the
-// device (StepState.arrest) and applied by S2/S3 as "V = 0".  A trailing energy pass
-// closes a call.  Compulsory traffic: 13 words per site and step when stages 2 and 3
-// run as one kernel (M_S23: S1 2, S2+S3 6, S4 5), 17 as four kernels (S2 3, S3 7 with
-// the l2 centres).
+// flow.cuh -- tiles, stencils and single-pass kernels over a lattice: the gradient hook, the
+// exact FP64 energy of the stored values, densities, charges and coupling partials, and the
+// reference's RK4 building blocks.  The flow's own step is in rk.cuh, on the same tiles.
 #pragma once
 
 #include <cuda.h>
@@ -33,7 +11,8 @@
 
 namespace ssb {
 
-// M_S23: stages 2 and 3 fused (one staging of phi, V, l1; writes l2 and l3)
+// Modes of flow_kernel (M_GRAD, M_ENERGY) and indices of the staging variants: M_S1, M_S2 the
+// step's phase A, M_S3, M_S4 its phase B, M_S23 kept for the pinning interface.
 enum FlowMode { M_GRAD = 0, M_S1 = 1, M_S2 = 2, M_S3 = 3, M_S4 = 4, M_ENERGY = 5, M_S23 = 6 };
 constexpr int N_FLOW_MODES = 7;
 enum { ST_TIMEOUT = 6 };
@@ -45,39 +24,14 @@ constexpr long long WAIT_CYCLES = 2000000000LL;
 
 template <typename R>
 struct FlowArgs {
-  CUtensorMap tm_phi;  // TMA maps (used when the kernel is instantiated with TMA):
-  CUtensorMap tm_vel;  //   halo boxes of the staged field (phi; T4 in S4), of V,
-  CUtensorMap tm_l;    //   of l1 (S3, M_S23),
-  CUtensorMap tm_cp;   //   and centre boxes of cP and cV (pipelined S4)
-  CUtensorMap tm_cv;
-  const R* phi;  // the staged field: phi, or T4 in S4
-  const R* vel;  // V (S2, S3, M_S23)
-  const R* la;   // l1 (S3, M_S23)
-  const R* lb;   // l2 (S3)
-  const R* cp;   // S4: cP = phi + dt V + dt (l1 + l2 + l3)/6
-  const R* cv;   // S4: cV = V + (l1 + 2 l2 + 2 l3)/6
-  R* out_l;      // S1, S2: l_s;  M_GRAD: l_out (nullable)
-  R* out_t4;     // S3 / M_S23: T4 = phi + dt (V + l2/2)
-  R* out_cp;     // S3 / M_S23: cP
-  R* out_cv;     // S3 / M_S23: cV
-  R* out_eg;     // M_GRAD: energy gradient (nullable)
-  R* phi_out;    // S4: phi' (may be the caller's phi: stage 4 reads neither phi nor V)
-  R* vel_out;    // S4: V'
-  const double* force;  // FP64 fields (nullable): added to the flow's gradient rows in every stage
-  double* partial;  // per-block energy partials
+  CUtensorMap tm_phi;  // TMA map of the field (used when the kernel is instantiated with TMA)
+  const R* phi;        // the staged field
+  R* out_l;            // M_GRAD: l_out (nullable)
+  R* out_eg;           // M_GRAD: energy gradient (nullable)
+  double* partial;     // per-block energy partials
   StepState* st;
-  double* E_traj;   // nullable
-  double* err_traj; // nullable
-  int E_idx;        // slot of E_traj the energy goes to (< 0: none)
-  int err_idx;      // slot of err_traj the S4 error goes to (< 0: none)
   int mode;
-  int with_energy;    // S1 / M_ENERGY: reduce the energy of the staged field
-  int arrest_update;  // after the energy: arrest = killkinen && E > E_last; E_last = E
-  int init_state;     // first S1 of a call: arrest = 0 and (unless NaN) E_last = prev_energy
-  double prev_energy;
   int grad_raw;           // M_GRAD: unprojected, not halo-zeroed dE/dphi with true saddle rows
-  int exact_energy;       // M_ENERGY on FP32 fields: 1 = FP64 stencil of the stored values
-                          // (observables), 0 = from the FP32 jets like stage 1 (flow energies)
   long long wait_cycles;  // bound of every mbarrier wait (clock64 cycles)
   unsigned tx_extra;      // test hook: bytes the barrier expects beyond what is loaded (normally 0)
   Grid G;
@@ -100,11 +54,6 @@ struct TileShape {
 template <typename R, int NF, int TX, int TY>
 __host__ __device__ constexpr size_t tile_buf_bytes() {
   return sizeof(R) * NF * (TX + 4) * (TY + 8);
-}
-
-// number of staged halo buffers a mode needs (phi, then V, then l1; T4 alone in S4)
-__host__ __device__ constexpr int flow_buffers(int mode) {
-  return mode == M_S2 ? 2 : (mode == M_S3 || mode == M_S23) ? 3 : 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -147,27 +96,26 @@ __device__ inline bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, long lo
   return true;
 }
 
-// T_s for one element from the staged inputs (the reference's k / Temp algebra,
-// core/integrator.py:51-96 and :323-334); stage 4's T4 is stored by stage 3
+// T2 = phi + k1/2 and T3 = phi + k2/2 of one element, rounded as the reference's k / Temp
+// algebra (core/integrator.py:51-96 and :323-334): used by plain-load staging
 template <typename R>
-__device__ inline R stage_value(int mode, R p, R v, R w, R dt) {
+__device__ inline R stage_t2(R p, R v, R dt) {
+  return p + (R)0.5 * (dt * v);
+}
+template <typename R>
+__device__ inline R stage_t3(R p, R v, R l1, R dt) {
   const R half = (R)0.5;
-  if (mode == M_S2) return p + half * (dt * v);
-  if (mode == M_S3) return p + half * (dt * (v + half * w));
-  return p;
+  return p + half * (dt * (v + half * l1));
 }
 
-// Plain-load staging of one halo buffer T = T_s(psrc, vsrc, wsrc) (all components;
-// vsrc / wsrc nullable), used when a TMA map cannot describe the buffers (row pitch
-// not a multiple of 16 bytes).  Every thread first issues all loads of one component
-// plane, then combines and stores, so each plane costs one memory round trip.
+// Plain-load staging of one field's halo buffer (all components), used when a TMA map cannot
+// describe the buffer (row pitch not a multiple of 16 bytes).  Every thread first issues all
+// loads of one component plane, then stores, so each plane costs one memory round trip.
 template <int NF, typename R, int TX, int TY, int NT>
-__device__ inline void stage_plain_buf(R* T, const Grid& G, const R* psrc, const R* vsrc, const R* wsrc, int x0,
-                                       int y0, int mode) {
+__device__ inline void stage_plain(R* T, const Grid& G, const R* src, int x0, int y0) {
   using TS = TileShape<TX, TY, NT>;
   constexpr int KM = (TS::PLANE + NT - 1) / NT;
   const long long N = G.N;
-  const R dt = (R)G.dt;
   long long off[KM];
   bool ok[KM];
 #pragma unroll
@@ -180,28 +128,15 @@ __device__ inline void stage_plain_buf(R* T, const Grid& G, const R* psrc, const
   }
 #pragma unroll
   for (int a = 0; a < NF; ++a) {
-    R p[KM], v[KM], w[KM];
-    const long long base = (long long)a * N;
+    R p[KM];
 #pragma unroll
-    for (int k = 0; k < KM; ++k) {
-      p[k] = ok[k] ? psrc[base + off[k]] : (R)0;
-      v[k] = (ok[k] && vsrc) ? vsrc[base + off[k]] : (R)0;
-      w[k] = (ok[k] && wsrc) ? wsrc[base + off[k]] : (R)0;
-    }
+    for (int k = 0; k < KM; ++k) p[k] = ok[k] ? src[(long long)a * N + off[k]] : (R)0;
 #pragma unroll
     for (int k = 0; k < KM; ++k) {
       const int i = threadIdx.x + k * NT;
-      if (i < TS::PLANE) T[a * TS::PLANE + i] = stage_value<R>(mode, p[k], v[k], w[k], dt);
+      if (i < TS::PLANE) T[a * TS::PLANE + i] = p[k];
     }
   }
-}
-
-// Plain-load staging of T_s into T (T4, stored by stage 3, in S4)
-template <int NF, typename R, int TX, int TY, int NT>
-__device__ inline void stage_plain(R* T, const FlowArgs<R>& A, int x0, int y0, int mode, bool arrest) {
-  const bool need_v = (mode == M_S2 || mode == M_S3) && !arrest;
-  stage_plain_buf<NF, R, TX, TY, NT>(T, A.G, A.phi, need_v ? A.vel : nullptr, mode == M_S3 ? A.la : nullptr, x0, y0,
-                                     mode);
 }
 
 // The unit-norm re-projection of a site pair's magnetisation components
@@ -384,43 +319,25 @@ __device__ __forceinline__ void flow_constraints(const Grid& G, const Jet<V, TH:
   }
 }
 
-// The per-site work of one staged tile.  Each thread owns y-adjacent site pairs;
-// FAST: the tile is interior (every derivative mask true, no halo site) and the
-// lattice row length is even, so pairs are aligned and need no lane masks.
-//   T      the staged stencil field: T1 (S1, M_GRAD, M_ENERGY), T2 (S2), T3 (S3, M_S23), T4 (S4)
-//   T2     M_S23: the staged T2 (l2 and l3 of a pair are computed in one pass)
-//   Praw   S3 / M_S23: the staged phi (else phi is read from A.phi)
-//   Vraw   S3: the staged V (else V is read from A.vel); unused when arrested
-//   Cp, Cv S4: the staged cP and cV centre tiles (else read from A.cp, A.cv)
-// JE (FP32 stage 1 and the energy pass): add the energy of the jets to *e_acc (when
-// non-null); in M_ENERGY the gradient itself is skipped.
-template <class TH, typename R, int TX, int TY, int NT, bool FAST, int MODE, bool JE = false>
-__device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int x0, int y0, bool arrest,
-                                          double& err_max, double* e_acc = nullptr, const R* Praw = nullptr,
-                                          const R* Vraw = nullptr, const R* T2 = nullptr, const R* Cp = nullptr,
-                                          const R* Cv = nullptr, R* out_l = nullptr) {
+// The gradient hook on one staged tile.  Each thread owns y-adjacent site pairs; FAST: the
+// tile is interior (every derivative mask true, no halo site) and the lattice row length is
+// even, so pairs are aligned and need no lane masks.
+template <class TH, typename R, int TX, int TY, int NT, bool FAST>
+__device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int x0, int y0) {
   using TS = TileShape<TX, TY, NT>;
   using V = typename PairOf<R>::type;
-  constexpr int NF = TH::NF;
-  constexpr int PAIRS = TY / 2;
-  constexpr int RPP = NT / PAIRS;
-  static_assert(NT % PAIRS == 0 && TX % RPP == 0, "pair mapping");
   using S = typename ScalarOf<V>::type;
+  constexpr int NF = TH::NF, PAIRS = TY / 2, RPP = NT / PAIRS;
+  static_assert(NT % PAIRS == 0 && TX % RPP == 0, "pair mapping");
   const Grid& G = A.G;
   const long long N = G.N;
   const PairCoef<V> kc(G);
   const V mdt(grid_k<S>(G, GK_MDT));
-  S emax = -INFINITY;
-  V chk(0.0);
-  double e_pair = 0.0;
   const int j = threadIdx.x % PAIRS;
   const int lxg = threadIdx.x / PAIRS;
-  // stage 1 and the FP32 energy pass give each thread adjacent rows; the energy pass
-  // unrolls them so that the rows share their x-neighbour loads
-  constexpr bool ADJ = sizeof(R) == 4 && (MODE == M_S1 || MODE == M_ENERGY);
-#pragma unroll((JE && MODE == M_ENERGY) ? 2 : 1)
+#pragma unroll 1
   for (int pass = 0; pass < TX / RPP; ++pass) {
-    const int lx = ADJ ? lxg * (TX / RPP) + pass : lxg + pass * RPP;
+    const int lx = lxg + pass * RPP;
     const int gx = x0 + lx, gy = y0 + 2 * j;
     bool v1 = true;
     Masks m0{true, true, true}, m1{true, true, true};
@@ -433,162 +350,26 @@ __device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int 
     }
     const int toff = (lx + 2) * TS::HY + TS::YOFF + 2 * j;
     const long long sidx = (long long)gx * G.Y + gy;
-    // M_S23: the pair's V and l1 (overwritten by T2 and T3 in shared memory) come back
-    // from L2; issued before the two stencils so that their latency hides behind them
-    // (FP32, up to four components: the six of the s+id model, and FP64 pairs, would spill)
-    constexpr bool PRE = MODE == M_S23 && NF <= 4 && sizeof(R) == 4;
-    constexpr int NPRE = PRE ? NF : 1;
-    V pre_v[NPRE], pre_l1[NPRE];
-    if constexpr (PRE) {
-#pragma unroll
-      for (int a = 0; a < NF; ++a) {
-        pre_v[a] = arrest ? V(0.0) : gload<V, R>(A.vel + a * N + sidx, FAST, v1);
-        pre_l1[a] = gload<V, R>(A.la + a * N + sidx, FAST, v1);
-      }
-    }
-    // S4 one tile per CTA (FP32, up to four components): cP and cV likewise, where they are
-    // not staged
-    constexpr bool PRE4 = MODE == M_S4 && sizeof(R) == 4 && NF <= 4;
-    V pre_cp[PRE4 ? NF : 1], pre_cv[PRE4 ? NF : 1];
-    if constexpr (PRE4) {
-#pragma unroll
-      for (int a = 0; a < NF; ++a) {
-        if (!Cp) pre_cp[a] = gload<V, R>(A.cp + a * N + sidx, FAST, v1);
-        if (!Cv) pre_cv[a] = gload<V, R>(A.cv + a * N + sidx, FAST, v1);
-      }
-    }
-
     Jet<V, NF> J;
     tile_jet<TH, V, R, TS::HY, TS::PLANE, FAST>(T, toff, kc, m0, m1, J);
-    if constexpr (JE) {
-      if (e_acc) {
-        if constexpr (TH::PAIR_ENERGY) {
-          // energy point in packed FP32; F2F keeps Inf/NaN
-          const V ep = TH::energy_pair(J, A.P);
-          e_pair += (double)Lanes<V>::get(ep, 0);
-          if (v1) e_pair += (double)Lanes<V>::get(ep, 1);
-        } else {
-          *e_acc += jet_energy<TH, V, NF>(J, A.P, G.dA, v1, chk);
-        }
-      }
-    }
-    if constexpr (MODE == M_ENERGY) continue;
-
-    // FP64 fields: a fixed field added to the flow's gradient rows (ss_set_forcing); uniform
-    auto add_force = [&](V* g) {
-      if constexpr (sizeof(R) == 8 && MODE != M_GRAD) {
-        if (A.force) {
-          V fo[NF];
-#pragma unroll
-          for (int a = 0; a < NF; ++a) fo[a] = gload<V, double>(A.force + a * N + sidx, FAST, v1);
-          TH::flow_rows(fo, A.P);
-#pragma unroll
-          for (int a = 0; a < NF; ++a) g[a] = g[a] + fo[a];
-        }
-      }
-    };
     V g[NF];
     TH::gradient(J, A.P, g);
-    add_force(g);
-    if constexpr (MODE == M_GRAD) {
-      if (A.grad_raw) {
-        // functional derivative of the energy: no halo zeroing, no projection, and
-        // rows the flow stores scaled (saddle fields) converted to dE/dphi
-        TH::true_rows(g, A.P);
-#pragma unroll
-        for (int a = 0; a < NF; ++a) {
-          if (A.out_eg) gstore<V, R>(A.out_eg + a * N + sidx, g[a], FAST, v1);
-        }
-        continue;
-      }
-    }
-    flow_constraints<TH, V, FAST>(G, J, g, gx, gy);
-    if constexpr (MODE == M_GRAD) {
+    if (A.grad_raw) {
+      // functional derivative of the energy: no halo zeroing, no projection, and rows the
+      // flow stores scaled (saddle fields) converted to dE/dphi
+      TH::true_rows(g, A.P);
 #pragma unroll
       for (int a = 0; a < NF; ++a) {
         if (A.out_eg) gstore<V, R>(A.out_eg + a * N + sidx, g[a], FAST, v1);
-        if (A.out_l) gstore<V, R>(A.out_l + a * N + sidx, mdt * g[a], FAST, v1);
       }
-    } else if constexpr (MODE == M_S1 || MODE == M_S2) {
-      R* const lo = out_l ? out_l : A.out_l;
-#pragma unroll
-      for (int a = 0; a < NF; ++a) gstore<V, R>(lo + a * N + sidx, mdt * g[a], FAST, v1);
-    } else if constexpr (MODE == M_S3 || MODE == M_S23) {
-      // l3 from T3; l2 from T2 (M_S23) or the stored l2 (S3); then the stage-4 inputs
-      // T4 = phi + dt (V + l2/2), cV = V + (l1 + 2 l2 + 2 l3)/6, cP = phi + dt V + dt (l1 + l2 + l3)/6
-      // (core/integrator.py:151-189 with k1 = dt V, k2 = dt (V + l1/2), k3 = dt (V + l2/2))
-      V l2[NF];
-      if constexpr (MODE == M_S23) {
-        Jet<V, NF> J2;
-        tile_jet<TH, V, R, TS::HY, TS::PLANE, FAST>(T2, toff, kc, m0, m1, J2);
-        TH::gradient(J2, A.P, l2);
-        add_force(l2);
-        flow_constraints<TH, V, FAST>(G, J2, l2, gx, gy);
-#pragma unroll
-        for (int a = 0; a < NF; ++a) l2[a] = mdt * l2[a];
-      } else {
-#pragma unroll
-        for (int a = 0; a < NF; ++a) l2[a] = gload<V, R>(A.lb + a * N + sidx, FAST, v1);
-      }
-      const V half(0.5), sixth(grid_k<S>(G, GK_SIXTH)), two(2.0), dtv(grid_k<S>(G, GK_DT)),
-          dt6(grid_k<S>(G, GK_DT6));
-#pragma unroll
-      for (int a = 0; a < NF; ++a) {
-        const long long idx = a * N + sidx;
-        const V p = Praw ? ld_pair(Praw + a * TS::PLANE + toff) : gload<V, R>(A.phi + idx, FAST, v1);
-        V v, l1;
-        if constexpr (PRE) {
-          v = pre_v[a];
-          l1 = pre_l1[a];
-        } else {
-          v = arrest ? V(0.0) : (Vraw ? ld_pair(Vraw + a * TS::PLANE + toff) : gload<V, R>(A.vel + idx, FAST, v1));
-          l1 = gload<V, R>(A.la + idx, FAST, v1);
-        }
-        const V l3 = mdt * g[a];
-        gstore<V, R>(A.out_t4 + idx, vfma(dtv, vfma(half, l2[a], v), p), FAST, v1);
-        gstore<V, R>(A.out_cv + idx, vfma(sixth, vfma(two, l3, vfma(two, l2[a], l1)), v), FAST, v1);
-        gstore<V, R>(A.out_cp + idx, vfma(dt6, (l1 + l2[a]) + l3, vfma(dtv, v, p)), FAST, v1);
-      }
-    } else {
-      // S4: V' = cV + l4/6 and phi' = cP, re-projected onto the sphere, then V' projected
-      // onto the tangent space of phi' (compute_norm_magnetization and
-      // project_orthogonal_magnetization, chiral_magnet/kernels.py:48-122)
-      V Pn[NF], Vn[NF];
-      const V sixth(grid_k<S>(G, GK_SIXTH));
-#pragma unroll
-      for (int a = 0; a < NF; ++a) {
-        const int coff = a * TX * TY + lx * TY + 2 * j;
-        V cv;
-        if constexpr (PRE4) {
-          cv = Cv ? ld_pair(Cv + coff) : pre_cv[a];
-          Pn[a] = Cp ? ld_pair(Cp + coff) : pre_cp[a];
-        } else {
-          cv = Cv ? ld_pair(Cv + coff) : gload<V, R>(A.cv + a * N + sidx, FAST, v1);
-          Pn[a] = Cp ? ld_pair(Cp + coff) : gload<V, R>(A.cp + a * N + sidx, FAST, v1);
-        }
-        Vn[a] = vfma(sixth, mdt * g[a], cv);
-        emax = fmax(emax, Lanes<V>::get(g[a], 0));
-        if (v1) emax = fmax(emax, Lanes<V>::get(g[a], 1));
-      }
-      if (TH::CONSTRAINED && G.unit_mag) {
-        unit_project<TH::NMAG>(Pn);
-        V lm = Vn[0] * Pn[0];
-#pragma unroll
-        for (int a = 1; a < TH::NMAG; ++a) lm = vfma(Vn[a], Pn[a], lm);
-        const V mlm = -lm;
-#pragma unroll
-        for (int a = 0; a < TH::NMAG; ++a) Vn[a] = vfma(mlm, Pn[a], Vn[a]);
-      }
-#pragma unroll
-      for (int a = 0; a < NF; ++a) {
-        gstore<V, R>(A.phi_out + a * N + sidx, Pn[a], FAST, v1);
-        gstore<V, R>(A.vel_out + a * N + sidx, Vn[a], FAST, v1);
-      }
+      continue;
     }
-  }
-  if (MODE == M_S4) err_max = fmax(err_max, (double)emax);
-  if constexpr (JE) {
-    if (e_acc) *e_acc += e_pair * G.dA + (double)(Lanes<V>::get(chk, 0) + Lanes<V>::get(chk, 1));
+    flow_constraints<TH, V, FAST>(G, J, g, gx, gy);
+#pragma unroll
+    for (int a = 0; a < NF; ++a) {
+      if (A.out_eg) gstore<V, R>(A.out_eg + a * N + sidx, g[a], FAST, v1);
+      if (A.out_l) gstore<V, R>(A.out_l + a * N + sidx, mdt * g[a], FAST, v1);
+    }
   }
 }
 
@@ -652,25 +433,7 @@ __device__ __forceinline__ double energy_tile(const FlowArgs<R>& A, const E* T, 
   return e_acc + (double)(Lanes<V>::get(chk, 0) + Lanes<V>::get(chk, 1));
 }
 
-// Expect and issue the TMA loads of one tile's staged halo buffers (called by one
-// thread, after the barrier is initialised): tm_phi into B0 (phi; T4 in S4), then V
-// into B0 + BUF in S2, S3 and M_S23 and l1 into B0 + 2 BUF in S3 and M_S23.  V is
-// staged whether or not an arrest is pending (an arrested step ignores it).
-template <class TH, typename R, int TX, int TY, int NT, int MODE>
-__device__ __forceinline__ void issue_tile(R* B0, const CUtensorMap* tm_phi, const CUtensorMap* tm_vel,
-                                           const CUtensorMap* tm_l, int x0, int y0, uint64_t* bar,
-                                           unsigned tx_extra) {
-  using TS = TileShape<TX, TY, NT>;
-  constexpr int BUF = TH::NF * TS::PLANE;
-  constexpr int NB = flow_buffers(MODE);
-  constexpr uint32_t bytes = (uint32_t)(sizeof(R) * BUF) * (uint32_t)NB;
-  mbar_expect_tx(bar, bytes + tx_extra);
-  tma_load_3d(B0, tm_phi, y0 - TS::YOFF, x0 - 2, 0, bar);
-  if constexpr (NB >= 2) tma_load_3d(B0 + BUF, tm_vel, y0 - TS::YOFF, x0 - 2, 0, bar);
-  if constexpr (NB >= 3) tma_load_3d(B0 + 2 * BUF, tm_l, y0 - TS::YOFF, x0 - 2, 0, bar);
-}
-
-// Shared scratch of the one-tile-per-CTA stage kernels besides the staged tile.
+// Shared scratch of the tile kernels besides the staged tile.
 template <int NT>
 struct StageShared {
   double red[NT / 32];
@@ -679,147 +442,13 @@ struct StageShared {
   int am_last;
 };
 
-// Stage, compute and reduce tile `tile` of a lattice of `nblk` tiles (one CTA per
-// tile).  tm_phi / tm_vel / tm_l are TMA maps in parameter or global memory.
-// issued: thread 0 has already initialised S.bar and issued the tile's loads
-// (issue_tile), so the caller's set-up overlapped them.
-template <class TH, typename R, int TX, int TY, int NT, bool TMA, int MODE>
-__device__ __forceinline__ void flow_tile(const FlowArgs<R>& A, const CUtensorMap* tm_phi, const CUtensorMap* tm_vel,
-                                          const CUtensorMap* tm_l, int tile, int nblk, unsigned char* smem_raw,
-                                          StageShared<NT>& S, bool issued = false) {
-  using TS = TileShape<TX, TY, NT>;
-  constexpr int NF = TH::NF;
-  constexpr int BUF = NF * TS::PLANE;
-  R* B0 = reinterpret_cast<R*>(smem_raw);
-  R* B1 = B0 + BUF;
-  R* B2 = B1 + BUF;
-  double* red = S.red;
-  double* sh_s = S.sh_s;
-  double* sh_c = S.sh_c;
-  uint64_t& bar = S.bar;
-  int& am_last = S.am_last;
-
-  const Grid& G = A.G;
-  const int tiles_y = (G.Y + TY - 1) / TY;
-  const int x0 = (tile / tiles_y) * TX;
-  const int y0 = (tile % tiles_y) * TY;
-  StepState* st = A.st;
-  constexpr bool uses_v = MODE == M_S2 || MODE == M_S3 || MODE == M_S23;
-  // The arrest flag (set by the last block of stage 1) is read only after the TMA
-  // copies are issued, so its global-memory round trip overlaps them.
-  bool arrest = false;
-  const bool do_energy = (MODE == M_S1 || MODE == M_ENERGY) && A.with_energy != 0;
-
-  if (A.init_state && tile == 0 && threadIdx.x == 0) {
-    st->arrest = 0;
-    if (!isnan(A.prev_energy)) st->E_last = A.prev_energy;
-  }
-
-  // ---- stage the halo tiles --------------------------------------------
-  R* T = B0;
-  if constexpr (TMA) {
-    if (!issued) {
-      if (threadIdx.x == 0) mbar_init(&bar, 1);
-      __syncthreads();
-      if (threadIdx.x == 0) issue_tile<TH, R, TX, TY, NT, MODE>(B0, tm_phi, tm_vel, tm_l, x0, y0, &bar, A.tx_extra);
-    }
-    if constexpr (uses_v) arrest = st->arrest != 0;
-    const bool ok = __syncthreads_and(mbar_wait_bounded(&bar, 0, A.wait_cycles));
-    if (!ok) {
-      if (threadIdx.x == 0) atomicExch(&st->status, (int)ST_TIMEOUT);
-      mbar_wait_bounded(&bar, 0, A.wait_cycles);
-      return;
-    }
-    using V = typename PairOf<R>::type;
-    const V half(0.5), hdt(grid_k<R>(G, GK_HDT));
-    if constexpr (MODE == M_S23) {
-      // T3 = phi + dt/2 (V + l1/2) in place of l1 and T2 = phi + dt/2 V in place of V, in
-      // one pass (each element reads its own phi, V, l1 before writing)
-      for (int i = 4 * threadIdx.x; i < BUF; i += 4 * NT) {
-        V p0, p1, v0(0.0), v1(0.0), w0, w1;
-        ld_quad(B0 + i, p0, p1);
-        if (!arrest) ld_quad(B1 + i, v0, v1);
-        ld_quad(B2 + i, w0, w1);
-        st_quad(B2 + i, vfma(hdt, vfma(half, w0, v0), p0), vfma(hdt, vfma(half, w1, v1), p1));
-        st_quad(B1 + i, vfma(hdt, v0, p0), vfma(hdt, v1, p1));
-      }
-      __syncthreads();
-    } else if constexpr (MODE == M_S2 || MODE == M_S3) {
-      // T2 in place of V, or T3 in place of l1 (OOB entries are zero in all)
-      R* dst = MODE == M_S3 ? B2 : B1;
-      for (int i = 4 * threadIdx.x; i < BUF; i += 4 * NT) {
-        V p0, p1, v0(0.0), v1(0.0), w0(0.0), w1(0.0);
-        ld_quad(B0 + i, p0, p1);
-        if (!arrest) ld_quad(B1 + i, v0, v1);
-        if (MODE == M_S3) ld_quad(B2 + i, w0, w1);
-        if (MODE == M_S2)
-          st_quad(dst + i, vfma(hdt, v0, p0), vfma(hdt, v1, p1));
-        else
-          st_quad(dst + i, vfma(hdt, vfma(half, w0, v0), p0), vfma(hdt, vfma(half, w1, v1), p1));
-      }
-      __syncthreads();
-      T = dst;
-    }
-  } else {
-    if constexpr (uses_v) arrest = st->arrest != 0;
-    stage_plain<NF, R, TX, TY, NT>(B0, A, x0, y0, MODE, arrest);
-    __syncthreads();
-  }
-
-  double e_acc = 0.0;
-  double err_max = -INFINITY;
-  const bool fast = (G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
-                    y0 + TY - 1 <= G.Y - G.halo - 2;
-  if constexpr (MODE == M_S23) {
-    // l3 from T3 (staged in B2) and l2 from T2 (staged in B1) per site pair, then the
-    // stage-4 inputs: the stage-2 and stage-3 arithmetic, so the results equal the two
-    // separate stages bitwise
-    if (fast)
-      grad_tile<TH, R, TX, TY, NT, true, M_S23>(A, B2, x0, y0, arrest, err_max, nullptr, B0, nullptr, B1);
-    else
-      grad_tile<TH, R, TX, TY, NT, false, M_S23>(A, B2, x0, y0, arrest, err_max, nullptr, B0, nullptr, B1);
-    return;
-  } else if constexpr (MODE == M_S1 || MODE == M_ENERGY) {
-    // FP32 fields: the flow energy from the stencil's jets (stage 1 and the trailing
-    // pass), or (observables) the exact FP64 differences of the stored values; FP64
-    // fields: the exact differences
-    constexpr bool JE = sizeof(R) == 4;
-    const bool je = JE && !(MODE == M_ENERGY && A.exact_energy);
-    double* ep = (je && do_energy) ? &e_acc : nullptr;
-    if (MODE == M_S1 || je) {
-      if (fast)
-        grad_tile<TH, R, TX, TY, NT, true, MODE, JE>(A, T, x0, y0, false, err_max, ep);
-      else
-        grad_tile<TH, R, TX, TY, NT, false, MODE, JE>(A, T, x0, y0, false, err_max, ep);
-    }
-    if (do_energy && !je) {
-      if (fast)
-        e_acc = energy_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
-      else
-        e_acc = energy_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
-    }
-  } else {
-    // S2, S3, S4, M_GRAD; stage 3 combines with the staged phi and V (TMA staging)
-    const R* Praw = (TMA && MODE == M_S3) ? B0 : nullptr;
-    const R* Vraw = (TMA && MODE == M_S3) ? B1 : nullptr;
-    if (fast)
-      grad_tile<TH, R, TX, TY, NT, true, MODE>(A, T, x0, y0, arrest, err_max, nullptr, Praw, Vraw);
-    else
-      grad_tile<TH, R, TX, TY, NT, false, MODE>(A, T, x0, y0, arrest, err_max, nullptr, Praw, Vraw);
-  }
-
-  // ---- reductions -------------------------------------------------------
-  const bool need_ticket = do_energy || MODE == M_S4;
-  if (!need_ticket) return;
-  if (do_energy) {
-    const double bs = block_sum_fixed<NT>(e_acc, red);
-    if (threadIdx.x == 0) A.partial[tile] = bs;
-  }
-  if (MODE == M_S4) {
-    const double bm = block_max<NT>(err_max, red);
-    if (threadIdx.x == 0 && bm > -INFINITY) atomicMax(&st->err_enc, enc_max(bm));
-  }
+// The sum of the blocks' energy partials by the last of `nblk` blocks (fixed order).
+template <int NT>
+__device__ __forceinline__ void energy_reduction(double e_acc, double* partial, StepState* st, int blk, int nblk,
+                                                 double* red, double* sh_s, double* sh_c, int& am_last) {
+  const double bs = block_sum_fixed<NT>(e_acc, red);
   if (threadIdx.x == 0) {
+    partial[blk] = bs;
     __threadfence();
     const unsigned t = atomicAdd(&st->ticket, 1u);
     am_last = (t == (unsigned)nblk - 1u);
@@ -827,142 +456,95 @@ __device__ __forceinline__ void flow_tile(const FlowArgs<R>& A, const CUtensorMa
   __syncthreads();
   if (!am_last) return;
   __threadfence();
-  if (do_energy) {
-    const double E = fixed_order_sum<NT>(A.partial, nblk, sh_s, sh_c);
-    if (threadIdx.x == 0) {
-      st->scalar = E;
-      if (!isfinite(E)) st->status = 3;
-      if (A.E_traj && A.E_idx >= 0) A.E_traj[A.E_idx] = E;
-      if (A.arrest_update) {
-        st->arrest = (G.killkinen && E > st->E_last) ? 1 : 0;
-        st->E_last = E;
-      }
-    }
-  }
+  const double E = fixed_order_sum<NT>(partial, nblk, sh_s, sh_c);
   if (threadIdx.x == 0) {
-    if (MODE == M_S4) {
-      const double err = dec_max(atomicExch(&st->err_enc, 0ULL));
-      if (A.err_traj && A.err_idx >= 0) A.err_traj[A.err_idx] = err;
-    }
+    st->scalar = E;
+    if (!isfinite(E)) st->status = 3;
     st->ticket = 0u;
   }
 }
 
-// Resident CTAs per SM a one-tile-per-CTA stage kernel is built for (the staging latency
-// of a tile is hidden only by other resident CTAs).  The fused FP32 stages 2+3 evaluate
-// two stencils per site pair: capped at three 256-thread CTAs (80 registers) for the
-// theories with up to four components and at two (128 registers; its 104 KB of staging
-// fits two anyway) for the six-component s+id.  FP64 stages 1 and 4 and the energy pass
-// (one staged buffer each) at two 256-thread CTAs, 128 registers, up to four components
-// (the s+id would spill ~380 bytes).  No bound otherwise.
-template <class TH, typename R, int MODE, int NT>
-__host__ __device__ constexpr int flow_min_ctas() {
-  if (NT != 256) return 1;
-  if (sizeof(R) == 4 && MODE == M_S23) return TH::NF <= 4 ? 3 : 2;
-  if (sizeof(R) == 8 && (MODE == M_S4 || MODE == M_S1 || MODE == M_ENERGY)) return TH::NF <= 4 ? 2 : 1;
-  return 1;
+template <class TH, typename R, int TX, int TY, int NT, int MODE>
+__device__ __forceinline__ void flow_compute(const FlowArgs<R>& A, const R* T, int x0, int y0, double& e_acc) {
+  const Grid& G = A.G;
+  const bool fast = (G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
+                    y0 + TY - 1 <= G.Y - G.halo - 2;
+  if constexpr (MODE == M_ENERGY) {
+    if (fast)
+      e_acc += energy_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
+    else
+      e_acc += energy_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
+  } else {
+    if (fast)
+      grad_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
+    else
+      grad_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
+  }
 }
 
+// One tile per CTA: the gradient hook (M_GRAD) or the exact energy (M_ENERGY).
 template <class TH, typename R, int TX, int TY, int NT, bool TMA, int MODE>
-__global__ void __launch_bounds__(NT, (flow_min_ctas<TH, R, MODE, NT>()))
+__global__ void __launch_bounds__(NT, (sizeof(R) == 8 && MODE == M_ENERGY && TH::NF <= 4 ? 2 : 1))
     flow_kernel(const __grid_constant__ FlowArgs<R> A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ StageShared<NT> S;
-  flow_tile<TH, R, TX, TY, NT, TMA, MODE>(A, &A.tm_phi, &A.tm_vel, &A.tm_l, blockIdx.x, gridDim.x, smem_raw, S);
+  R* T = reinterpret_cast<R*>(smem_raw);
+  const int tiles_y = (A.G.Y + TY - 1) / TY;
+  const int x0 = (blockIdx.x / tiles_y) * TX, y0 = (blockIdx.x % tiles_y) * TY;
+  if constexpr (TMA) {
+    using TS = TileShape<TX, TY, NT>;
+    if (threadIdx.x == 0) {
+      mbar_init(&S.bar, 1);
+      mbar_expect_tx(&S.bar, (uint32_t)(sizeof(R) * TH::NF * TS::PLANE) + A.tx_extra);
+      tma_load_3d(T, &A.tm_phi, y0 - TS::YOFF, x0 - 2, 0, &S.bar);
+    }
+    __syncthreads();
+    const bool ok = __syncthreads_and(mbar_wait_bounded(&S.bar, 0, A.wait_cycles));
+    if (!ok) {
+      if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
+      mbar_wait_bounded(&S.bar, 0, A.wait_cycles);
+      return;
+    }
+  } else {
+    stage_plain<TH::NF, R, TX, TY, NT>(T, A.G, A.phi, x0, y0);
+    __syncthreads();
+  }
+  double e_acc = 0.0;
+  flow_compute<TH, R, TX, TY, NT, MODE>(A, T, x0, y0, e_acc);
+  if constexpr (MODE == M_ENERGY)
+    energy_reduction<NT>(e_acc, A.partial, A.st, blockIdx.x, gridDim.x, S.red, S.sh_s, S.sh_c, S.am_last);
 }
 
-// ---------------------------------------------------------------------------
-// Persistent, TMA-pipelined form of flow_kernel (FP32 fields): one CTA per SM
+// Persistent, TMA-pipelined form of flow_kernel (FP32 fields): one 512-thread CTA per SM
 // walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ... through a ring of STAGES
-// shared-memory slots, so the bulk tensor loads of the next tiles are in flight
-// while the current tile is computed.  Stage 4 also stages the centre tiles of cP and cV.
-// Energy partials are per CTA in tile order (deterministic for a fixed grid).
-// ---------------------------------------------------------------------------
-template <int MODE>
-__host__ __device__ constexpr int pipe_halo_buffers() {
-  return flow_buffers(MODE);
-}
-template <int MODE>
-__host__ __device__ constexpr int pipe_centre_buffers() {
-  return MODE == M_S4 ? 2 : 0;
-}
-template <typename R, int NF, int TX, int TY, int MODE>
-__host__ __device__ constexpr size_t pipe_slot_bytes() {
-  return tile_buf_bytes<R, NF, TX, TY>() * pipe_halo_buffers<MODE>() +
-         sizeof(R) * NF * TX * TY * pipe_centre_buffers<MODE>();
-}
-
-// Persistent CTAs per SM: for stage 1 and the energy pass the theory's S1_CTAS (four
-// 256-thread CTAs for the light chiral stencil, issue-bound: two site pairs per thread
-// per tile halve the per-tile overhead, and four CTAs keep 32 warps per SM), one
-// 512-thread CTA otherwise.
-template <class TH, int MODE>
-__host__ __device__ constexpr int pipe_ctas() {
-  return (MODE == M_S1 || MODE == M_ENERGY) ? TH::S1_CTAS : 1;
-}
-template <class TH, int MODE>
-__host__ __device__ constexpr int pipe_threads() {
-  return pipe_ctas<TH, MODE>() == 4 ? 256 : 512;
-}
-
+// shared-memory slots, so the bulk tensor loads of the next tiles are in flight while the
+// current tile is computed.  Energy partials are per CTA in tile order.
 template <class TH, typename R, int TX, int TY, int NT, int MODE, int STAGES>
-__global__ void __launch_bounds__(NT, (pipe_ctas<TH, MODE>())) flow_kernel_pipe(const __grid_constant__ FlowArgs<R> A) {
+__global__ void __launch_bounds__(NT, 1) flow_kernel_pipe(const __grid_constant__ FlowArgs<R> A) {
   using TS = TileShape<TX, TY, NT>;
-  constexpr int NF = TH::NF;
-  constexpr int BUF = NF * TS::PLANE;             // elements of one halo buffer
-  constexpr int CBUF = NF * TX * TY;              // elements of one centre buffer
-  constexpr int SLOT = BUF * pipe_halo_buffers<MODE>() + CBUF * pipe_centre_buffers<MODE>();
-  static_assert(MODE != M_S23, "the fused stages 2+3 run one tile per CTA");
+  constexpr int SLOT = TH::NF * TS::PLANE;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* ring = reinterpret_cast<R*>(smem_raw);
-  __shared__ double red[NT / 32];
-  __shared__ double sh_s[NT / 32], sh_c[NT / 32];
-  __shared__ int am_last;
-  __shared__ int timed_out;
+  __shared__ StageShared<NT> S;
   __shared__ __align__(8) uint64_t full[STAGES];
-
   const Grid& G = A.G;
   const int tiles_y = (G.Y + TY - 1) / TY;
   const int ntiles = ((G.X + TX - 1) / TX) * tiles_y;
-  StepState* st = A.st;
-  const bool arrest = (MODE == M_S2 || MODE == M_S3) && (st->arrest != 0);
-  const bool do_energy = (MODE == M_S1 || MODE == M_ENERGY) && A.with_energy != 0;
-  // second halo buffer: V in S2 / S3 (not loaded when arrested)
-  const bool load_b1 = (MODE == M_S2 || MODE == M_S3) && !arrest;
-  constexpr bool load_b2 = MODE == M_S3;
-  const uint32_t bytes = (uint32_t)(sizeof(R) * (BUF * (1 + (load_b1 ? 1 : 0) + (load_b2 ? 1 : 0)) +
-                                                 CBUF * pipe_centre_buffers<MODE>()));
-
-  if (A.init_state && blockIdx.x == 0 && threadIdx.x == 0) {
-    st->arrest = 0;
-    if (!isnan(A.prev_energy)) st->E_last = A.prev_energy;
-  }
+  constexpr uint32_t bytes = (uint32_t)(sizeof(R) * SLOT);
   auto issue = [&](int slot, int tile) {
-    R* base = ring + slot * SLOT;
-    const int x0 = (tile / tiles_y) * TX, y0 = (tile % tiles_y) * TY;
     mbar_expect_tx(&full[slot], bytes + A.tx_extra);
-    tma_load_3d(base, &A.tm_phi, y0 - TS::YOFF, x0 - 2, 0, &full[slot]);
-    if (load_b1) tma_load_3d(base + BUF, &A.tm_vel, y0 - TS::YOFF, x0 - 2, 0, &full[slot]);
-    if (load_b2) tma_load_3d(base + 2 * BUF, &A.tm_l, y0 - TS::YOFF, x0 - 2, 0, &full[slot]);
-    if (MODE == M_S4) {
-      tma_load_3d(base + BUF, &A.tm_cp, y0, x0, 0, &full[slot]);
-      tma_load_3d(base + BUF + CBUF, &A.tm_cv, y0, x0, 0, &full[slot]);
-    }
+    tma_load_3d(ring + slot * SLOT, &A.tm_phi, (tile % tiles_y) * TY - TS::YOFF, (tile / tiles_y) * TX - 2, 0,
+                &full[slot]);
   };
   if (threadIdx.x == 0) {
-    timed_out = 0;
     for (int s = 0; s < STAGES; ++s) mbar_init(&full[s], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       const int t = blockIdx.x + s * gridDim.x;
       if (t < ntiles) issue(s, t);
     }
   }
-
+  __syncthreads();
   double e_acc = 0.0;
-  double err_max = -INFINITY;
   int k = 0;
   // tile coordinates advanced without a division per tile
   const int dq = gridDim.x / tiles_y, dr = gridDim.x % tiles_y;
@@ -973,7 +555,7 @@ __global__ void __launch_bounds__(NT, (pipe_ctas<TH, MODE>())) flow_kernel_pipe(
     const bool ok = __syncthreads_and(mbar_wait_bounded(&full[slot], parity, A.wait_cycles));
     if (!ok) {
       // record, then wait (bounded) for every load still in flight before leaving
-      if (threadIdx.x == 0) atomicExch(&st->status, (int)ST_TIMEOUT);
+      if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
       for (int s = 0; s < STAGES; ++s) {
         const int kk = k + s;
         if (blockIdx.x + kk * gridDim.x < ntiles)
@@ -981,75 +563,12 @@ __global__ void __launch_bounds__(NT, (pipe_ctas<TH, MODE>())) flow_kernel_pipe(
       }
       return;
     }
-    R* base = ring + slot * SLOT;
-    R* B0 = base;
-    R* B1 = base + BUF;
-    R* B2 = base + 2 * BUF;
-    const int x0 = tx * TX, y0 = ty * TY;
+    flow_compute<TH, R, TX, TY, NT, MODE>(A, ring + slot * SLOT, tx * TX, ty * TY, e_acc);
     tx += dq;
     ty += dr;
     if (ty >= tiles_y) {
       ty -= tiles_y;
       ++tx;
-    }
-    R* T = B0;
-    if constexpr (MODE == M_S2 || MODE == M_S3) {
-      // T2 in place of V, or T3 in place of l1
-      R* dst = MODE == M_S3 ? B2 : B1;
-      using V = typename PairOf<R>::type;
-      const V half(0.5), hdt(grid_k<R>(G, GK_HDT));
-      for (int i = 4 * threadIdx.x; i < BUF; i += 4 * NT) {
-        V p0, p1, v0(0.0), v1(0.0), w0(0.0), w1(0.0);
-        ld_quad(B0 + i, p0, p1);
-        if (!arrest) ld_quad(B1 + i, v0, v1);
-        if (MODE == M_S3) ld_quad(B2 + i, w0, w1);
-        if (MODE == M_S2)
-          st_quad(dst + i, vfma(hdt, v0, p0), vfma(hdt, v1, p1));
-        else
-          st_quad(dst + i, vfma(hdt, vfma(half, w0, v0), p0), vfma(hdt, vfma(half, w1, v1), p1));
-      }
-      __syncthreads();
-      T = dst;
-    }
-    const bool fast = (G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 &&
-                      y0 >= G.halo + 1 && y0 + TY - 1 <= G.Y - G.halo - 2;
-    if constexpr (MODE == M_S4) {
-      const R* Cp = base + BUF;
-      const R* Cv = base + BUF + CBUF;
-      if (fast)
-        grad_tile<TH, R, TX, TY, NT, true, M_S4>(A, T, x0, y0, false, err_max, nullptr, nullptr, nullptr, nullptr, Cp,
-                                                 Cv);
-      else
-        grad_tile<TH, R, TX, TY, NT, false, M_S4>(A, T, x0, y0, false, err_max, nullptr, nullptr, nullptr, nullptr, Cp,
-                                                  Cv);
-    } else if constexpr (MODE == M_S1 || MODE == M_ENERGY) {
-      constexpr bool JE = sizeof(R) == 4;
-      // the four-CTA energy pass is built for the flow energy only (the exact FP64 energy
-      // would spill out of its 64 registers); the host sends exact energies to flow_kernel
-      constexpr bool EXACT = !(MODE == M_ENERGY && pipe_ctas<TH, MODE>() == 4);
-      const bool je = JE && !(MODE == M_ENERGY && EXACT && A.exact_energy);
-      double* ep = (je && do_energy) ? &e_acc : nullptr;
-      if (MODE == M_S1 || je) {
-        if (fast)
-          grad_tile<TH, R, TX, TY, NT, true, MODE, JE>(A, T, x0, y0, false, err_max, ep);
-        else
-          grad_tile<TH, R, TX, TY, NT, false, MODE, JE>(A, T, x0, y0, false, err_max, ep);
-      }
-      if constexpr (EXACT) {
-        if (do_energy && !je) {
-          if (fast)
-            e_acc += energy_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
-          else
-            e_acc += energy_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
-        }
-      }
-    } else {
-      const R* Praw = MODE == M_S3 ? B0 : nullptr;
-      const R* Vraw = MODE == M_S3 ? B1 : nullptr;
-      if (fast)
-        grad_tile<TH, R, TX, TY, NT, true, MODE>(A, T, x0, y0, arrest, err_max, nullptr, Praw, Vraw);
-      else
-        grad_tile<TH, R, TX, TY, NT, false, MODE>(A, T, x0, y0, arrest, err_max, nullptr, Praw, Vraw);
     }
     __syncthreads();  // every thread is done with this slot
     if (threadIdx.x == 0) {
@@ -1057,55 +576,8 @@ __global__ void __launch_bounds__(NT, (pipe_ctas<TH, MODE>())) flow_kernel_pipe(
       if (nt < ntiles) issue(slot, nt);
     }
   }
-
-  // ---- reductions (as flow_kernel) ----------------------------------------
-  const bool need_ticket = do_energy || MODE == M_S4;
-  if (!need_ticket) return;
-  if (do_energy) {
-    const double bs = block_sum_fixed<NT>(e_acc, red);
-    if (threadIdx.x == 0) A.partial[blockIdx.x] = bs;
-  }
-  if (MODE == M_S4) {
-    const double bm = block_max<NT>(err_max, red);
-    if (threadIdx.x == 0 && bm > -INFINITY) atomicMax(&st->err_enc, enc_max(bm));
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned tk = atomicAdd(&st->ticket, 1u);
-    am_last = (tk == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  if (do_energy) {
-    const double E = fixed_order_sum<NT>(A.partial, gridDim.x, sh_s, sh_c);
-    if (threadIdx.x == 0) {
-      st->scalar = E;
-      if (!isfinite(E)) st->status = 3;
-      if (A.E_traj && A.E_idx >= 0) A.E_traj[A.E_idx] = E;
-      if (A.arrest_update) {
-        st->arrest = (G.killkinen && E > st->E_last) ? 1 : 0;
-        st->E_last = E;
-      }
-    }
-  }
-  if (threadIdx.x == 0) {
-    if (MODE == M_S4) {
-      const double err = dec_max(atomicExch(&st->err_enc, 0ULL));
-      if (A.err_traj && A.err_idx >= 0) A.err_traj[A.err_idx] = err;
-    }
-    st->ticket = 0u;
-  }
-}
-
-// Apply a pending arrest (V = 0) left by the trailing energy pass at the end of a call,
-// and copy the call's status to status_out (nullable; e.g. mapped host memory).
-template <typename R>
-__global__ void finish_kernel(R* vel, long long n, const StepState* st, int* status_out) {
-  if (status_out && blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)status_out = st->status;
-  if (st->arrest == 0) return;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    vel[i] = (R)0;
+  if constexpr (MODE == M_ENERGY)
+    energy_reduction<NT>(e_acc, A.partial, A.st, blockIdx.x, gridDim.x, S.red, S.sh_s, S.sh_c, S.am_last);
 }
 
 // ---------------------------------------------------------------------------
@@ -1127,12 +599,7 @@ __global__ void __launch_bounds__(NT)
   const int tiles_y = (G.Y + TY - 1) / TY;
   const int x0 = (blockIdx.x / tiles_y) * TX;
   const int y0 = (blockIdx.x % tiles_y) * TY;
-  {
-    FlowArgs<R> A;
-    A.phi = phi;
-    A.G = G;
-    stage_plain<NF, R, TX, TY, NT>(tile, A, x0, y0, M_GRAD, false);
-  }
+  stage_plain<NF, R, TX, TY, NT>(tile, G, phi, x0, y0);
   __syncthreads();
   const Inv<double> ivd(G);
   const int ly = threadIdx.x % TY;

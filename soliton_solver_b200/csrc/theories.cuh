@@ -8,11 +8,10 @@
 //   NEED_XY          mixed derivatives used
 //   gradient<R>()    dE/dphi at one site in working precision R (before projection)
 //   energy()         energy density (FP64), already multiplied by dA
-//   PAIR_ENERGY      energy_pair<V>() exists: the energy point (without dA) of a packed
-//                    FP32 site pair, used for the flow's per-step energy in stage 1
-//   S1_CTAS          resident CTAs per SM of the pipelined stage 1 and energy pass: 4
-//                    (256 threads, 64 registers) for the light chiral stencil, else 1
-//                    (512 threads)
+//   PAIR_ENERGY      energy_pair<V>() exists: the energy point (without dA) of a site pair,
+//                    used for the flow's per-step energy
+//   S1_CTAS          4: phase A of the FP32 step runs four CTAs per SM at 64 registers (the
+//                    light chiral stencil)
 // plus the charge densities / coupling partials it supports.  Every function
 // states the reference lines it restates.
 #pragma once
@@ -133,8 +132,9 @@ struct ChiralMagnet {
     return e * dA;
   }
 
-  // The same energy point (without dA) in the stage's own arithmetic, for a packed
-  // FP32 site pair of jets: the flow's per-step energy in stage 1.
+  // The same energy point (without dA) for a site pair of jets: the flow's per-step energy,
+  // in the field's precision, in explicit fused multiply-adds so that phases A and E of the
+  // step round alike.
   template <typename V>
   __device__ static inline V energy_pair(const Jet<V, NF>& J, const Phys& P) {
     const double D00 = P.c[3], D01 = P.c[4], D10 = P.c[5], D11 = P.c[6];
@@ -230,54 +230,40 @@ struct BabySkyrme {
   // do_gradient_step_point, kernels.py:308-458 (projection applied by the caller)
   template <typename R>
   __device__ static inline void gradient(const Jet<R, NF>& J, const Phys& P, R g[NF]) {
-    const R mpi2 = pk<R>(P, 2), kappa2 = pk<R>(P, 3);
+    const R mpi2 = pk<R>(P, 2);
     const R m1 = J.f[0], m2 = J.f[1], m3 = J.f[2];
-    const R F00 = J.dx[0], F01 = J.dx[1], F02 = J.dx[2];
-    const R F10 = J.dy[0], F11 = J.dy[1], F12 = J.dy[2];
-    const R S000 = J.dxx[0], S001 = J.dxx[1], S002 = J.dxx[2];
-    const R S110 = J.dyy[0], S111 = J.dyy[1], S112 = J.dyy[2];
-    const R S010 = J.dxy[0], S011 = J.dxy[1], S012 = J.dxy[2];
-    const R S100 = S010, S101 = S011, S102 = S012;
-    const R sum_F0_sq = F00 * F00 + F01 * F01 + F02 * F02;
-    const R sum_F1_sq = F10 * F10 + F11 * F11 + F12 * F12;
-    R g0 = -(S000 + S110), g1 = -(S001 + S111), g2 = -(S002 + S112);
-    const R sum_all_sq = sum_F0_sq + sum_F1_sq;
-    g0 -= kappa2 * S000 * sum_all_sq;
-    g1 -= kappa2 * S001 * sum_all_sq;
-    g2 -= kappa2 * S002 * sum_all_sq;
-    g0 += kappa2 * S000 * sum_F0_sq;
-    g1 += kappa2 * S001 * sum_F0_sq;
-    g2 += kappa2 * S002 * sum_F0_sq;
-    const R sumA = (S010 * F10 - S110 * F00) + (S011 * F11 - S111 * F01) + (S012 * F12 - S112 * F02);
-    const R dot01 = F00 * F10 + F01 * F11 + F02 * F12;
-    g0 -= kappa2 * (F00 * sumA - S010 * dot01);
-    g1 -= kappa2 * (F01 * sumA - S011 * dot01);
-    g2 -= kappa2 * (F02 * sumA - S012 * dot01);
-    g0 -= kappa2 * S110 * sum_all_sq;
-    g1 -= kappa2 * S111 * sum_all_sq;
-    g2 -= kappa2 * S112 * sum_all_sq;
-    g0 += kappa2 * S110 * sum_F1_sq;
-    g1 += kappa2 * S111 * sum_F1_sq;
-    g2 += kappa2 * S112 * sum_F1_sq;
-    const R sumB = (S100 * F00 - S000 * F10) + (S101 * F01 - S001 * F11) + (S102 * F02 - S002 * F12);
-    g0 -= kappa2 * (F10 * sumB - S100 * dot01);
-    g1 -= kappa2 * (F11 * sumB - S101 * dot01);
-    g2 -= kappa2 * (F12 * sumB - S102 * dot01);
+    // Skyrme term: with a = dx.dx, b = dy.dy, c = dx.dy (products over the components)
+    //   xx b + yy a - 2 xy c + dx (xy.dy - yy.dx) + dy (xy.dx - xx.dy)
+    // The reference's sums over all pairs, in which xx a and yy b cancel, without the
+    // cancelling terms.  Every product feeds an explicit fused multiply-add, so the rounding
+    // does not depend on what the compiler contracts around it.
+    auto dot = [](const R* u, const R* v) { return vfma(u[0], v[0], vfma(u[1], v[1], u[2] * v[2])); };
+    const R a = dot(J.dx, J.dx), b = dot(J.dy, J.dy), m2c = R(-2.0) * dot(J.dx, J.dy);
+    const R sA = dot(J.dxy, J.dy) - dot(J.dyy, J.dx), sB = dot(J.dxy, J.dx) - dot(J.dxx, J.dy);
+    const R mk2 = -pk<R>(P, 3);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const R t = vfma(J.dxx[i], b, vfma(J.dyy[i], a, vfma(J.dx[i], sA, vfma(J.dy[i], sB, J.dxy[i] * m2c))));
+      g[i] = vfma(mk2, t, -(J.dxx[i] + J.dyy[i]));
+    }
+    R g0 = g[0], g1 = g[1], g2 = g[2];
+    const R one(1.0);
     if (P.k[0]) g2 -= mpi2;
-    if (P.k[1]) { const R t = (R)1 - m3; g2 -= (R)4 * mpi2 * t * t * t; }
-    if (P.k[2]) g0 += mpi2 * m1;
+    if (P.k[1]) { const R t = one - m3; g2 = vfma(R(-4.0) * mpi2 * t, t * t, g2); }
+    if (P.k[2]) g0 = vfma(mpi2, m1, g0);
     if (P.k[3]) {
-      g0 -= mpi2 * ((R)1 - m3 * m3) * m1;
-      g2 -= mpi2 * ((R)1 - m1 * m1) * m3;
+      g0 = vfma(-mpi2 * m1, vfma(-m3, m3, one), g0);
+      g2 = vfma(-mpi2 * m3, vfma(-m1, m1, one), g2);
     }
     if (P.k[4]) {
-      const R t = (R)1 - m3, t3 = t * t * t;
-      g2 -= mpi2 * ((R)0.5 * ((R)1 + t3) + (R)1.5 * t3);
+      const R t = one - m3;
+      g2 = vfma(-mpi2, vfma(R(2.0) * t, t * t, R(0.5)), g2);
     }
     if (P.k[5]) {
-      g0 += (R)48 * mpi2 * (m2 * m2 - m1 * m1) * ((R)1 - m3);
-      g1 += (R)96 * mpi2 * m1 * m2 * ((R)1 - m3);
-      g2 -= (R)16 * mpi2 * (-(m1 * m1 * m1) + (R)3 * m1 * (m2 * m2) + ((R)1 - (R)3 * m3) * ((R)1 - (R)3 * m3));
+      const R t = one - m3, w = vfma(R(-3.0), m3, one);
+      g0 = vfma(R(48.0) * mpi2 * t, vfma(m2, m2, -(m1 * m1)), g0);
+      g1 = vfma(R(96.0) * mpi2 * t, m1 * m2, g1);
+      g2 = vfma(R(-16.0) * mpi2, vfma(w, w, m1 * vfma(R(3.0) * m2, m2, -(m1 * m1))), g2);
     }
     if (P.k[6]) {
       // broken potential: transcendental, evaluated site by site
@@ -292,7 +278,7 @@ struct BabySkyrme {
         Lanes<R>::set(g2, l, a2);
       }
     }
-    if (P.k[7]) g2 -= (R)2 * mpi2 * m3;
+    if (P.k[7]) g2 = vfma(R(-2.0) * mpi2, m3, g2);
     g[0] = g0; g[1] = g1; g[2] = g2;
   }
 
@@ -352,11 +338,14 @@ struct BabySkyrme {
     return e * dA;
   }
 
-  // the same energy point for a packed FP32 site pair, without dA (the flow's per-step
-  // energy from the gradient's jets; FP32 rounding per site, FP64 sums)
+  // the same energy point for a site pair, without dA: the flow's per-step energy from the
+  // gradient's jets, in the field's precision (FP64 sums), in explicit fused multiply-adds so
+  // that phases A and E of the step round alike
   template <typename V>
   __device__ static inline V energy_pair(const Jet<V, NF>& J, const Phys& P) {
-    const V mpi2(P.cf[0] * P.cf[0]), hk2(0.5f * (P.cf[1] * P.cf[1])), half(0.5f), one(1.0f);
+    using S = typename ScalarOf<V>::type;
+    const S mpi = phys_k<S>(P, 0), kappa = phys_k<S>(P, 1);
+    const V mpi2(mpi * mpi), hk2((S)0.5 * (kappa * kappa)), half(0.5f), one(1.0f);
     V g = J.dx[0] * J.dx[0];
     g = vfma(J.dx[1], J.dx[1], g);
     g = vfma(J.dx[2], J.dx[2], g);
@@ -377,7 +366,7 @@ struct BabySkyrme {
     if (P.k[3]) u = vfma(half * vfma(-m1, m1, one), vfma(-m3, m3, one), u);
     if (P.k[4]) u = vfma(half * t, vfma(t * t, t, one), u);
     if (P.k[5]) {
-      const V q = vfma(V(3.0f) * m1, m2 * m2, vfma(V(3.0f) * m3, m3, one)) - m1 * m1 * m1;
+      const V q = vfma(-(m1 * m1), m1, vfma(V(3.0f) * m1, m2 * m2, vfma(V(3.0f) * m3, m3, one)));
       u = vfma(V(16.0f) * t, q, u);
     }
     if (P.k[6]) {
@@ -469,12 +458,13 @@ struct GinzburgLandau {
     return e * dA;
   }
 
-  // the same energy point for a packed FP32 site pair, without dA (flow energies from
-  // the gradient's jets, FP64 sums); u as above
+  // the same energy point for a site pair, without dA (flow energies from the gradient's
+  // jets, FP64 sums; explicit fused multiply-adds as above); u as above
   template <typename V>
   __device__ static inline V energy_pair(const Jet<V, NF>& J, const Phys& P) {
-    const float qf = P.cf[0], uf = P.cf[3];
-    const V q(qf), hq2(0.5f * (qf * qf)), lam8(0.125f * P.cf[1]), u2(uf * uf), half(0.5f);
+    using S = typename ScalarOf<V>::type;
+    const S qf = phys_k<S>(P, 0), uf = phys_k<S>(P, 3);
+    const V q(qf), hq2((S)0.5 * (qf * qf)), lam8((S)0.125 * phys_k<S>(P, 1)), u2(uf * uf), half(0.5f);
     const V A1 = J.f[0], A2 = J.f[1], p1 = J.f[2], p2 = J.f[3];
     const V p1x = J.dx[2], p1y = J.dy[2], p2x = J.dx[3], p2y = J.dy[3];
     const V psq = vfma(p1, p1, p2 * p2);
@@ -530,12 +520,6 @@ struct Anisotropic {
     if (a == 1 && b == 1) return pk<R>(P, 14);
     return i == 0 ? -pk<R>(P, 15) : pk<R>(P, 15);
   }
-  __device__ static inline double gam(int i, int a, int b, const Phys& P) {
-    if (a == 0 && b == 0) return 2.0 * P.c[8];
-    if (a == 1 && b == 1) return 2.0 * P.c[9];
-    return (i == 0 ? -2.0 : 2.0) * P.c[10];
-  }
-
   // derived slots: c[12] kappa^2, c[13..15] 2 gamma1, 2 gamma2, 2 gamma12
   static void derive(Phys& P) {
     P.c[12] = P.c[0] * P.c[0];
@@ -603,38 +587,31 @@ struct Anisotropic {
     for (int a = 0; a < 6; ++a) g[a] = EG[a];
   }
 
-  // compute_energy_point, kernels.py:97-170 (T: double, or a dual number, adjoint.cuh)
+  // compute_energy_point, kernels.py:97-170, in covariant derivatives: 0.5 gamma_ab D p_a . D p_b
+  // with D p = d p + i Q A p (T: double, or a dual number, adjoint.cuh)
   template <typename T>
   __device__ static inline T energy(const Jet1<T, NF>& J, const Phys& P, double dA) {
-    const double kappa = P.c[0], Q = P.c[1], a1 = P.c[2], a2 = P.c[3];
+    const double Q = P.c[1], a1 = P.c[2], a2 = P.c[3];
     const double b1 = P.c[4], b2 = P.c[5], b3 = P.c[6], b4 = P.c[7];
-    const T A[2] = {J.f[0], J.f[1]};
+    const double g1 = P.c[8], g2 = P.c[9], g12 = P.c[15];
     const T p1r = J.f[2], p1i = J.f[3], p2r = J.f[4], p2i = J.f[5];
-    const T p1sq = p1r * p1r + p1i * p1i, p2sq = p2r * p2r + p2i * p2i;
+    const T n1 = vfma(p1r, p1r, p1i * p1i), n2 = vfma(p2r, p2r, p2i * p2i);
     const T curl = J.dx[1] - J.dy[0];
-    const T F_mag = 0.5 * kappa * kappa * (curl * curl);
-    T F_pot = T(0.0);
-    F_pot += a1 * p1sq + a2 * p2sq;
-    F_pot += b1 * p1sq * p1sq + b2 * p2sq * p2sq + b3 * p1sq * p2sq;
-    F_pot += 2.0 * b4 * (p1r * p1r * p2r * p2r + p1i * p1i * p2i * p2i - p1i * p1i * p2r * p2r -
-                         p1r * p1r * p2i * p2i + 4.0 * p1r * p1i * p2r * p2i);
-    T F_kin = T(0.0);
+    T e = (T(0.5 * P.c[12]) * curl) * curl;
+    // Re(conj(psi1)^2 psi2^2) = (p1.p2)^2 - (p1 x p2)^2
+    const T u = vfma(p1r, p2r, p1i * p2i), w = vfma(p1r, p2i, -(p1i * p2r));
+    e = vfma(n1, vfma(T(b1), n1, vfma(T(b3), n2, T(a1))), e);
+    e = vfma(n2, vfma(T(b2), n2, T(a2)), e);
+    e = vfma(T(2.0 * b4), vfma(u, u, -(w * w)), e);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const T Ai = A[i];
       const T* d = (i == 0) ? J.dx : J.dy;
-      const double g00 = gam(i, 0, 0, P), g01 = gam(i, 0, 1, P), g10 = gam(i, 1, 0, P), g11 = gam(i, 1, 1, P);
-      const T r1 = d[2], i1 = d[3], r2 = d[4], i2 = d[5];
-      F_kin += 0.5 * g00 * (r1 * r1 + i1 * i1 + Q * Ai * (p1r * i1 - p1i * r1) + Q * Ai * (p1r * i1 - p1i * r1) +
-                            Q * Q * Ai * Ai * p1sq);
-      F_kin += 0.5 * g01 * (r1 * r2 + i1 * i2 + Q * Ai * (p1r * i2 - p1i * r2) + Q * Ai * (p2r * i1 - p2i * r1) +
-                            Q * Q * Ai * Ai * (p1r * p2r + p1i * p2i));
-      F_kin += 0.5 * g10 * (r2 * r1 + i2 * i1 + Q * Ai * (p2r * i1 - p2i * r1) + Q * Ai * (p1r * i2 - p1i * r2) +
-                            Q * Q * Ai * Ai * (p2r * p1r + p2i * p1i));
-      F_kin += 0.5 * g11 * (r2 * r2 + i2 * i2 + Q * Ai * (p2r * i2 - p2i * r2) + Q * Ai * (p2r * i2 - p2i * r2) +
-                            Q * Q * Ai * Ai * p2sq);
+      const T QA = T(Q) * J.f[i];
+      const T r1 = vfma(-QA, p1i, d[2]), i1 = vfma(QA, p1r, d[3]), r2 = vfma(-QA, p2i, d[4]), i2 = vfma(QA, p2r, d[5]);
+      e = vfma(T(g1), vfma(r1, r1, i1 * i1), e);
+      e = vfma(T(g2), vfma(r2, r2, i2 * i2), e);
+      e = vfma(T(i == 0 ? -g12 : g12), vfma(r1, r2, i1 * i2), e);
     }
-    T e = F_kin + F_mag + F_pot;
     e -= P.c[11];
     return e * dA;
   }
