@@ -113,7 +113,9 @@ int ss_workspace_bytes(const ss_handle *h, size_t *bytes);
 int ss_bind(ss_handle *h, void *field, void *velocity, void *workspace, size_t workspace_bytes,
             void *stream);
 
-/* n_steps arrested-Newton-flow RK4 steps of the bound Field/Velocity.
+/* n_steps arrested-Newton-flow RK4 steps of the bound Field/Velocity.  A lattice small
+ * enough for all its tiles to be resident on the GPU at once runs all steps of a call in
+ * one cooperative launch, unless a stage's variant was pinned (ss_set_variant).
  * Replaces Simulation.step / do_arrested_newton_flow
  * (soliton_solver/core/simulation.py:388-409, core/integrator.py:217-348).
  * energy_traj[s] / err_traj[s] (host, nullable) receive E after step s and the

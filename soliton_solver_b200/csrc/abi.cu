@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "flow.cuh"
 #include "rk.cuh"
+#include "coop.cuh"
 #include "plain.cuh"
 #include "batch.cuh"
 #include "render.cuh"
@@ -29,6 +30,7 @@ using namespace ssb;
 namespace {
 
 constexpr int TX = 16, TY = 64, NT = 256;  // fused tile: 16 x 64 sites, 256 threads
+constexpr int COOP_MAX_TILES = 4096;        // energy partials kept for the cooperative step
 constexpr int TRAJ_CAP = 1024;              // device trajectory slots used by ss_step
 constexpr size_t ALIGN = 256;
 // Tensor maps of a bound handle (halo boxes): phi and V of the caller's buffers and of the
@@ -121,6 +123,8 @@ struct ss_handle {
   double* entmp = nullptr;
   double E_last_host = NAN;
   std::vector<double> host_partial;
+  bool pinned = false;  // a stage's variant was pinned (ss_set_variant): the two-launch step runs it
+  int coop = 0;  // small lattices: 1 + tile shape of the cooperative step (0: two launches per step)
   // TMA maps of the bound buffers (index constants TM_*)
   CUtensorMap tm[TM_COUNT];
   bool tma = false;
@@ -160,7 +164,7 @@ size_t layout(ss_handle* h, char* base) {
   const size_t field_bytes = h->elem * (size_t)h->nf * (size_t)h->G.N;
   h->st = (StepState*)take(sizeof(StepState));
   // energy partials: one per tile of 16 rows, or of 8 in the step's phases
-  const size_t np = (size_t)std::max(2 * h->nblocks, std::max(h->plain_sum_blocks, h->plain_max_blocks));
+  const size_t np = (size_t)std::max(std::max(2 * h->nblocks, COOP_MAX_TILES), std::max(h->plain_sum_blocks, h->plain_max_blocks));
   h->partial = (double*)take(np * sizeof(double));
   h->traj_E = (double*)take(TRAJ_CAP * sizeof(double));
   h->traj_err = (double*)take(TRAJ_CAP * sizeof(double));
@@ -300,6 +304,20 @@ int check_bound(const ss_handle* h) {
   if (!h) return fail(SS_ERR_ARG, "NULL handle");
   if (!h->ws) return fail(SS_ERR_STATE, "no workspace bound: call ss_bind first");
   return SS_OK;
+}
+
+// Tile shapes of the cooperative step (rows, columns, threads; SPLIT: two threads per site
+// pair, one per stencil field, which takes FP64 baby Skyrme 128^2 from 11.4 to 9.1 us per
+// step).  8 x 32 tiles hold FP32 lattices of up to ~110 000 sites (three CTAs per SM), 16 x 32
+// up to ~220 000, 16 x 64 up to ~300 000; about half that in FP64.
+constexpr int N_COOP_SHAPES = 3;
+constexpr int COOP_TX[N_COOP_SHAPES] = {8, 16, 16};
+constexpr int COOP_TY[N_COOP_SHAPES] = {32, 32, 64};
+constexpr int COOP_NT[N_COOP_SHAPES] = {256, 128, 256};
+constexpr bool COOP_SPLIT[N_COOP_SHAPES] = {true, false, false};
+int coop_tiles(const Grid& G, int shape) {
+  const long long t = (long long)((G.X + COOP_TX[shape] - 1) / COOP_TX[shape]) * ((G.Y + COOP_TY[shape] - 1) / COOP_TY[shape]);
+  return (int)std::min(t, 0x7fffffffLL);
 }
 
 // Opt a kernel into more than 48 KB of dynamic shared memory, once per device.
@@ -463,10 +481,70 @@ struct Fused {
     A.vel = (const R*)(pair ? h->vel2 : h->vel);
   }
 
+  // ---- small lattices: all steps of a call in one cooperative launch (coop.cuh) ----
+  template <int S, int VW>
+  static int launch_coop(const ss_handle* h, const StepArgs<R>& A, const CoopArgs<R>& C, int* capacity) {
+    constexpr int CX = COOP_TX[S], CY = COOP_TY[S], CN = COOP_NT[S];
+    using CT = CoopTile<TH, R, CX, CY, CN, COOP_SPLIT[S]>;
+    if constexpr (CT::SMEM > 220 * 1024) {
+      if (capacity) *capacity = 0;
+      return capacity ? SS_OK : fail(SS_ERR_ARG, "bad cooperative shape");
+    } else {
+      auto k = coop_step_kernel<TH, R, CX, CY, CN, COOP_SPLIT[S], VW>;
+      static unsigned long long done = 0;
+      set_smem(k, CT::SMEM, done);
+      if (capacity) {  // co-resident CTAs
+        int occ = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, CN, CT::SMEM) != cudaSuccess) occ = 0;
+        *capacity = occ * h->num_sms;
+        return SS_OK;
+      }
+      void* args[2] = {const_cast<StepArgs<R>*>(&A), const_cast<CoopArgs<R>*>(&C)};
+      CK(cudaLaunchCooperativeKernel((const void*)k, dim3(coop_tiles(h->G, S)), dim3(CN), args, CT::SMEM, h->stream));
+      return SS_OK;
+    }
+  }
+  static int coop_any(const ss_handle* h, int shape, const StepArgs<R>& A, const CoopArgs<R>& C, int* capacity) {
+    constexpr int VW = 16 / (int)sizeof(R);
+    switch (shape) {
+      case 0: return h->tma ? launch_coop<0, VW>(h, A, C, capacity) : launch_coop<0, 1>(h, A, C, capacity);
+      case 1: return h->tma ? launch_coop<1, VW>(h, A, C, capacity) : launch_coop<1, 1>(h, A, C, capacity);
+    }
+    return h->tma ? launch_coop<2, VW>(h, A, C, capacity) : launch_coop<2, 1>(h, A, C, capacity);
+  }
+  // whether the lattice's tiles of `shape` are all resident at once
+  static bool coop_fits(const ss_handle* h, int shape) {
+    const long long t = coop_tiles(h->G, shape);
+    int cap = 0;
+    return t <= COOP_MAX_TILES && coop_any(h, shape, StepArgs<R>{}, CoopArgs<R>{}, &cap) == SS_OK && t <= cap;
+  }
+  static int step_coop(ss_handle* h, int n, double prev, double* E_dev, double* err_dev, int* status_out) {
+    StepArgs<R> A = step_args(h);
+    A.wait_cycles = 16 * h->wait_cycles;  // other work on the GPU may hold up a CTA of the grid
+    CoopArgs<R> C;
+    C.phi[0] = (R*)h->field;
+    C.phi[1] = (R*)h->phi2;
+    C.vel[0] = (R*)h->vel;
+    C.vel[1] = (R*)h->vel2;
+    C.l1 = (R*)h->l[0];
+    C.l2 = (R*)h->l[1];
+    C.status_out = status_out;
+    for (int done = 0; done < n; done += C.n) {
+      C.n = std::min(n - done, 4096);
+      A.prev_energy = done ? NAN : prev;
+      A.E_traj = E_dev ? E_dev + done : nullptr;
+      A.err_traj = err_dev ? err_dev + done : nullptr;
+      const int rc = coop_any(h, h->coop - 1, A, C, nullptr);
+      if (rc) return rc;
+    }
+    return SS_OK;
+  }
+
   // n flow steps of the bound buffers, in place; trajectories to device arrays (nullable)
   // status_out (nullable, device-visible): the finish kernel copies the call's status there
   static int step(ss_handle* h, int n, double prev, double* E_dev, double* err_dev, int* status_out = nullptr) {
     if (n <= 0) return SS_OK;
+    if (h->coop && !h->inject_timeout) return step_coop(h, n, prev, E_dev, err_dev, status_out);
     StepArgs<R> A = step_args(h);
     A.E_traj = E_dev;
     A.err_traj = err_dev;
@@ -744,6 +822,27 @@ void step_shape(const ss_handle* h, int& txa, int& txb) {
   });
 }
 
+// Whether (and in which tile shape) the handle's steps run cooperatively: 1 + shape, or 0.
+// The first shape whose tiles are all resident: wherever one fits, the cooperative step was
+// the faster (us per step, two launches -> cooperative: chiral magnet FP32 150 x 200 19.6 ->
+// 7.1, 321 x 256 19.6 -> 10.5, 384 x 400 26.6 -> 15.5, 512 x 560 27.4 -> 18.9; FP64 240 x 256
+// 24.7 -> 11.1, 321 x 256 28.6 -> 20.8; s+id FP32 240 x 256 22.7 -> 11.3), and of two shapes
+// that fit the smaller tile (10.5 against 12.9 and 12.7 at 321 x 256).
+int coop_plan(const ss_handle* h) {
+  if (h->pinned) return 0;
+  int dev = 0, ok = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&ok, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !ok)
+    return 0;
+  int got = 0;
+  for (int s = 0; s < N_COOP_SHAPES && !got; ++s)
+    dispatch(h, [&](auto* tag) -> int {
+      using TH = std::remove_pointer_t<decltype(tag)>;
+      if (h->precision == SS_FP32 ? Fused<TH, float>::coop_fits(h, s) : Fused<TH, double>::coop_fits(h, s)) got = s + 1;
+      return SS_OK;
+    });
+  return got;
+}
+
 int read_state(ss_handle* h, StepState* out) {
   CK(cudaMemcpyAsync(out, h->st, sizeof(StepState), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -902,10 +1001,12 @@ int ss_bind(ss_handle* h, void* field, void* velocity, void* workspace, size_t w
       ok = encode_tile_map(&h->tm[TM_L + i], h->l[i], h->elem, h->G.X, h->G.Y, h->nf, false, txb, TY);
     h->tma = ok;
   }
+  h->coop = 0;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) == cudaSuccess &&
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
     h->num_sms = sms;
+  if (h->precision != SS_PLAIN_FP64 && field && velocity) h->coop = coop_plan(h);
   return SS_OK;
 }
 
@@ -952,6 +1053,10 @@ int ss_set_variant(ss_handle* h, int mode, int variant) {
                 "stage 1", mode);
   if (variant != 0 && variant != 1) return fail(SS_ERR_ARG, "variant %d: 0 (one tile per CTA) or 1 (pipelined)", variant);
   if (h->precision == SS_PLAIN_FP64) return fail(SS_ERR_ARG, "the plain FP64 form has no staging variants");
+  if (mode != M_GRAD) {  // the step's launches were asked for
+    h->pinned = true;
+    h->coop = 0;
+  }
   if (mode == M_S23) {  // 1: stages 2 and 3 in one kernel (used with TMA staging), 0: two kernels
     h->fuse23 = variant;
     return SS_OK;
