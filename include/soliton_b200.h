@@ -72,6 +72,11 @@ extern "C" {
 #define SS_COUPLING_COUP_H 4  /* chiral magnet coup_h (p_f[7]) */
 #define SS_COUPLING_COUP_MU 5 /* chiral magnet coup_mu (p_f[8]) */
 
+/* kinds for ss_observables */
+#define SS_OBS_ENERGY 0   /* ss_energy */
+#define SS_OBS_CHARGE 1   /* ss_charge; which: SS_CHARGE_* */
+#define SS_OBS_COUPLING 2 /* ss_coupling_grad; which: SS_COUPLING_* */
+
 /* colormaps for ss_render_rgba */
 #define SS_RENDER_JET 0           /* core/colormaps.py render_jet_density_to_rgba */
 #define SS_RENDER_GRAY 1          /* core/colormaps.py render_gray_density_to_rgba */
@@ -105,9 +110,9 @@ const char *ss_last_error(void);
 int ss_create(int theory, const int32_t *p_i, int n_i, const double *p_f, int n_f, int precision,
               ss_handle **out);
 int ss_destroy(ss_handle *h);
-/* Bytes of caller-owned device workspace ss_bind() needs (four field-sized flow
- * buffers: l1, l2 and the second field and velocity that steps alternate with; reduction
- * partials and the device-side step state). */
+/* Bytes of caller-owned device workspace ss_bind() needs (five field-sized
+ * buffers: l1, l2, the second field and velocity that steps alternate with, and scratch;
+ * reduction partials and the device-side step state). */
 int ss_workspace_bytes(const ss_handle *h, size_t *bytes);
 /* Bind the caller's Field and Velocity buffers, the workspace and the stream. */
 int ss_bind(ss_handle *h, void *field, void *velocity, void *workspace, size_t workspace_bytes,
@@ -288,6 +293,12 @@ int ss_field_density(ss_handle *h, const void *field, int kind, double *out);
  * fixed field.  At a relaxed (stationary) field this is dE_min/dc by the envelope
  * theorem.  No reference counterpart: a new capability of this backend. */
 int ss_coupling_grad(ss_handle *h, const void *field, int coupling, double *out);
+
+/* Several totals of `field` in one pass and one synchronisation: out[i] is the energy, a
+ * charge or a coupling partial (kinds[i], which[i]; n = 1..4), as ss_energy, ss_charge and
+ * ss_coupling_grad give them.  Replaces the calls of Simulation.observables
+ * (soliton_solver/core/simulation.py:168-192). */
+int ss_observables(ss_handle *h, const void *field, int n, const int *kinds, const int *which, double *out);
 
 /* Total energy of `field` (SS_FP32 or SS_FP64 elements, reference layout) with no
  * handle and no allocation of any kind.  No counterpart in the reference: it exists

@@ -118,6 +118,7 @@ _SIG = {
     "ss_charge_density": ([_P, _P, _I, _P], _I),
     "ss_charge": ([_P, _P, _I, ctypes.POINTER(_D)], _I),
     "ss_coupling_grad": ([_P, _P, _I, ctypes.POINTER(_D)], _I),
+    "ss_observables": ([_P, _P, _I, _P, _P, _P], _I),
     "ss_field_density": ([_P, _P, _I, _P], _I),
     "ss_convert_field": ([_P, _P, _I, _P, _I, _I], _I),
     "ss_energy_gradient_exact": ([_P, _P, _P, _I], _I),

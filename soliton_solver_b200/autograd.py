@@ -153,7 +153,7 @@ def _partials(sim, solver, field, names):
     reduced couplings' chain rule, plus the reduced ones)."""
     mod = sim.theory.__name__.rsplit(".", 1)[-1]
     if mod == "chiral_magnet":
-        red = {c: solver.coupling_grad(field, c) for c in _REDUCED[mod]}
+        red = solver.observables(field, _REDUCED[mod])
         chain = sim.theory.params.coupling_chain(sim.rp)
         out = dict(red)
         for phys, parts in chain.items():
@@ -163,7 +163,7 @@ def _partials(sim, solver, field, names):
         return out
     avail = {"baby_skyrme": ("kappa", "mpi"), "ginzburg_landau_superconductor": ("Lambda",)}.get(mod, ())
     names = avail if names is None else names
-    return {c: solver.coupling_grad(field, c) for c in names}
+    return solver.observables(field, names) if names else {}
 
 
 def coupling_gradients(sim, names=None) -> dict:

@@ -289,15 +289,14 @@ class Simulation:
     def observables(self):
         """Energy plus every charge the theory's observables module provides
         (soliton_solver/core/simulation.py:168-192)."""
-        obs = {"energy": self.solver.energy(self.Field)}
         om = self.observables_mod
-        if hasattr(om, "compute_skyrmion_number"):
-            obs["skyrmion_number"] = self.solver.charge(self.Field, "skyrmion")
-        if hasattr(om, "compute_vortex_number"):
-            obs["vortex_number"] = self.solver.charge(self.Field, "vortex")
-        if hasattr(om, "compute_magnetic_charge"):
-            obs["magnetic_charge"] = self.solver.charge(self.Field, "magnetic")
-        return obs
+        names = {"energy": "energy"}
+        for name, charge in (("skyrmion_number", "skyrmion"), ("vortex_number", "vortex"),
+                             ("magnetic_charge", "magnetic")):
+            if hasattr(om, f"compute_{name}"):
+                names[name] = charge
+        got = self.solver.observables(self.Field, names.values())
+        return {name: got[q] for name, q in names.items()}
 
     def projected_energy(self) -> float:
         """FP64 energy of sim.Field with every site's magnetisation divided by its FP64

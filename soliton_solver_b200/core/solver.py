@@ -303,6 +303,23 @@ class Solver:
             nat.check(self._lib.ss_coupling_grad(self._h, _ptr(field), _COUPLINGS[which], ctypes.byref(out)))
         return out.value
 
+    def observables(self, field, quantities):
+        """Totals of `field` in one pass (at most four per pass): `quantities` lists "energy",
+        charge names and coupling names; returns {name: float}."""
+        self._check(field)
+        names = list(quantities)
+        out = {}
+        for i in range(0, len(names), 4):
+            part = names[i:i + 4]
+            code = [(0, 0) if n == "energy" else (1, _CHARGES[n]) if n in _CHARGES else (2, _COUPLINGS[n]) for n in part]
+            kinds = (ctypes.c_int * len(part))(*[k for k, _ in code])
+            which = (ctypes.c_int * len(part))(*[w for _, w in code])
+            vals = (ctypes.c_double * len(part))()
+            with torch.cuda.device(self.device):
+                nat.check(self._lib.ss_observables(self._h, _ptr(field), len(part), kinds, which, vals))
+            out.update(zip(part, vals))
+        return out
+
     def rk4_stage(self, k_out, velocity, l_in, temp, field, k_prev, factor: float):
         with torch.cuda.device(self.device):
             nat.check(self._lib.ss_rk4_stage(self._h, _ptr(k_out), _ptr(velocity), _ptr(l_in), _ptr(temp),

@@ -163,8 +163,9 @@ size_t layout(ss_handle* h, char* base) {
   };
   const size_t field_bytes = h->elem * (size_t)h->nf * (size_t)h->G.N;
   h->st = (StepState*)take(sizeof(StepState));
-  // energy partials: one per tile of 16 rows, or of 8 in the step's phases
-  const size_t np = (size_t)std::max(std::max(2 * h->nblocks, COOP_MAX_TILES), std::max(h->plain_sum_blocks, h->plain_max_blocks));
+  // partials: per tile of 16 rows one for each quantity of an observables pass, or one per
+  // tile of 8 rows in the step's phases
+  const size_t np = (size_t)std::max(std::max(OBS_MAX * h->nblocks, COOP_MAX_TILES), std::max(h->plain_sum_blocks, h->plain_max_blocks));
   h->partial = (double*)take(np * sizeof(double));
   h->traj_E = (double*)take(TRAJ_CAP * sizeof(double));
   h->traj_err = (double*)take(TRAJ_CAP * sizeof(double));
@@ -182,6 +183,7 @@ size_t layout(ss_handle* h, char* base) {
     h->l[2] = h->l[3] = nullptr;
     h->phi2 = take(field_bytes);
     h->vel2 = take(field_bytes);
+    take(field_bytes);  // five field-sized buffers, the size callers know (scratch of the exact gradient)
   }
   return off;
 }
@@ -345,55 +347,43 @@ dim3 grid_1d(long long n) {
 template <class TH, typename R>
 struct Fused {
   static constexpr size_t BUF = tile_buf_bytes<R, TH::NF, TX, TY>();
-  static inline unsigned long long smem_done_density = 0;
 
-  // tma: use the TMA-staged instantiation (A.tm_* must describe A's buffers)
-  static inline unsigned long long smem_done[2][N_FLOW_MODES] = {};
-
-  template <bool TMA_, int MODE>
-  static int launch_mode(const ss_handle* h, const FlowArgs<R>& A) {
-    auto k = flow_kernel<TH, R, TX, TY, NT, TMA_, MODE>;
-    set_smem(k, BUF, smem_done[TMA_ ? 1 : 0][MODE]);
+  // the gradient hook: one tile per CTA, or (FP32) persistent and TMA-pipelined
+  static constexpr int PIPE_STAGES = 212 * 1024 / BUF > 4 ? 4 : (int)(212 * 1024 / BUF);
+  template <bool TMA_>
+  static int launch_grad_tile(const ss_handle* h, const FlowArgs<R>& A) {
+    auto k = flow_kernel<TH, R, TX, TY, NT, TMA_>;
+    static unsigned long long done = 0;
+    set_smem(k, BUF, done);
     k<<<h->nblocks, NT, BUF, h->stream>>>(A);
     CK(cudaGetLastError());
     return SS_OK;
   }
-
-  template <bool TMA_>
-  static int launch_tma(const ss_handle* h, const FlowArgs<R>& A) {
-    return A.mode == M_GRAD ? launch_mode<TMA_, M_GRAD>(h, A) : launch_mode<TMA_, M_ENERGY>(h, A);
-  }
-
-  // persistent TMA-pipelined variant: FP32 fields
-  static constexpr int PIPE_STAGES = 212 * 1024 / BUF > 4 ? 4 : (int)(212 * 1024 / BUF);
-  static inline unsigned long long smem_done_pipe[N_FLOW_MODES] = {};
-  template <int MODE>
-  static int launch_pipe(const ss_handle* h, const FlowArgs<R>& A) {
-    if constexpr (sizeof(R) == 4) {
-      auto k = flow_kernel_pipe<TH, R, TX, TY, 2 * NT, MODE, PIPE_STAGES>;
-      set_smem(k, PIPE_STAGES * BUF, smem_done_pipe[MODE]);
-      k<<<std::min(h->nblocks, h->num_sms), 2 * NT, PIPE_STAGES * BUF, h->stream>>>(A);
-      CK(cudaGetLastError());
-      return SS_OK;
-    } else {
-      return launch_mode<true, MODE>(h, A);
-    }
-  }
-
   // whether a mode has a pipelined variant (phase A's, M_S1 and M_S2, is accepted and ignored)
   static bool uses_pipe(int) { return sizeof(R) == 4; }
 
   // tma: use the TMA-staged instantiations (A.tm_phi must describe A.phi)
   static int launch(const ss_handle* h, const FlowArgs<R>& A0, bool tma) {
     FlowArgs<R> A = A0;
-    if (h->inject_timeout && tma) {
-      A.tx_extra = 16;
-      h->inject_timeout = 0;
+    A.tx_extra = take_injection(h, tma);
+    if (!tma) return launch_grad_tile<false>(h, A);
+    if constexpr (sizeof(R) == 4) {
+      if (h->use_pipe[M_GRAD]) {
+        auto k = flow_kernel_pipe<TH, R, TX, TY, 2 * NT, PIPE_STAGES>;
+        static unsigned long long done = 0;
+        set_smem(k, PIPE_STAGES * BUF, done);
+        k<<<std::min(h->nblocks, h->num_sms), 2 * NT, PIPE_STAGES * BUF, h->stream>>>(A);
+        CK(cudaGetLastError());
+        return SS_OK;
+      }
     }
-    if (!tma) return launch_tma<false>(h, A);
-    // the chiral magnet's exact energy is better one tile per CTA
-    if (!h->use_pipe[A.mode] || (A.mode == M_ENERGY && TH::S1_CTAS == 4)) return launch_tma<true>(h, A);
-    return A.mode == M_GRAD ? launch_pipe<M_GRAD>(h, A) : launch_pipe<M_ENERGY>(h, A);
+    return launch_grad_tile<true>(h, A);
+  }
+  // bytes the next TMA barrier expects beyond its loads (the injected timeout, consumed)
+  static unsigned take_injection(const ss_handle* h, bool tma) {
+    if (!tma || !h->inject_timeout) return 0u;
+    h->inject_timeout = 0;
+    return 16u;
   }
 
   static FlowArgs<R> base_args(const ss_handle* h) {
@@ -403,7 +393,6 @@ struct Fused {
     A.G = h->G;
     A.P = h->P;
     A.st = h->st;
-    A.partial = h->partial;
     return A;
   }
 
@@ -422,11 +411,7 @@ struct Fused {
     auto k = step_kernel<TH, R, TMA_, PH>;
     static unsigned long long done = 0;  // one per instantiation
     set_smem(k, smem, done);
-    A.tx_extra = 0;
-    if (TMA_ && h->inject_timeout) {
-      A.tx_extra = 16;
-      h->inject_timeout = 0;
-    }
+    A.tx_extra = take_injection(h, TMA_);
     constexpr int TXP = StepShape<TH, R, PH>::TX;
     const int tiles = ((h->G.X + TXP - 1) / TXP) * ((h->G.Y + TY - 1) / TY);
     k<<<tiles, NTP, smem, h->stream>>>(M ? *M : phase_maps(h, A, PH == PH_B ? TM_B : TM_A), A);
@@ -439,11 +424,7 @@ struct Fused {
       auto k = step_kernel_pipe<TH, R>;
       static unsigned long long done = 0;
       set_smem(k, SH::SLOTS * SH::SLOT, done);
-      A.tx_extra = 0;
-      if (h->inject_timeout) {
-        A.tx_extra = 16;
-        h->inject_timeout = 0;
-      }
+      A.tx_extra = take_injection(h, true);
       const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + SH::TY - 1) / SH::TY);
       k<<<std::min(tiles, h->num_sms), SH::NT, SH::SLOTS * SH::SLOT, h->stream>>>(phase_maps(h, A, TM_B), A);
       CK(cudaGetLastError());
@@ -619,7 +600,6 @@ struct Fused {
     for (int v = 0; v < 2; ++v) h->tune_ms[M_S23][v] = h->tune_ms[M_S1][0] + h->tune_ms[M_S4][h->use_pipe[M_S4]];
     if (uses_pipe(M_GRAD)) {
       FlowArgs<R> F = base_args(h);
-      F.mode = M_GRAD;
       F.phi = (const R*)h->field;
       F.out_l = (R*)h->l[0];
       const bool tma = encode_tile_map(&F.tm_phi, F.phi, sizeof(R), h->G.X, h->G.Y, TH::NF);
@@ -636,7 +616,6 @@ struct Fused {
 
   static int gradient(ss_handle* h, const void* field, void* eg, void* l_out, int raw = 0) {
     FlowArgs<R> A = base_args(h);
-    A.mode = M_GRAD;
     A.grad_raw = raw;
     A.phi = (const R*)field;
     A.out_eg = (R*)eg;
@@ -670,11 +649,10 @@ struct Fused {
       const bool tma = encode_tile_map(&M.phi, field, sizeof(R), h->G.X, h->G.Y, TH::NF, false, TXA, TY);
       return tma ? launch_phase<true, PH_E>(h, S, &M) : launch_phase<false, PH_E>(h, S);
     }
-    FlowArgs<R> A = base_args(h);
-    A.mode = M_ENERGY;
-    A.phi = (const R*)field;
-    const bool tma = encode_tile_map(&A.tm_phi, field, sizeof(R), h->G.X, h->G.Y, TH::NF);
-    return launch(h, A, tma);
+    ObsList L{};
+    L.n = 1;
+    L.comps = ~0u;
+    return observe(h, field, nullptr, true, L);
   }
 
   // FP64 energy of the sphere projection of `field` (element type R).  The FP64 copy
@@ -688,13 +666,33 @@ struct Fused {
     return Fused<TH, double>::energy(h, copy);
   }
 
+  static unsigned obs_comps(int kind, int which) {
+    return kind == D_ENERGY ? ~0u : kind == D_CHARGE ? TH::charge_comps(which) : TH::coupling_comps(which);
+  }
+  // the quantities of L (comps filled in) of `field`: their sums (reduce) and, for one of
+  // them, its density (nullable)
+  static int observe(const ss_handle* h, const void* field, double* dens, bool reduce, const ObsList& L,
+                     bool allow_tma = true) {
+    CUtensorMap map{};
+    const bool tma = allow_tma && encode_tile_map(&map, field, sizeof(R), h->G.X, h->G.Y, TH::NF);
+    auto go = [&](auto k, unsigned long long& done) -> int {
+      set_smem(k, BUF, done);
+      k<<<h->nblocks, NT, BUF, h->stream>>>(map, (const R*)field, dens, reduce ? h->partial : nullptr, h->st, L, h->G,
+                                            h->P, h->wait_cycles, take_injection(h, tma));
+      CK(cudaGetLastError());
+      return SS_OK;
+    };
+    static unsigned long long done_tma = 0, done_plain = 0;
+    return tma ? go(observe_kernel<TH, R, TX, TY, NT, true>, done_tma)
+               : go(observe_kernel<TH, R, TX, TY, NT, false>, done_plain);
+  }
   static int density(ss_handle* h, const void* field, double* dens, bool reduce, int kind, int which) {
-    auto k = density_kernel<TH, R, TX, TY, NT>;
-    set_smem(k, BUF, smem_done_density);
-    k<<<h->nblocks, NT, BUF, h->stream>>>((const R*)field, dens, reduce ? h->partial : nullptr, h->st, kind, which,
-                                           h->G, h->P);
-    CK(cudaGetLastError());
-    return SS_OK;
+    ObsList L{};
+    L.n = 1;
+    L.kind[0] = kind;
+    L.which[0] = which;
+    L.comps = obs_comps(kind, which);
+    return observe(h, field, dens, reduce, L);
   }
 
   static int rk4_stage(ss_handle* h, void* k_out, const void* vel, const void* l_in, void* temp, const void* field,
@@ -943,7 +941,7 @@ int ss_create(int theory, const int32_t* p_i, int n_i, const double* p_f, int n_
   h->elem = precision == SS_FP32 ? 4 : 8;
   // the step's phases tile at 8 rows where 16 do not fit: up to twice the tiles
   const long long tiles = (long long)((h->G.X + TX - 1) / TX) * ((h->G.Y + TY - 1) / TY);
-  if (tiles > 0x3fffffffLL) {
+  if (tiles > 0x1fffffffLL) {
     delete h;
     return fail(SS_ERR_ARG, "lattice too large");
   }
@@ -1352,6 +1350,41 @@ int ss_charge(ss_handle* h, const void* field, int which, double* out) {
   return scalar_result(h, out);
 }
 
+int ss_observables(ss_handle* h, const void* field, int n, const int* kinds, const int* which, double* out) {
+  int rc = check_bound(h);
+  if (rc) return rc;
+  if (!field || !kinds || !which || !out) return fail(SS_ERR_ARG, "NULL argument");
+  if (n < 1 || n > OBS_MAX) return fail(SS_ERR_ARG, "n must be 1..%d", OBS_MAX);
+  ObsList L{};
+  for (int i = 0; i < n; ++i) {
+    if (kinds[i] < SS_OBS_ENERGY || kinds[i] > SS_OBS_COUPLING) return fail(SS_ERR_ARG, "unknown kind %d", kinds[i]);
+    if (kinds[i] == SS_OBS_CHARGE && !theory_has_charge(h->theory, which[i]))
+      return fail(SS_ERR_ARG, "charge %d not defined for theory %d", which[i], h->theory);
+    if (kinds[i] == SS_OBS_COUPLING && !theory_has_coupling(h->theory, which[i]))
+      return fail(SS_ERR_ARG, "coupling %d not defined for theory %d", which[i], h->theory);
+    if (h->precision != SS_FP32 && kinds[i] == SS_OBS_ENERGY) {
+      // the flow's own FP64 energy (ss_energy): equal to the last step's to the last bit
+      if ((rc = ss_energy(h, field, out + i))) return rc;
+      continue;
+    }
+    L.kind[L.n] = kinds[i];
+    L.which[L.n++] = which[i];
+  }
+  if (!L.n) return SS_OK;
+  rc = dispatch(h, [&](auto* tag) -> int {
+    using TH = std::remove_pointer_t<decltype(tag)>;
+    for (int i = 0; i < L.n; ++i) L.comps |= Fused<TH, float>::obs_comps(L.kind[i], L.which[i]);
+    if (h->precision == SS_FP32) return Fused<TH, float>::observe(h, field, nullptr, true, L);
+    return Fused<TH, double>::observe(h, field, nullptr, true, L);
+  });
+  if (rc) return rc;
+  StepState s;
+  if ((rc = read_state(h, &s))) return rc;
+  for (int i = 0, k = 0; i < n; ++i)
+    if (!(h->precision != SS_FP32 && kinds[i] == SS_OBS_ENERGY)) out[i] = s.scalars[k++];
+  return s.status ? take_status(h) : SS_OK;
+}
+
 int ss_coupling_grad(ss_handle* h, const void* field, int coupling, double* out) {
   int rc = check_bound(h);
   if (rc) return rc;
@@ -1525,16 +1558,11 @@ extern "C" int ss_energy_noalloc(int theory, const int32_t* p_i, int n_i, const 
   CK(cudaMemsetAsync(h.st, 0, sizeof(StepState), h.stream));
   rc = dispatch(&h, [&](auto* tag) -> int {
     using TH = std::remove_pointer_t<decltype(tag)>;
-    if (precision == SS_FP32) {
-      FlowArgs<float> A = Fused<TH, float>::base_args(&h);
-      A.mode = M_ENERGY;
-        A.phi = (const float*)field;
-      return Fused<TH, float>::template launch_mode<false, M_ENERGY>(&h, A);
-    }
-    FlowArgs<double> A = Fused<TH, double>::base_args(&h);
-    A.mode = M_ENERGY;
-    A.phi = (const double*)field;
-    return Fused<TH, double>::template launch_mode<false, M_ENERGY>(&h, A);
+    ObsList L{};
+    L.n = 1;
+    L.comps = ~0u;
+    return precision == SS_FP32 ? Fused<TH, float>::observe(&h, field, nullptr, true, L, false)
+                                : Fused<TH, double>::observe(&h, field, nullptr, true, L, false);
   });
   if (rc) return rc;
   StepState s;

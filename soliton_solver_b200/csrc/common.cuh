@@ -62,6 +62,7 @@ struct StepState {
   int status;                    // 0 ok, SS_ERR_NONFINITE on a non-finite reduction
   int pad;
   double scalar;                 // result slot of single reductions (energy / charge / coupling)
+  double scalars[4];             // results of a pass over several quantities
   unsigned int bar, leave;       // grid barrier of the cooperative step: arrivals, CTAs that left
   unsigned long long err2[2];    // its err maxima of even and odd steps (ordered encoding)
 };

@@ -11,8 +11,8 @@
 
 namespace ssb {
 
-// Modes of flow_kernel (M_GRAD, M_ENERGY) and indices of the staging variants: M_S1, M_S2 the
-// step's phase A, M_S3, M_S4 its phase B, M_S23 kept for the pinning interface.
+// Indices of the staging variants: M_GRAD the gradient hook, M_S1, M_S2 the step's phase A,
+// M_S3, M_S4 its phase B; M_ENERGY and M_S23 are kept for the pinning interface.
 enum FlowMode { M_GRAD = 0, M_S1 = 1, M_S2 = 2, M_S3 = 3, M_S4 = 4, M_ENERGY = 5, M_S23 = 6 };
 constexpr int N_FLOW_MODES = 7;
 enum { ST_TIMEOUT = 6 };
@@ -28,9 +28,7 @@ struct FlowArgs {
   const R* phi;        // the staged field
   R* out_l;            // M_GRAD: l_out (nullable)
   R* out_eg;           // M_GRAD: energy gradient (nullable)
-  double* partial;     // per-block energy partials
   StepState* st;
-  int mode;
   int grad_raw;           // M_GRAD: unprojected, not halo-zeroed dE/dphi with true saddle rows
   long long wait_cycles;  // bound of every mbarrier wait (clock64 cycles)
   unsigned tx_extra;      // test hook: bytes the barrier expects beyond what is loaded (normally 0)
@@ -373,66 +371,6 @@ __device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int 
   }
 }
 
-// FP64 energy of the staged field (T_1 = phi): first derivatives from the exact
-// differences f(x+k) - f(x-k) of the stored values, evaluated in FP64.
-template <class TH, typename R, int TX, int TY, int NT, bool FAST, typename E = R>
-__device__ __forceinline__ double energy_tile(const FlowArgs<R>& A, const E* T, int x0, int y0) {
-  using TS = TileShape<TX, TY, NT>;
-  using V = typename PairOf<E>::type;
-  using SV = ScaledValue<E>;
-  constexpr int NF = TH::NF;
-  constexpr int PAIRS = TY / 2;
-  constexpr int RPP = NT / PAIRS;
-  const Grid& G = A.G;
-  const double c23x = FD::c23 * G.ihx * SV::SCALE, c12x = FD::c12 * G.ihx * SV::SCALE;
-  const double c23y = FD::c23 * G.ihy * SV::SCALE, c12y = FD::c12 * G.ihy * SV::SCALE;
-  const int j = threadIdx.x % PAIRS;
-  const int lxg = threadIdx.x / PAIRS;
-  double e_acc = 0.0;
-  V chk(0.0f);  // stays zero unless a centre value is Inf or NaN
-#pragma unroll 1
-  for (int pass = 0; pass < TX / RPP; ++pass) {
-    const int lx = lxg + pass * RPP;
-    const int gx = x0 + lx, gy = y0 + 2 * j;
-    bool v1 = true;
-    Masks m0{true, true, true}, m1{true, true, true};
-    if (!FAST) {
-      if (gx >= G.X || gy >= G.Y) continue;
-      v1 = gy + 1 < G.Y;
-      m0 = site_masks(G, gx, gy);
-      m1 = site_masks(G, gx, gy + 1);
-    }
-    const int toff = (lx + 2) * TS::HY + TS::YOFF + 2 * j;
-    Jet1<double, NF> J0, J1;
-#pragma unroll
-    for (int a = 0; a < NF; ++a) {
-      const E* row = T + a * TS::PLANE + toff;
-      // six y values cover both sites' y stencils; converted once
-      const V Ap = ld_pair(row - 2), B = ld_pair(row), C = ld_pair(row + 2);
-      chk = vfma(B, V(0.0f), chk);
-      const double y_2 = SV::get(Lanes<V>::get(Ap, 0)), y_1 = SV::get(Lanes<V>::get(Ap, 1));
-      const double y0v = SV::get(Lanes<V>::get(B, 0)), y1v = SV::get(Lanes<V>::get(B, 1));
-      const double y2 = SV::get(Lanes<V>::get(C, 0)), y3 = SV::get(Lanes<V>::get(C, 1));
-      const V xp1 = ld_pair(row + TS::HY), xm1 = ld_pair(row - TS::HY);
-      const V xp2 = ld_pair(row + 2 * TS::HY), xm2 = ld_pair(row - 2 * TS::HY);
-#pragma unroll
-      for (int l = 0; l < 2; ++l) {
-        Jet1<double, NF>& J = l ? J1 : J0;
-        const Masks& m = l ? m1 : m0;
-        const double ddx = (c23x * (SV::get(Lanes<V>::get(xp1, l)) - SV::get(Lanes<V>::get(xm1, l))) -
-                            c12x * (SV::get(Lanes<V>::get(xp2, l)) - SV::get(Lanes<V>::get(xm2, l))));
-        const double ddy = l ? (c23y * (y2 - y0v) - c12y * (y3 - y_1)) : (c23y * (y1v - y_1) - c12y * (y2 - y_2));
-        J.f[a] = (l ? y1v : y0v) * SV::SCALE;
-        J.dx[a] = m.x ? ddx : 0.0;
-        J.dy[a] = m.y ? ddy : 0.0;
-      }
-    }
-    e_acc += TH::energy(J0, A.P, G.dA);
-    if (v1) e_acc += TH::energy(J1, A.P, G.dA);
-  }
-  return e_acc + (double)(Lanes<V>::get(chk, 0) + Lanes<V>::get(chk, 1));
-}
-
 // Shared scratch of the tile kernels besides the staged tile.
 template <int NT>
 struct StageShared {
@@ -442,90 +380,63 @@ struct StageShared {
   int am_last;
 };
 
-// The sum of the blocks' energy partials by the last of `nblk` blocks (fixed order).
-template <int NT>
-__device__ __forceinline__ void energy_reduction(double e_acc, double* partial, StepState* st, int blk, int nblk,
-                                                 double* red, double* sh_s, double* sh_c, int& am_last) {
-  const double bs = block_sum_fixed<NT>(e_acc, red);
+template <class TH, typename R, int TX, int TY, int NT>
+__device__ __forceinline__ void grad_any_tile(const FlowArgs<R>& A, const R* T, int x0, int y0) {
+  const Grid& G = A.G;
+  if ((G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
+      y0 + TY - 1 <= G.Y - G.halo - 2)
+    grad_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
+  else
+    grad_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
+}
+
+// One halo tile of `map` (all components) into T by the CTA: TMA load, bounded wait.  Returns
+// false in every thread, with the status recorded, when the wait ran out.
+template <int NF, typename R, int TX, int TY, int NT>
+__device__ __forceinline__ bool stage_tma(R* T, const CUtensorMap* map, uint64_t* bar, int x0, int y0, unsigned tx_extra,
+                                          long long limit, StepState* st) {
+  using TS = TileShape<TX, TY, NT>;
   if (threadIdx.x == 0) {
-    partial[blk] = bs;
-    __threadfence();
-    const unsigned t = atomicAdd(&st->ticket, 1u);
-    am_last = (t == (unsigned)nblk - 1u);
+    mbar_init(bar, 1);
+    mbar_expect_tx(bar, (uint32_t)(sizeof(R) * NF * TS::PLANE) + tx_extra);
+    tma_load_3d(T, map, y0 - TS::YOFF, x0 - 2, 0, bar);
   }
   __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  const double E = fixed_order_sum<NT>(partial, nblk, sh_s, sh_c);
-  if (threadIdx.x == 0) {
-    st->scalar = E;
-    if (!isfinite(E)) st->status = 3;
-    st->ticket = 0u;
+  const bool ok = __syncthreads_and(mbar_wait_bounded(bar, 0, limit));
+  if (!ok) {
+    if (threadIdx.x == 0) atomicExch(&st->status, (int)ST_TIMEOUT);
+    mbar_wait_bounded(bar, 0, limit);
   }
+  return ok;
 }
 
-template <class TH, typename R, int TX, int TY, int NT, int MODE>
-__device__ __forceinline__ void flow_compute(const FlowArgs<R>& A, const R* T, int x0, int y0, double& e_acc) {
-  const Grid& G = A.G;
-  const bool fast = (G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
-                    y0 + TY - 1 <= G.Y - G.halo - 2;
-  if constexpr (MODE == M_ENERGY) {
-    if (fast)
-      e_acc += energy_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
-    else
-      e_acc += energy_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
-  } else {
-    if (fast)
-      grad_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
-    else
-      grad_tile<TH, R, TX, TY, NT, false>(A, T, x0, y0);
-  }
-}
-
-// One tile per CTA: the gradient hook (M_GRAD) or the exact energy (M_ENERGY).
-template <class TH, typename R, int TX, int TY, int NT, bool TMA, int MODE>
-__global__ void __launch_bounds__(NT, (sizeof(R) == 8 && MODE == M_ENERGY && TH::NF <= 4 ? 2 : 1))
-    flow_kernel(const __grid_constant__ FlowArgs<R> A) {
+// The gradient hook, one tile per CTA.
+template <class TH, typename R, int TX, int TY, int NT, bool TMA>
+__global__ void __launch_bounds__(NT) flow_kernel(const __grid_constant__ FlowArgs<R> A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ StageShared<NT> S;
+  __shared__ uint64_t bar;
   R* T = reinterpret_cast<R*>(smem_raw);
   const int tiles_y = (A.G.Y + TY - 1) / TY;
   const int x0 = (blockIdx.x / tiles_y) * TX, y0 = (blockIdx.x % tiles_y) * TY;
   if constexpr (TMA) {
-    using TS = TileShape<TX, TY, NT>;
-    if (threadIdx.x == 0) {
-      mbar_init(&S.bar, 1);
-      mbar_expect_tx(&S.bar, (uint32_t)(sizeof(R) * TH::NF * TS::PLANE) + A.tx_extra);
-      tma_load_3d(T, &A.tm_phi, y0 - TS::YOFF, x0 - 2, 0, &S.bar);
-    }
-    __syncthreads();
-    const bool ok = __syncthreads_and(mbar_wait_bounded(&S.bar, 0, A.wait_cycles));
-    if (!ok) {
-      if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
-      mbar_wait_bounded(&S.bar, 0, A.wait_cycles);
-      return;
-    }
+    if (!stage_tma<TH::NF, R, TX, TY, NT>(T, &A.tm_phi, &bar, x0, y0, A.tx_extra, A.wait_cycles, A.st)) return;
   } else {
     stage_plain<TH::NF, R, TX, TY, NT>(T, A.G, A.phi, x0, y0);
     __syncthreads();
   }
-  double e_acc = 0.0;
-  flow_compute<TH, R, TX, TY, NT, MODE>(A, T, x0, y0, e_acc);
-  if constexpr (MODE == M_ENERGY)
-    energy_reduction<NT>(e_acc, A.partial, A.st, blockIdx.x, gridDim.x, S.red, S.sh_s, S.sh_c, S.am_last);
+  grad_any_tile<TH, R, TX, TY, NT>(A, T, x0, y0);
 }
 
 // Persistent, TMA-pipelined form of flow_kernel (FP32 fields): one 512-thread CTA per SM
 // walks the tiles blockIdx.x, blockIdx.x + gridDim.x, ... through a ring of STAGES
 // shared-memory slots, so the bulk tensor loads of the next tiles are in flight while the
-// current tile is computed.  Energy partials are per CTA in tile order.
-template <class TH, typename R, int TX, int TY, int NT, int MODE, int STAGES>
+// current tile is computed.
+template <class TH, typename R, int TX, int TY, int NT, int STAGES>
 __global__ void __launch_bounds__(NT, 1) flow_kernel_pipe(const __grid_constant__ FlowArgs<R> A) {
   using TS = TileShape<TX, TY, NT>;
   constexpr int SLOT = TH::NF * TS::PLANE;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* ring = reinterpret_cast<R*>(smem_raw);
-  __shared__ StageShared<NT> S;
   __shared__ __align__(8) uint64_t full[STAGES];
   const Grid& G = A.G;
   const int tiles_y = (G.Y + TY - 1) / TY;
@@ -544,7 +455,6 @@ __global__ void __launch_bounds__(NT, 1) flow_kernel_pipe(const __grid_constant_
     }
   }
   __syncthreads();
-  double e_acc = 0.0;
   int k = 0;
   // tile coordinates advanced without a division per tile
   const int dq = gridDim.x / tiles_y, dr = gridDim.x % tiles_y;
@@ -563,7 +473,7 @@ __global__ void __launch_bounds__(NT, 1) flow_kernel_pipe(const __grid_constant_
       }
       return;
     }
-    flow_compute<TH, R, TX, TY, NT, MODE>(A, ring + slot * SLOT, tx * TX, ty * TY, e_acc);
+    grad_any_tile<TH, R, TX, TY, NT>(A, ring + slot * SLOT, tx * TX, ty * TY);
     tx += dq;
     ty += dr;
     if (ty >= tiles_y) {
@@ -576,76 +486,113 @@ __global__ void __launch_bounds__(NT, 1) flow_kernel_pipe(const __grid_constant_
       if (nt < ntiles) issue(slot, nt);
     }
   }
-  if constexpr (MODE == M_ENERGY)
-    energy_reduction<NT>(e_acc, A.partial, A.st, blockIdx.x, gridDim.x, S.red, S.sh_s, S.sh_c, S.am_last);
 }
 
 // ---------------------------------------------------------------------------
-// densities (energy, charges, coupling partials) with optional reduction
+// observables: energy, charges and coupling partials, as sums and as densities
 // ---------------------------------------------------------------------------
 enum DensityKind { D_ENERGY = 0, D_CHARGE = 1, D_COUPLING = 2 };
+constexpr int OBS_MAX = 4;  // quantities per pass
+struct ObsList {
+  int n;
+  int kind[OBS_MAX], which[OBS_MAX];
+  unsigned comps;  // components whose jets any of them reads
+};
 
-template <class TH, typename R, int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT)
-    density_kernel(const R* __restrict__ phi, double* density, double* partial, StepState* st, int kind,
-                   int which, Grid G, Phys P) {
+// n quantities of the stored field in one pass: FP64 jets (values and masked first
+// derivatives) of the components they need, the theory's points on them, one fixed-order
+// compensated sum each (partial: n * gridDim.x slots, nullable) and, for n = 1, the density.
+// A thread owns four adjacent rows of one column and takes them two at a time, so that the
+// two rows' x neighbours are read and converted once.  Bound for FP32 fields by the
+// conversions (XU pipe: 16 per clock and SM) and FP64 arithmetic.
+template <class TH, typename R, int TX, int TY, int NT, bool TMA>
+__global__ void __launch_bounds__(NT, (TH::NF <= 4 ? 3 : 2))
+    observe_kernel(const __grid_constant__ CUtensorMap map, const R* __restrict__ phi, double* density, double* partial,
+                   StepState* st, const __grid_constant__ ObsList L, const __grid_constant__ Grid G,
+                   const __grid_constant__ Phys P, long long wait_cycles, unsigned tx_extra) {
   using TS = TileShape<TX, TY, NT>;
-  constexpr int NF = TH::NF;
+  constexpr int NF = TH::NF, ROWS = TX / (NT / TY), PER = 2;
+  static_assert(NT % TY == 0 && ROWS % PER == 0, "column mapping");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* tile = reinterpret_cast<R*>(smem_raw);
-  __shared__ double red[NT / 32];
-  __shared__ double sh_s[NT / 32], sh_c[NT / 32];
-  __shared__ int am_last;
+  __shared__ StageShared<NT> S;
   const int tiles_y = (G.Y + TY - 1) / TY;
   const int x0 = (blockIdx.x / tiles_y) * TX;
   const int y0 = (blockIdx.x % tiles_y) * TY;
-  stage_plain<NF, R, TX, TY, NT>(tile, G, phi, x0, y0);
-  __syncthreads();
-  const Inv<double> ivd(G);
-  const int ly = threadIdx.x % TY;
-  const int lxg = threadIdx.x / TY;
-  double acc = 0.0;
+  if constexpr (TMA) {
+    if (!stage_tma<NF, R, TX, TY, NT>(tile, &map, &S.bar, x0, y0, tx_extra, wait_cycles, st)) return;
+  } else {
+    stage_plain<NF, R, TX, TY, NT>(tile, G, phi, x0, y0);
+    __syncthreads();
+  }
+  const double ihx = G.ihx, ihy = G.ihy;
+  const int ly = threadIdx.x % TY, gy = y0 + ly;
+  double acc[OBS_MAX] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
-  for (int s = 0; s < TS::SITES_PER_THREAD; ++s) {
-    const int lx = lxg + s * TS::ROWS_PER_PASS;
-    const int gx = x0 + lx, gy = y0 + ly;
-    if (gx >= G.X || gy >= G.Y) continue;
-    const Masks mk = site_masks(G, gx, gy);
+  for (int s = 0; s < ROWS; s += PER) {
+    const int lx = (threadIdx.x / TY) * ROWS + s;
+    if (x0 + lx >= G.X || gy >= G.Y) break;
     const R* base = tile + (lx + 2) * TS::HY + (ly + TS::YOFF);
-    Jet1<double, NF> J1;
+    Jet1<double, NF> J[PER];
 #pragma unroll
     for (int a = 0; a < NF; ++a) {
+      if (!((L.comps >> a) & 1u)) {
+#pragma unroll
+        for (int p = 0; p < PER; ++p) J[p].f[a] = J[p].dx[a] = J[p].dy[a] = 0.0;
+        continue;
+      }
       const R* pa = base + a * TS::PLANE;
-      auto accs = [pa](int dx, int dy) -> double { return (double)pa[dx * TS::HY + dy]; };
-      fill_jet1_comp<double>(accs, mk, ivd, J1.f[a], J1.dx[a], J1.dy[a]);
+      double x[PER + 4];
+#pragma unroll
+      for (int k = 0; k < PER + 4; ++k) x[k] = (double)pa[(k - 2) * TS::HY];
+#pragma unroll
+      for (int p = 0; p < PER; ++p) {
+        const R* pr = pa + p * TS::HY;
+        const Masks mk = site_masks(G, x0 + lx + p, gy);
+        const double dx = d1_stencil<double>(x[p], x[p + 1], x[p + 3], x[p + 4], ihx);
+        const double dy = d1_stencil<double>((double)pr[-2], (double)pr[-1], (double)pr[1], (double)pr[2], ihy);
+        J[p].f[a] = x[p + 2];
+        J[p].dx[a] = mk.x ? dx : 0.0;
+        J[p].dy[a] = mk.y ? dy : 0.0;
+      }
     }
-    double v;
-    if (kind == D_ENERGY)
-      v = TH::energy(J1, P, G.dA);
-    else if (kind == D_CHARGE)
-      v = TH::charge(J1, P, which, G.dA);
-    else
-      v = TH::coupling(J1, P, which, G.dA);
-    if (density) density[(long long)gx * G.Y + gy] = v;
-    acc += v;
+#pragma unroll
+    for (int p = 0; p < PER; ++p) {
+      const int gx = x0 + lx + p;
+      if (gx >= G.X) break;
+#pragma unroll
+      for (int q = 0; q < OBS_MAX; ++q) {
+        if (q >= L.n) break;
+        const double v = L.kind[q] == D_ENERGY   ? TH::energy(J[p], P, G.dA)
+                         : L.kind[q] == D_CHARGE ? TH::charge(J[p], P, L.which[q], G.dA)
+                                                 : TH::coupling(J[p], P, L.which[q], G.dA);
+        if (q == 0 && density) density[(long long)gx * G.Y + gy] = v;
+        acc[q] += v;
+      }
+    }
   }
   if (!partial) return;
-  const double bs = block_sum_fixed<NT>(acc, red);
+  for (int q = 0; q < L.n; ++q) {
+    const double bs = block_sum_fixed<NT>(q == 0 ? acc[0] : q == 1 ? acc[1] : q == 2 ? acc[2] : acc[3], S.red);
+    if (threadIdx.x == 0) partial[(long long)q * gridDim.x + blockIdx.x] = bs;
+  }
   if (threadIdx.x == 0) {
-    partial[blockIdx.x] = bs;
     __threadfence();
     const unsigned t = atomicAdd(&st->ticket, 1u);
-    am_last = (t == gridDim.x - 1);
+    S.am_last = (t == gridDim.x - 1);
   }
   __syncthreads();
-  if (!am_last) return;
+  if (!S.am_last) return;
   __threadfence();
-  const double E = fixed_order_sum<NT>(partial, gridDim.x, sh_s, sh_c);
-  if (threadIdx.x == 0) {
-    st->scalar = E;
-    if (!isfinite(E)) st->status = 3;
-    st->ticket = 0u;
+  for (int q = 0; q < L.n; ++q) {
+    const double E = fixed_order_sum<NT>(partial + (long long)q * gridDim.x, gridDim.x, S.sh_s, S.sh_c);
+    if (threadIdx.x == 0) {
+      st->scalars[q] = E;
+      if (q == 0) st->scalar = E;
+      if (!isfinite(E)) st->status = 3;
+    }
   }
+  if (threadIdx.x == 0) st->ticket = 0u;
 }
 
 // do_rk4_step_kernel (core/integrator.py:51-96)

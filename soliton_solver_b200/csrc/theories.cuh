@@ -182,6 +182,9 @@ struct ChiralMagnet {
     return 0.0;
   }
   static constexpr bool has_coupling(int w) { return w == CP_COUP_K || w == CP_COUP_H || w == CP_COUP_MU; }
+  // components a charge / coupling partial reads
+  static constexpr unsigned charge_comps(int w) { return w == CH_SKYRMION ? 7u : 3u; }
+  static constexpr unsigned coupling_comps(int w) { return w == CP_COUP_MU ? 8u : 4u; }
 };
 
 // ===========================================================================
@@ -399,6 +402,8 @@ struct BabySkyrme {
     return 0.0;
   }
   static constexpr bool has_coupling(int w) { return w == CP_KAPPA || w == CP_MPI; }
+  static constexpr unsigned charge_comps(int) { return 7u; }
+  static constexpr unsigned coupling_comps(int) { return 7u; }
 };
 
 // ===========================================================================
@@ -497,6 +502,8 @@ struct GinzburgLandau {
     return (u * u - psi_sq) * (u * u - psi_sq) / 8.0 * dA;
   }
   static constexpr bool has_coupling(int w) { return w == CP_LAMBDA; }
+  static constexpr unsigned charge_comps(int) { return 3u; }
+  static constexpr unsigned coupling_comps(int) { return 12u; }
 };
 
 // ===========================================================================
@@ -624,6 +631,8 @@ struct Anisotropic {
   static constexpr bool has_charge(int which) { return which == CH_VORTEX; }
   __device__ static inline double coupling(const Jet1<double, NF>&, const Phys&, int, double) { return 0.0; }
   static constexpr bool has_coupling(int) { return false; }
+  static constexpr unsigned charge_comps(int) { return 3u; }
+  static constexpr unsigned coupling_comps(int) { return 0u; }
 };
 
 }  // namespace ssb
