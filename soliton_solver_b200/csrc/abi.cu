@@ -420,18 +420,14 @@ struct Fused {
   }
   static int launch_phase_pipe(const ss_handle* h, StepArgs<R>& A) {
     using SH = PipeShape<TH, R>;
-    if constexpr (SH::OK) {
-      auto k = step_kernel_pipe<TH, R>;
-      static unsigned long long done = 0;
-      set_smem(k, SH::SLOTS * SH::SLOT, done);
-      A.tx_extra = take_injection(h, true);
-      const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + SH::TY - 1) / SH::TY);
-      k<<<std::min(tiles, h->num_sms), SH::NT, SH::SLOTS * SH::SLOT, h->stream>>>(phase_maps(h, A, TM_B), A);
-      CK(cudaGetLastError());
-      return SS_OK;
-    } else {
-      return launch_phase<true, PH_B>(h, A);
-    }
+    auto k = step_kernel_pipe<TH, R>;
+    static unsigned long long done = 0;  // one per instantiation
+    set_smem(k, SH::SLOTS * SH::SLOT, done);
+    A.tx_extra = take_injection(h, true);
+    const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + SH::TY - 1) / SH::TY);
+    k<<<std::min(tiles, SH::CTAS * h->num_sms), SH::NT, SH::SLOTS * SH::SLOT, h->stream>>>(phase_maps(h, A, TM_B), A);
+    CK(cudaGetLastError());
+    return SS_OK;
   }
   template <int PH>
   static int launch_phase(const ss_handle* h, StepArgs<R>& A) {
@@ -585,7 +581,7 @@ struct Fused {
     A.vel_out = (R*)h->vel2;
     int rc = SS_OK;
     for (int m : {(int)M_S1, (int)M_S4}) {
-      const bool two = m == M_S4 && PipeShape<TH, R>::OK;
+      const bool two = m == M_S4;
       for (int v = 0; v < 2 && !rc; ++v) {
         if (two) h->use_pipe[M_S3] = h->use_pipe[M_S4] = v;
         set_input(h, A, 0);

@@ -60,8 +60,9 @@ struct StepArgs {
 
 // Tile rows, threads and resident CTAs per SM of each phase (tiles are TX x 64 sites, a
 // warp owns rows).  Registers follow from the CTAs: 64 for the chiral magnet's phase A, 80
-// for the other FP32 theories with up to four components, else 128 (no spills but for 92-104
-// bytes in the FP32 phase B); the s+id model's FP64 stencils take up to 254 and one CTA.
+// for the phase A of the other FP32 theories with up to four components and for the baby
+// Skyrme phase B, else 128 (at most 48 bytes of spills); the s+id model's FP64 stencils take
+// up to 254 and one CTA.
 // Phase B stages four halo buffers: 16 rows where two CTAs' buffers fit an SM (FP32, up to
 // four components), else 8.
 template <class TH, typename R, int PH>
@@ -70,7 +71,11 @@ struct StepShape {
   static constexpr int BYTES = (int)sizeof(R) * TH::NF;  // per site
   static constexpr bool F32 = sizeof(R) == 4;
   static constexpr int TX = BYTES <= (PH == PH_B ? 16 : 32) ? 16 : 8;
-  static constexpr int CTAS = TH::NF > 4 ? (F32 ? 2 : 1) : !F32 || PH == PH_B ? 2 : PH == PH_E || TH::S1_CTAS == 4 ? 4 : 3;
+  static constexpr int CTAS = TH::NF > 4                       ? (F32 ? 2 : 1)
+                              : !F32                           ? 2
+                              : PH == PH_B                     ? (TH::NF <= 3 ? 3 : 2)
+                              : PH == PH_E || TH::S1_CTAS == 4 ? 4
+                                                               : 3;
 };
 // halo buffers staged per phase (TMA: phi; V; l1, l2.  Plain loads combine on the way in: T1, T2 / T3, T4)
 template <int PH, bool TMA>
@@ -275,6 +280,7 @@ __device__ __forceinline__ void second_half(const StepArgs<R>& A, const R* T3, c
       gstore<V, R>(A.phi_out + a * N + sidx, Pn[a], FAST, v1);
       gstore<V, R>(A.vel_out + a * N + sidx, Vn[a], FAST, v1);
     }
+    asm volatile("" ::: "memory");  // one row at a time: the next row's loads would spill
   }
   err_max = fmax(err_max, (double)emax);
 }
@@ -527,24 +533,22 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
   step_reductions<NT, R, PH>(A, S, e_acc, err_max, tile, nblk);
 }
 
-// Persistent phase B (FP32, TMA staging, up to four components): one 512-thread CTA per SM
-// walks the tiles b, b + gridDim.x, ... through a ring of two or three staged tiles (92 KB
-// each for four components), so the loads of the next tile are in flight while one is
-// computed and the set-up of a CTA is paid once.  4096^2 chiral magnet, FP32: 377 us against
-// 447 us one tile per CTA (764 against 916 instructions per warp and row; issue-bound at 45%
-// with 16 warps per SM; HBM floor 246 us); 2048^2 baby Skyrme 114 against 122 us.  Phase A
-// is better one tile per CTA (246 against 260 us at 4096^2: its two buffers leave room for
-// four CTAs per SM).
+// Persistent phase B (TMA staging): the resident CTAs walk the tiles b, b + gridDim.x, ...
+// through one staged tile each, so that a CTA's set-up is paid once and its SM's other CTAs
+// compute while it waits for a tile.  us, one tile per CTA -> persistent: 4096^2 chiral magnet
+// FP32 441 -> 361 (HBM floor 246; issue-bound), 2048^2 baby Skyrme FP32 118 -> 95, 1024^2
+// Abelian Higgs FP64 79 -> 66, 1024^2 s+id FP32 64 -> 53.  A ring of two tiles under one
+// 512-thread CTA per SM took 391 us (chiral), 112 us (baby Skyrme).  Phase A gains nothing
+// (four CTAs per SM already hide its waits: 241 against 244 us) and stays one tile per CTA.
 template <class TH, typename R>
-struct PipeShape {
-  static constexpr int TX = 16, TY = 64, NT = 512;
-  static constexpr size_t SLOT = 4 * tile_buf_bytes<R, TH::NF, TX, TY>();
-  static constexpr int SLOTS = (int)(220 * 1024 / SLOT);
-  static constexpr bool OK = sizeof(R) == 4 && SLOTS >= 2;
+struct PipeShape : StepShape<TH, R, PH_B> {
+  using SH = StepShape<TH, R, PH_B>;
+  static constexpr size_t SLOT = 4 * tile_buf_bytes<R, TH::NF, SH::TX, SH::TY>();
+  static constexpr int SLOTS = 1;
 };
 
 template <class TH, typename R>
-__global__ void __launch_bounds__((PipeShape<TH, R>::NT), 1)
+__global__ void __launch_bounds__((PipeShape<TH, R>::NT), (PipeShape<TH, R>::CTAS))
     step_kernel_pipe(const __grid_constant__ StepMaps M, const __grid_constant__ StepArgs<R> A) {
   using SH = PipeShape<TH, R>;
   using V = typename PairOf<R>::type;
