@@ -179,6 +179,10 @@ int ss_gradient(ss_handle *h, const void *field, void *energy_gradient, void *l_
  * gradient of the total energy up to O(h^4) and boundary terms; it is the backward
  * of the autograd energy.  No reference counterpart (new capability). */
 int ss_energy_gradient(ss_handle *h, const void *field, void *grad);
+/* The backward of the total energy in one pass: *grad_E * dA * ss_energy_gradient(field)
+ * into `grad` (element type of the handle), the factor *grad_E * dA rounded to that type
+ * first; grad_E is a device double.  Asynchronous.  No reference counterpart. */
+int ss_energy_vjp(ss_handle *h, const void *field, const double *grad_E, void *grad);
 /* Per-site energy x dA (double).  Replaces compute_energy_kernel
  * (e.g. theories/chiral_magnet/kernels.py:219-251). */
 int ss_energy_density(ss_handle *h, const void *field, double *density);

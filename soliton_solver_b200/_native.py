@@ -106,6 +106,7 @@ _SIG = {
     "ss_debug_wait_timeout": ([_P, ctypes.c_longlong, _I], _I),
     "ss_gradient": ([_P, _P, _P, _P], _I),
     "ss_energy_gradient": ([_P, _P, _P], _I),
+    "ss_energy_vjp": ([_P, _P, _P, _P], _I),
     "ss_energy_density": ([_P, _P, _P], _I),
     "ss_energy": ([_P, _P, ctypes.POINTER(_D)], _I),
     "ss_energy_projected": ([_P, _P, ctypes.POINTER(_D)], _I),

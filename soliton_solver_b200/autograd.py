@@ -13,6 +13,7 @@ torch's dispatcher (fake tensors, opcheck); solvers are passed by an integer key
 
   soliton_b200::energy(field, key) -> f64 scalar          ss_energy (differentiable)
   soliton_b200::energy_gradient(field, key) -> like field  ss_energy_gradient
+  soliton_b200::energy_vjp(field, grad_E, key) -> like field  ss_energy_vjp (the energy's backward)
   soliton_b200::gradient(field, key) -> like field         ss_gradient (projected EG)
   soliton_b200::charge(field, key, which) -> f64 scalar    ss_charge
   soliton_b200::coupling_grad(field, key, name) -> f64     ss_coupling_grad
@@ -48,7 +49,7 @@ def register(solver) -> int:
 @torch.library.custom_op("soliton_b200::energy", mutates_args=())
 def energy_op(field: torch.Tensor, key: int) -> torch.Tensor:
     s = _SOLVERS[key]
-    return torch.tensor(s.energy(field.contiguous()), dtype=torch.float64, device=field.device)
+    return torch.full((), s.energy(field.contiguous()), dtype=torch.float64, device=field.device)
 
 
 @energy_op.register_fake
@@ -64,6 +65,17 @@ def energy_gradient_op(field: torch.Tensor, key: int) -> torch.Tensor:
 
 @energy_gradient_op.register_fake
 def _(field, key):
+    return torch.empty_like(field)
+
+
+@torch.library.custom_op("soliton_b200::energy_vjp", mutates_args=())
+def energy_vjp_op(field: torch.Tensor, grad_E: torch.Tensor, key: int) -> torch.Tensor:
+    s = _SOLVERS[key]
+    return s.energy_vjp(field.contiguous(), grad_E.to(torch.float64).contiguous())
+
+
+@energy_vjp_op.register_fake
+def _(field, grad_E, key):
     return torch.empty_like(field)
 
 
@@ -131,6 +143,8 @@ def _setup(ctx, inputs, output):
 
 def _backward(ctx, grad_E):
     (field,) = ctx.saved_tensors
+    if not torch.is_grad_enabled():  # no graph of the backward itself: one pass
+        return energy_vjp_op(field, grad_E, ctx.key), None
     s = _SOLVERS[ctx.key]
     g = energy_gradient_op(field, ctx.key)
     dA = float(s.p_f[4])

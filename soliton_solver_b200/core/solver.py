@@ -8,6 +8,7 @@ device and of the solver's element type.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 
@@ -23,6 +24,9 @@ _DENSITIES = {"higgs": nat.SS_DENSITY_HIGGS, "higgs1": nat.SS_DENSITY_HIGGS1, "h
 _COUPLINGS = {"kappa": nat.SS_COUPLING_KAPPA, "mpi": nat.SS_COUPLING_MPI, "Lambda": nat.SS_COUPLING_LAMBDA,
               "coup_K": nat.SS_COUPLING_COUP_K, "coup_h": nat.SS_COUPLING_COUP_H,
               "coup_mu": nat.SS_COUPLING_COUP_MU}
+
+
+_HERE = contextlib.nullcontext()
 
 
 def _ptr(t) -> int | None:
@@ -64,6 +68,11 @@ class Solver:
         self.stream = stream
         self._bind(None, None)
 
+    def _on_device(self):
+        """Context with the solver's device current (nothing to do where it already is)."""
+        i = self.device.index
+        return _HERE if i is None or i == torch.cuda.current_device() else torch.cuda.device(i)
+
     # ------------------------------------------------------------------ binding
     def _stream_handle(self):
         if self.stream is not None:
@@ -71,7 +80,7 @@ class Solver:
         return int(torch.cuda.current_stream(self.device).cuda_stream)
 
     def _bind(self, field, velocity):
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_bind(self._h, _ptr(field), _ptr(velocity), self.workspace.data_ptr(),
                                         self.workspace.numel(), self._stream_handle()))
         self.field, self.velocity = field, velocity
@@ -103,7 +112,7 @@ class Solver:
         """Advance the bound buffers; returns (energy_traj, err_traj) numpy arrays."""
         E = np.empty(max(n_steps, 0))
         err = np.empty(max(n_steps, 0))
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_step(self._h, int(n_steps), float(prev_energy), E.ctypes.data, err.ctypes.data))
         return E, err
 
@@ -114,7 +123,7 @@ class Solver:
                 self._check(t, torch.float64)
                 if t.numel() < n_steps:
                     raise ValueError("trajectory buffer shorter than n_steps")
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_step_async(self._h, int(n_steps), float(prev_energy), _ptr(energy_traj),
                                               _ptr(err_traj)))
 
@@ -126,12 +135,12 @@ class Solver:
                 if t.numel() < n_steps:
                     raise ValueError("trajectory buffer shorter than n_steps")
         self._graph_bufs = (energy_traj, err_traj)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_graph_create(self._h, int(n_steps), _ptr(energy_traj), _ptr(err_traj)))
 
     def replay(self):
         """Launch the captured graph on the bound stream (no host synchronisation)."""
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_graph_launch(self._h))
 
     @property
@@ -146,7 +155,7 @@ class Solver:
         the step's first kernel, which has one form; 3 and 4: its second) and {6: (ms of both
         kernels, the same, pinned value)}."""
         ms = np.zeros(14, dtype=np.float32)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_autotune(self._h, int(iters), ms.ctypes.data))
         return {m: (float(ms[2 * m]), float(ms[2 * m + 1]), int(self._lib.ss_get_variant(self._h, m)))
                 for m in (1, 2, 3, 4, 6)}
@@ -158,7 +167,7 @@ class Solver:
         self._check(field)
         if velocity is not None:
             self._check(velocity)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_initialize(self._h, _ptr(field), _ptr(velocity), int(mode), int(ansatz),
                                               float(rotation), float(vortex_number)))
 
@@ -167,7 +176,7 @@ class Solver:
         """Add a skyrmion (chiral magnet, baby Skyrme) or a vortex (Abelian Higgs, s+id)
         centred on lattice point (pxi, pxj) to `field`; see ss_insert_soliton."""
         self._check(field)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_insert_soliton(self._h, _ptr(field), int(pxi), int(pxj), int(ansatz),
                                                   int(vortex), float(rotation)))
 
@@ -193,7 +202,7 @@ class Solver:
         for t in (field, energy_gradient, l_out):
             if t is not None:
                 self._check(t)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_gradient(self._h, _ptr(field), _ptr(energy_gradient), _ptr(l_out)))
 
     def energy_gradient(self, field, out=None):
@@ -201,8 +210,19 @@ class Solver:
         self._check(field)
         out = out if out is not None else torch.empty_like(field)
         self._check(out)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_energy_gradient(self._h, _ptr(field), _ptr(out)))
+        return out
+
+    def energy_vjp(self, field, grad_E, out=None):
+        """grad_E * dA * dE/dphi per site (grad_E: FP64 scalar tensor on the device), the
+        backward of the energy in one pass (see ss_energy_vjp)."""
+        self._check(field)
+        self._check(grad_E, torch.float64)
+        out = out if out is not None else torch.empty_like(field)
+        self._check(out)
+        with self._on_device():
+            nat.check(self._lib.ss_energy_vjp(self._h, _ptr(field), _ptr(grad_E), _ptr(out)))
         return out
 
     def energy_gradient_exact(self, field, out=None, minus_stencil: bool = False):
@@ -213,7 +233,7 @@ class Solver:
         self._check(field)
         out = out if out is not None else torch.empty(self.nf * self.N, dtype=torch.float64, device=self.device)
         self._check(out, torch.float64)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_energy_gradient_exact(self._h, _ptr(field), _ptr(out), 1 if minus_stencil else 0))
         return out
 
@@ -231,7 +251,7 @@ class Solver:
     def energy(self, field) -> float:
         self._check(field)
         out = ctypes.c_double()
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_energy(self._h, _ptr(field), ctypes.byref(out)))
         return out.value
 
@@ -240,7 +260,7 @@ class Solver:
         (ss_energy_projected).  Uses the workspace's l buffers: not during a step."""
         self._check(field)
         out = ctypes.c_double()
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_energy_projected(self._h, _ptr(field), ctypes.byref(out)))
         return out.value
 
@@ -248,14 +268,14 @@ class Solver:
         self._check(field)
         out = out if out is not None else torch.empty(self.N, dtype=torch.float64, device=self.device)
         self._check(out, torch.float64)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_energy_density(self._h, _ptr(field), _ptr(out)))
         return out
 
     def charge(self, field, which: str) -> float:
         self._check(field)
         out = ctypes.c_double()
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_charge(self._h, _ptr(field), _CHARGES[which], ctypes.byref(out)))
         return out.value
 
@@ -263,7 +283,7 @@ class Solver:
         self._check(field)
         out = out if out is not None else torch.empty(self.N, dtype=torch.float64, device=self.device)
         self._check(out, torch.float64)
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_charge_density(self._h, _ptr(field), _CHARGES[which], _ptr(out)))
         return out
 
@@ -277,7 +297,7 @@ class Solver:
                 raise ValueError(f"convert needs contiguous FP32/FP64 tensors of {self.nf * self.N} entries on "
                                  f"{self.device}")
         code = {torch.float32: nat.SS_FP32, torch.float64: nat.SS_FP64}
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_convert_field(self._h, _ptr(src), code[src.dtype], _ptr(dst), code[dst.dtype],
                                                  1 if project else 0))
         return dst
@@ -292,14 +312,14 @@ class Solver:
         self._check(out, torch.float64)
         if out.numel() < n:
             raise ValueError(f"output buffer needs {n} entries")
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_field_density(self._h, _ptr(field), _DENSITIES[kind], _ptr(out)))
         return out
 
     def coupling_grad(self, field, which: str) -> float:
         self._check(field)
         out = ctypes.c_double()
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_coupling_grad(self._h, _ptr(field), _COUPLINGS[which], ctypes.byref(out)))
         return out.value
 
@@ -315,18 +335,18 @@ class Solver:
             kinds = (ctypes.c_int * len(part))(*[k for k, _ in code])
             which = (ctypes.c_int * len(part))(*[w for _, w in code])
             vals = (ctypes.c_double * len(part))()
-            with torch.cuda.device(self.device):
+            with self._on_device():
                 nat.check(self._lib.ss_observables(self._h, _ptr(field), len(part), kinds, which, vals))
             out.update(zip(part, vals))
         return out
 
     def rk4_stage(self, k_out, velocity, l_in, temp, field, k_prev, factor: float):
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_rk4_stage(self._h, _ptr(k_out), _ptr(velocity), _ptr(l_in), _ptr(temp),
                                              _ptr(field), _ptr(k_prev), float(factor)))
 
     def rk4_finalize(self, velocity, field, k1, k2, k3, k4, l1, l2, l3, l4):
-        with torch.cuda.device(self.device):
+        with self._on_device():
             nat.check(self._lib.ss_rk4_finalize(self._h, _ptr(velocity), _ptr(field), *(
                 _ptr(t) for t in (k1, k2, k3, k4, l1, l2, l3, l4))))
 

@@ -32,6 +32,7 @@ namespace {
 constexpr int TX = 16, TY = 64, NT = 256;  // fused tile: 16 x 64 sites, 256 threads
 constexpr int COOP_MAX_TILES = 4096;        // energy partials kept for the cooperative step
 constexpr int TRAJ_CAP = 1024;              // device trajectory slots used by ss_step
+constexpr size_t STAGE_TAIL = 64 + 192;      // bytes of ss_handle::host_stage behind the trajectories: status, state
 constexpr size_t ALIGN = 256;
 // Tensor maps of a bound handle (halo boxes): phi and V of the caller's buffers and of the
 // workspace's pair in the tile shapes of phases A and B, l1 and l2 in phase B's
@@ -138,9 +139,9 @@ struct ss_handle {
   mutable int inject_timeout = 0;  // test hook, consumed by the next flow launch
   cudaGraphExec_t graph = nullptr;  // captured n-step relaxation (ss_graph_create)
   const double* force = nullptr;    // FP64 flows: field added to the gradient rows (ss_set_forcing)
-  // mapped page-locked staging of ss_step, written by the kernels themselves: the energy
-  // and err trajectories of one chunk and the status of the call (allocated on the first
-  // ss_step; host_stage_dev is its device address)
+  // mapped page-locked staging: the energy and err trajectories of one ss_step chunk and the
+  // status of the call, written by the kernels themselves, and behind them the step state as
+  // read back by read_state (allocated on first use; host_stage_dev is its device address)
   double* host_stage = nullptr;
   double* host_stage_dev = nullptr;
   ~ss_handle() {
@@ -610,9 +611,11 @@ struct Fused {
     return rc;
   }
 
-  static int gradient(ss_handle* h, const void* field, void* eg, void* l_out, int raw = 0) {
+  static int gradient(ss_handle* h, const void* field, void* eg, void* l_out, int raw = 0,
+                      const double* scale = nullptr) {
     FlowArgs<R> A = base_args(h);
     A.grad_raw = raw;
+    A.scale = scale;
     A.phi = (const R*)field;
     A.out_eg = (R*)eg;
     A.out_l = (R*)l_out;
@@ -837,9 +840,22 @@ int coop_plan(const ss_handle* h) {
   return got;
 }
 
+// the handle's page-locked staging (mapped; allocated on first use)
+static_assert(sizeof(StepState) <= 192, "fits behind the staged status");
+int host_staging(ss_handle* h) {
+  if (h->host_stage) return SS_OK;
+  CK(cudaHostAlloc((void**)&h->host_stage, 2 * TRAJ_CAP * sizeof(double) + STAGE_TAIL, cudaHostAllocMapped));
+  CK(cudaHostGetDevicePointer((void**)&h->host_stage_dev, h->host_stage, 0));
+  return SS_OK;
+}
+
 int read_state(ss_handle* h, StepState* out) {
-  CK(cudaMemcpyAsync(out, h->st, sizeof(StepState), cudaMemcpyDeviceToHost, h->stream));
+  int rc = host_staging(h);  // page-locked: the copy needs no intermediate buffer
+  if (rc) return rc;
+  StepState* s = reinterpret_cast<StepState*>(h->host_stage + 2 * TRAJ_CAP + 8);
+  CK(cudaMemcpyAsync(s, h->st, sizeof(StepState), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  *out = *s;
   return SS_OK;
 }
 
@@ -1096,10 +1112,7 @@ int ss_step(ss_handle* h, int n_steps, double prev_energy, double* energy_traj, 
   if (n_steps == 0) return take_status(h);
   // each chunk's trajectories and status are written by the kernels into mapped
   // page-locked memory: one synchronisation per chunk and no copies
-  if (!h->host_stage) {
-    CK(cudaHostAlloc((void**)&h->host_stage, 2 * TRAJ_CAP * sizeof(double) + 64, cudaHostAllocMapped));
-    CK(cudaHostGetDevicePointer((void**)&h->host_stage_dev, h->host_stage, 0));
-  }
+  if ((rc = host_staging(h))) return rc;
   double* hE = h->host_stage;
   double* hErr = h->host_stage + TRAJ_CAP;
   volatile int* hstatus = reinterpret_cast<volatile int*>(h->host_stage + 2 * TRAJ_CAP);
@@ -1161,6 +1174,18 @@ int ss_energy_gradient(ss_handle* h, const void* field, void* grad) {
     using TH = std::remove_pointer_t<decltype(tag)>;
     if (h->precision == SS_FP32) return Fused<TH, float>::gradient(h, field, grad, nullptr, 1);
     return Fused<TH, double>::gradient(h, field, grad, nullptr, 1);
+  });
+}
+
+int ss_energy_vjp(ss_handle* h, const void* field, const double* grad_E, void* grad) {
+  int rc = check_bound(h);
+  if (rc) return rc;
+  if (!field || !grad || !grad_E) return fail(SS_ERR_ARG, "NULL argument");
+  if (h->precision == SS_PLAIN_FP64) return fail(SS_ERR_ARG, "ss_energy_vjp needs SS_FP32 or SS_FP64");
+  return dispatch(h, [&](auto* tag) -> int {
+    using TH = std::remove_pointer_t<decltype(tag)>;
+    if (h->precision == SS_FP32) return Fused<TH, float>::gradient(h, field, grad, nullptr, 1, grad_E);
+    return Fused<TH, double>::gradient(h, field, grad, nullptr, 1, grad_E);
   });
 }
 

@@ -29,6 +29,7 @@ struct FlowArgs {
   R* out_l;            // M_GRAD: l_out (nullable)
   R* out_eg;           // M_GRAD: energy gradient (nullable)
   StepState* st;
+  const double* scale;    // grad_raw: rows times *scale * dA, rounded to R (nullable: unscaled)
   int grad_raw;           // M_GRAD: unprojected, not halo-zeroed dE/dphi with true saddle rows
   long long wait_cycles;  // bound of every mbarrier wait (clock64 cycles)
   unsigned tx_extra;      // test hook: bytes the barrier expects beyond what is loaded (normally 0)
@@ -331,6 +332,7 @@ __device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int 
   const long long N = G.N;
   const PairCoef<V> kc(G);
   const V mdt(grid_k<S>(G, GK_MDT));
+  const V scale(A.scale ? (S)*A.scale * (S)G.dA : (S)1);
   const int j = threadIdx.x % PAIRS;
   const int lxg = threadIdx.x / PAIRS;
 #pragma unroll 1
@@ -356,6 +358,10 @@ __device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int 
       // functional derivative of the energy: no halo zeroing, no projection, and rows the
       // flow stores scaled (saddle fields) converted to dE/dphi
       TH::true_rows(g, A.P);
+      if (A.scale) {
+#pragma unroll
+        for (int a = 0; a < NF; ++a) g[a] = g[a] * scale;
+      }
 #pragma unroll
       for (int a = 0; a < NF; ++a) {
         if (A.out_eg) gstore<V, R>(A.out_eg + a * N + sidx, g[a], FAST, v1);
