@@ -50,7 +50,8 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
         return LIB
     os.makedirs(LIBDIR, exist_ok=True)
     tmp = LIB + ".tmp"
-    cmd = [_nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
+    # --split-compile=0: the kernels of the one translation unit are optimised on all cores
+    cmd = [_nvcc(), *ARCH, "-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "--split-compile=0",
            "-Xcompiler", "-fPIC", "-shared", "-cudart", "shared",
            "-Xlinker", "-rpath,/usr/local/cuda/lib64",
            "-I", INCLUDE, "-I", CSRC, "-o", tmp]

@@ -518,6 +518,25 @@ struct Fused {
     return SS_OK;
   }
 
+  static int launch_a2(const ss_handle* h, const StepArgs<R>& A) {
+    constexpr size_t smem = step_smem<TH, R, PH_A, false>();
+    constexpr int CX = StepShape<TH, R, PH_A>::TX;
+    const long long tiles = (long long)((h->G.X + CX - 1) / CX) * ((h->G.Y + TY - 1) / TY);
+    auto go = [&](auto k, unsigned long long& done) -> int {
+      set_smem(k, smem, done);
+      k<<<(int)std::min<long long>(tiles, 2 * h->num_sms), StepShape<TH, R, PH_A>::NT, smem, h->stream>>>(A);
+      CK(cudaGetLastError());
+      return SS_OK;
+    };
+    static unsigned long long done_fused = 0, done_plain = 0;
+    return h->tma ? go(step_a2_kernel<TH, R, true>, done_fused) : go(step_a2_kernel<TH, R, false>, done_plain);
+  }
+  // flows whose energy rises (psi of the chiral magnet's demag field is maximised): nearly
+  // every step is arrested, and phase A predicts it
+  static bool saddle_flow(const ss_handle* h) {
+    return h->P.k[0] && h->G.killkinen;
+  }
+
   // n flow steps of the bound buffers, in place; trajectories to device arrays (nullable)
   // status_out (nullable, device-visible): the finish kernel copies the call's status there
   static int step(ss_handle* h, int n, double prev, double* E_dev, double* err_dev, int* status_out = nullptr) {
@@ -534,8 +553,12 @@ struct Fused {
       A.init_state = s == 0;
       A.prev_energy = prev;
       set_input(h, A, cur);
+      if constexpr (std::is_same_v<TH, ChiralMagnet>) A.predict = s > 0 && saddle_flow(h);
       if ((rc = launch_phase<PH_A>(h, A))) return rc;
       A.init_state = 0;
+      if constexpr (std::is_same_v<TH, ChiralMagnet>) {
+        if (A.predict && (rc = launch_a2(h, A))) return rc;
+      }
       // B: phi' and V' into the other pair, err
       A.err_idx = s;
       A.phi_out = (R*)(cur ? h->field : h->phi2);
@@ -544,6 +567,7 @@ struct Fused {
       if ((rc = launch_phase<PH_B>(h, A))) return rc;
     }
     // trailing energy of the final field and its arrest test; phi back to the caller's buffer
+    A.predict = 0;
     A.with_energy = A.arrest_update = 1;
     A.E_idx = n - 1;
     A.phi_out = cur ? (R*)h->field : nullptr;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__((BatchShape<TH, R, PH, SMALL>::NT), (BatchShap
       const int tiles_y = (I.G.Y + TY - 1) / TY;
       mbar_init(&S.bar, 1);
       issue_step_tile<TH, R, TX, TY, NT, PH>(reinterpret_cast<R*>(smem_raw), tm_phi, tm_vel, tm_l1, tm_l1 + 1,
-                                             (tile / tiles_y) * TX, (tile % tiles_y) * TY, &S.bar, I.st, 0u);
+                                             (tile / tiles_y) * TX, (tile % tiles_y) * TY, &S.bar, I.st, 0u, 0);
     }
   }
   {  // the lattice's parameters into shared memory (word copy)
@@ -98,6 +98,7 @@ __global__ void __launch_bounds__((BatchShape<TH, R, PH, SMALL>::NT), (BatchShap
     A.with_energy = B.with_energy;
     A.arrest_update = B.arrest_update;
     A.init_state = B.init_state;
+    A.predict = 0;
     A.prev_energy = B.prev_energy ? B.prev_energy[inst] : NAN;
     A.wait_cycles = B.wait_cycles;
     A.tx_extra = 0;

@@ -60,9 +60,11 @@ struct StepState {
   unsigned int ticket;           // last-block-done counter, reset by the last block
   int arrest;                    // 1: treat the velocity as zero in this step's stages 2-4
   int status;                    // 0 ok, SS_ERR_NONFINITE on a non-finite reduction
-  int pad;
+  int streak;                    // arrested steps in a row (saddle flows: predicts the next)
   double scalar;                 // result slot of single reductions (energy / charge / coupling)
   double scalars[4];             // results of a pass over several quantities
+  int l2_missing;                // phase A left l2 out on a prediction that did not hold
+  int pad;
   unsigned int bar, leave;       // grid barrier of the cooperative step: arrivals, CTAs that left
   unsigned long long err2[2];    // its err maxima of even and odd steps (ordered encoding)
 };

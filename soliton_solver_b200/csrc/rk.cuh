@@ -19,13 +19,17 @@
 // decides (V = 0) is applied by phase B: V = 0 means T2 = T1, so l2 = l1 and phase B takes
 // l1 for l2 (and loads neither V nor l2); phase A's l2, computed before the decision, is
 // dropped.
+// Saddle flows (the chiral magnet with demag: its psi is maximised, E rises) arrest nearly
+// every step.  After two arrested steps in a row phase A expects the next: it reads phi alone
+// and writes l1 alone, and should the energy fall after all, phase A2 (a launch that returns
+// at once otherwise) supplies l2 before phase B: 6 words and three gradients per arrested step.
 #pragma once
 
 #include "flow.cuh"
 
 namespace ssb {
 
-enum StepPhase { PH_A = 0, PH_B = 1, PH_E = 2 };
+enum StepPhase { PH_A = 0, PH_B = 1, PH_E = 2, PH_A2 = 3 };
 
 // TMA maps of a phase's inputs: halo boxes of its tile shape
 struct StepMaps {
@@ -51,6 +55,7 @@ struct StepArgs {
   int with_energy;    // A, E: reduce the energy of phi
   int arrest_update;  // after the energy: arrest = killkinen && E > E_last; E_last = E
   int init_state;     // first phase A of a call: arrest = 0 and (unless NaN) E_last = prev_energy
+  int predict;        // A: leave l2 out after two arrested steps in a row
   double prev_energy;
   long long wait_cycles;  // bound of every mbarrier wait (clock64 cycles)
   unsigned tx_extra;      // test hook: bytes the barrier expects beyond what is loaded (normally 0)
@@ -80,7 +85,7 @@ struct StepShape {
 // halo buffers staged per phase (TMA: phi; V; l1, l2.  Plain loads combine on the way in: T1, T2 / T3, T4)
 template <int PH, bool TMA>
 __host__ __device__ constexpr int step_buffers() {
-  return PH == PH_E ? 1 : (PH == PH_B && TMA) ? 4 : 2;
+  return PH == PH_E ? 1 : (PH == PH_B && TMA) ? 4 : 2;  // A, A2: phi, V
 }
 template <class TH, typename R, int PH, bool TMA>
 __host__ __device__ constexpr size_t step_smem() {
@@ -137,10 +142,11 @@ __device__ __forceinline__ double pair_energy(const Jet<V, TH::NF>& J, const Phy
   }
 }
 
-// Phase A (l1, l2 and the energy) or phase E (the energy, and a copy of phi) of a staged tile.
+// Phase A (l1, l2 and the energy; skip: no l2), A2 (l2) or E (the energy, and a copy of phi) of
+// a staged tile.
 template <class TH, typename R, int TX, int TY, int NT, bool FAST, int PH>
 __device__ __forceinline__ void first_half(const StepArgs<R>& A, const R* T1, const R* T2, int x0, int y0,
-                                           double* e_acc) {
+                                           bool skip, double* e_acc) {
   using TS = TileShape<TX, TY, NT>;
   using V = typename PairOf<R>::type;
   using S = typename ScalarOf<V>::type;
@@ -179,10 +185,13 @@ __device__ __forceinline__ void first_half(const StepArgs<R>& A, const R* T1, co
       }
     } else {
       V g[NF];
-      pair_gradient<TH, V, R, TS::HY, TS::PLANE, FAST>(A, T1, toff, kc, m0, m1, gx, gy, sidx, v1, J, g);
-      if (e_acc) e_sum += pair_energy<TH, V, R>(J, A.P, v1, chk);
+      if constexpr (PH == PH_A) {
+        pair_gradient<TH, V, R, TS::HY, TS::PLANE, FAST>(A, T1, toff, kc, m0, m1, gx, gy, sidx, v1, J, g);
+        if (e_acc) e_sum += pair_energy<TH, V, R>(J, A.P, v1, chk);
 #pragma unroll
-      for (int a = 0; a < NF; ++a) gstore<V, R>(A.out_l1 + a * N + sidx, mdt * g[a], FAST, v1);
+        for (int a = 0; a < NF; ++a) gstore<V, R>(A.out_l1 + a * N + sidx, mdt * g[a], FAST, v1);
+        if (skip) continue;
+      }
       pair_gradient<TH, V, R, TS::HY, TS::PLANE, FAST>(A, T2, toff, kc, m0, m1, gx, gy, sidx, v1, J, g);
 #pragma unroll
       for (int a = 0; a < NF; ++a) gstore<V, R>(A.out_l2 + a * N + sidx, mdt * g[a], FAST, v1);
@@ -287,8 +296,9 @@ __device__ __forceinline__ void second_half(const StepArgs<R>& A, const R* T3, c
 
 // Plain-load staging of a phase (row pitch not a multiple of 16 bytes): T1 = phi and T2 (A),
 // T1 (E) or T3 and T4 (B; an arrested step takes V = 0 and l1 for l2) into D0 and D1.  Every
-// thread issues the loads of one component plane before it combines them.
-template <int NF, typename R, int TX, int TY, int NT, int PH>
+// thread issues the loads of one component plane before it combines them.  FUSED_T2: T2 rounded
+// as in TMA-staged tiles.
+template <int NF, typename R, int TX, int TY, int NT, int PH, bool FUSED_T2 = false>
 __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int x0, int y0, bool arrest) {
   using TS = TileShape<TX, TY, NT>;
   constexpr int KM = (TS::PLANE + NT - 1) / NT;
@@ -327,18 +337,20 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
         D1[a * TS::PLANE + i] = vfma(dt, vfma((R)0.5, l2, v[k]), p[k]);
       } else {
         D0[a * TS::PLANE + i] = p[k];
-        if constexpr (PH == PH_A) D1[a * TS::PLANE + i] = stage_t2<R>(p[k], v[k], dt);
+        if constexpr (PH == PH_A)
+          D1[a * TS::PLANE + i] = FUSED_T2 ? vfma(grid_k<R>(G, GK_HDT), v[k], p[k]) : stage_t2<R>(p[k], v[k], dt);
       }
     }
   }
 }
 
 // Expect and issue the TMA loads of one tile (one thread, barrier initialised).  Phase B
-// leaves V and l2 out of an arrested step; phi and l1 are issued before the flag is read.
+// leaves V and l2 out of an arrested step, phase A leaves V out of a predicted one; phi and l1
+// are issued before the flag is read.
 template <class TH, typename R, int TX, int TY, int NT, int PH>
 __device__ __forceinline__ void issue_step_tile(R* B0, const CUtensorMap* tm_phi, const CUtensorMap* tm_vel,
                                                 const CUtensorMap* tm_l1, const CUtensorMap* tm_l2, int x0, int y0,
-                                                uint64_t* bar, const StepState* st, unsigned tx_extra) {
+                                                uint64_t* bar, const StepState* st, unsigned tx_extra, int predict) {
   using TS = TileShape<TX, TY, NT>;
   constexpr int BUF = TH::NF * TS::PLANE;
   constexpr uint32_t bytes = (uint32_t)(sizeof(R) * BUF);
@@ -347,8 +359,9 @@ __device__ __forceinline__ void issue_step_tile(R* B0, const CUtensorMap* tm_phi
   if constexpr (PH == PH_E) {
     mbar_expect_tx(bar, bytes + tx_extra);
   } else if constexpr (PH == PH_A) {
-    tma_load_3d(B0 + BUF, tm_vel, c0, c1, 0, bar);
-    mbar_expect_tx(bar, 2 * bytes + tx_extra);
+    const bool skip = predict && __ldcg(&st->streak) >= 2;
+    if (!skip) tma_load_3d(B0 + BUF, tm_vel, c0, c1, 0, bar);
+    mbar_expect_tx(bar, (skip ? 1 : 2) * bytes + tx_extra);
   } else {
     tma_load_3d(B0 + 2 * BUF, tm_l1, c0, c1, 0, bar);
     const bool arrest = __ldcg(&st->arrest) != 0;
@@ -395,8 +408,11 @@ __device__ __forceinline__ void step_reductions(const StepArgs<R>& A, StageShare
       if (!isfinite(E)) st->status = 3;
       if (A.E_traj && A.E_idx >= 0) A.E_traj[A.E_idx] = E;
       if (A.arrest_update) {
-        st->arrest = (A.G.killkinen && E > st->E_last) ? 1 : 0;
+        const int arrest = (A.G.killkinen && E > st->E_last) ? 1 : 0;
+        st->arrest = arrest;
         st->E_last = E;
+        st->l2_missing = PH == PH_A && A.predict && st->streak >= 2 && !arrest;
+        st->streak = arrest ? min(st->streak + 1, 2) : 0;
       }
     }
   }
@@ -414,6 +430,7 @@ __device__ __forceinline__ void combine_tile(const Grid& G, R* B0, bool arrest, 
   R* B1 = B0 + BUF;
   const V half(0.5), hdt(grid_k<R>(G, GK_HDT)), dtv(grid_k<R>(G, GK_DT));
   if constexpr (PH == PH_A) {
+    if (arrest) return;  // phase A: no l2 wanted
     for (int i = 4 * threadIdx.x; i < BUF; i += 4 * NT) {
       V p0, p1, v0, v1;
       ld_quad(B0 + i, p0, p1);
@@ -460,7 +477,7 @@ __device__ __forceinline__ void combine_tile(const Grid& G, R* B0, bool arrest, 
   }
 }
 
-// The stencils of a staged (and combined) tile.
+// The stencils of a staged (and combined) tile.  `arrest`: phase B's arrest, phase A's skip.
 template <class TH, typename R, int TX, int TY, int NT, bool TMA, int PH, class CL>
 __device__ __forceinline__ void compute_tile(const StepArgs<R>& A, const R* B0, const CL& C, int x0, int y0,
                                              bool arrest, double& e_acc, double& err_max) {
@@ -477,9 +494,9 @@ __device__ __forceinline__ void compute_tile(const StepArgs<R>& A, const R* B0, 
   } else {
     double* ep = A.with_energy ? &e_acc : nullptr;
     if (fast)
-      first_half<TH, R, TX, TY, NT, true, PH>(A, B0, B0 + BUF, x0, y0, ep);
+      first_half<TH, R, TX, TY, NT, true, PH>(A, B0, B0 + BUF, x0, y0, arrest, ep);
     else
-      first_half<TH, R, TX, TY, NT, false, PH>(A, B0, B0 + BUF, x0, y0, ep);
+      first_half<TH, R, TX, TY, NT, false, PH>(A, B0, B0 + BUF, x0, y0, arrest, ep);
   }
 }
 
@@ -487,6 +504,7 @@ template <typename R>
 __device__ __forceinline__ void step_init(const StepArgs<R>& A, int cta) {
   if (A.init_state && cta == 0 && threadIdx.x == 0) {
     A.st->arrest = 0;
+    A.st->l2_missing = 0;
     if (!isnan(A.prev_energy)) A.st->E_last = A.prev_energy;
   }
 }
@@ -511,11 +529,13 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
     if (!issued) {
       if (threadIdx.x == 0) {
         mbar_init(&S.bar, 1);
-        issue_step_tile<TH, R, TX, TY, NT, PH>(B0, tm_phi, tm_vel, tm_l1, tm_l2, x0, y0, &S.bar, A.st, A.tx_extra);
+        issue_step_tile<TH, R, TX, TY, NT, PH>(B0, tm_phi, tm_vel, tm_l1, tm_l2, x0, y0, &S.bar, A.st, A.tx_extra,
+                                               A.predict);
       }
       __syncthreads();
     }
     if constexpr (PH == PH_B) arrest = __ldcg(&A.st->arrest) != 0;
+    if constexpr (PH == PH_A) arrest = A.predict && __ldcg(&A.st->streak) >= 2;
     const bool ok = __syncthreads_and(mbar_wait_bounded(&S.bar, 0, A.wait_cycles));
     if (!ok) {
       if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
@@ -527,6 +547,7 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
     if constexpr (PH == PH_B) arrest = __ldcg(&A.st->arrest) != 0;
     stage_step_plain<NF, R, TX, TY, NT, PH>(B0, B0 + BUF, A, x0, y0, arrest);
     __syncthreads();
+    if constexpr (PH == PH_A) arrest = A.predict && __ldcg(&A.st->streak) >= 2;
   }
   double e_acc = 0.0, err_max = -INFINITY;
   compute_tile<TH, R, TX, TY, NT, TMA, PH>(A, B0, C, x0, y0, arrest, e_acc, err_max);
@@ -637,6 +658,28 @@ __global__ void __launch_bounds__((StepShape<TH, R, PH>::NT), (StepShape<TH, R, 
   __shared__ StageShared<SH::NT> S;
   step_tile<TH, R, SH::TX, SH::TY, SH::NT, TMA, PH>(A, &M.phi, &M.vel, &M.l1, &M.l2, blockIdx.x, gridDim.x,
                                                     smem_raw, S);
+}
+
+// Phase A2: l2 where phase A left it out on a prediction that did not hold, else nothing.  A
+// resident grid walks the tiles with plain loads (it runs once in a while, and an idle launch
+// must cost no more than its CTAs' start: 28 us with one CTA per tile at 4096^2).
+template <class TH, typename R, bool FUSED_T2>
+__global__ void __launch_bounds__((StepShape<TH, R, PH_A>::NT)) step_a2_kernel(const __grid_constant__ StepArgs<R> A) {
+  using SH = StepShape<TH, R, PH_A>;
+  constexpr int TX = SH::TX, TY = SH::TY, NT = SH::NT, NF = TH::NF;
+  if (__ldcg(&A.st->l2_missing) == 0) return;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  R* D0 = reinterpret_cast<R*>(smem_raw);
+  R* D1 = D0 + NF * TileShape<TX, TY, NT>::PLANE;
+  const Grid& G = A.G;
+  const int tiles_y = (G.Y + TY - 1) / TY, ntiles = ((G.X + TX - 1) / TX) * tiles_y;
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const int x0 = (t / tiles_y) * TX, y0 = (t % tiles_y) * TY;
+    stage_step_plain<NF, R, TX, TY, NT, PH_A, FUSED_T2>(D0, D1, A, x0, y0, false);
+    __syncthreads();
+    first_half<TH, R, TX, TY, NT, false, PH_A2>(A, D0, D1, x0, y0, false, nullptr);
+    __syncthreads();
+  }
 }
 
 // End of a call: a pending arrest left by the trailing energy pass (V = 0), the copy of V out

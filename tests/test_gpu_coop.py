@@ -104,3 +104,44 @@ def test_cooperative_steps_on_concurrent_streams():
     for g, w in zip(got, want):
         np.testing.assert_array_equal(g[2], w[2])
         np.testing.assert_array_equal(g[0], w[0])
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("Y", [192, 150], ids=["tma", "plain"])
+def test_mispredicted_arrest(prec, Y):
+    """Saddle flow as two launches: two arrested steps make the next step's first kernel leave
+    l2 out; the energy of the smooth field falls instead, so l2 comes from the extra kernel.
+    Against one-step calls, which never predict.  FP32 bitwise; FP64 as above."""
+    case = _case("Chiral magnet", 256, Y, 5)
+    tid, p_i, p_f, F, V = case
+    dt = torch.float32 if prec == "fp32" else torch.float64
+    # a long-wave texture at rest with a weak demag coupling runs downhill for many steps
+    p_f = p_f.copy()
+    p_f[8] = 1e-3
+    x, y = np.meshgrid(np.arange(256), np.arange(Y), indexing="ij")
+    m = np.stack([0.4 * np.sin(0.2 * x), 0.4 * np.cos(0.15 * y), np.ones_like(x, dtype=float)])
+    F = np.concatenate([m / np.sqrt((m * m).sum(0)), np.zeros((1, 256, Y))]).reshape(-1)
+    V = np.zeros_like(V)
+    outs = []
+    for split in ([5], [1] * 5):
+        s = Solver(tid, p_i, p_f, prec)
+        f, v = (torch.tensor(a, dtype=dt, device="cuda") for a in (F, V))
+        s.bind(f, v)
+        s.set_variant(6, 1)
+        for _ in range(3):
+            s.step(1, -1e300)
+        f.copy_(torch.tensor(F, dtype=dt))
+        v.copy_(torch.tensor(V, dtype=dt))
+        Es = []
+        for i, k in enumerate(split):
+            Es.extend(s.step(k, 1e300 if i == 0 else math.nan)[0])
+        assert Es[0] < 1e300 and Es[1] < Es[0]  # the prediction was wrong
+        outs.append((np.array(Es), f.cpu().numpy(), v.cpu().numpy()))
+    (Ea, fa, va), (Eb, fb, vb) = outs
+    if prec == "fp32":
+        np.testing.assert_array_equal(fa, fb)
+        np.testing.assert_array_equal(va, vb)
+    else:
+        assert np.abs(fa - fb).max() <= 1e-12 * np.abs(fb).max()
+        assert np.abs(va - vb).max() <= 1e-12 * max(np.abs(vb).max(), np.abs(fb).max())
+    np.testing.assert_allclose(Ea, Eb, rtol=1e-12)
