@@ -38,11 +38,19 @@ XSIZE = 128.0
 METRIC = "Mpoint-updates/s per flow step at dE/E<=1e-6 vs plain FP64; achieved HBM GB/s"
 UNIT = "Mpoint-updates/s"
 # words of nf components moved per site and step: phase A 4 (phi, V in; l1, l2 out), phase B 6
-# (phi, V, l1, l2 in; phi', V' out)
-WORDS = 10
+# (phi, V, l1, l2 in; phi', V' out).  An arrested step has V = 0 and l2 = l1: 2 + 4.
+WORDS, WORDS_ARRESTED = 10, 6
 # end to end: one host->device load of the field and velocity, E2E_CALLS one-step
 # Simulation.step calls (each returns E and err to the host), one device->host read-back
 E2E_CALLS = 100
+
+
+def words_per_step(E):
+    """Mean words per site and step of a call from its energies: step s is arrested when its starting
+    energy E[s-1] rose above E[s-2].  Step 1's test involves the energy before the call, so it is
+    counted at the smaller figure; step 0 tests nothing."""
+    arrested = int((E[1:-1] > E[:-2]).sum()) + (1 if len(E) > 1 else 0)
+    return WORDS - (WORDS - WORDS_ARRESTED) * arrested / len(E)
 
 
 def chiral_params(xlen=None, ylen=None, xsize=None):
@@ -299,7 +307,7 @@ def gpu_arm(args, rank, world, local_rank):
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     tuning = s.autotune(5)
     if args.variants:
-        # pinned staging variants (S1..S4), e.g. to profile the set a normal run picks
+        # pinned staging variants (stages 1..4; stage 4 is phase B), e.g. to profile the set a normal run picks
         for m, v in enumerate(args.variants.split(","), start=1):
             s.set_variant(m, int(v))
         tuning = {m: (a, b, s._lib.ss_get_variant(s._h, m)) for m, (a, b, _) in tuning.items()}
@@ -320,8 +328,9 @@ def gpu_arm(args, rank, world, local_rank):
     ms = max_over_ranks(ev0.elapsed_time(ev1))
     ms_step = ms / K
     value = world * N * K / (ms / 1e3) / 1e6
-    # two launches per step, then the call's trailing energy pass and finish kernel
-    launches = 2 * K + 2
+    # phases A and B per step and, from the second step on (demag: the arrest is predicted), the kernel
+    # that supplies l2 when it is needed after all; then the trailing energy pass and finish kernel
+    launches = 2 * K + (K - 1) + 2
 
     # roofline of the step's two phase kernels
     from soliton_solver_b200._native import load as _load  # noqa: F401 (library loaded)
@@ -332,7 +341,8 @@ def gpu_arm(args, rank, world, local_rank):
         pass
     peak = float(peaks.get("hbm_gbs", 6650.0))
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
-    bytes_step = WORDS * 4 * 4 * N
+    words = words_per_step(E_traj)
+    bytes_step = words * 4 * 4 * N
     achieved = bytes_step / (ms_step / 1e3) / 1e9
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "flow_kernel_traffic.json")
@@ -382,7 +392,7 @@ def gpu_arm(args, rank, world, local_rank):
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
                              "kernel": "step_kernel<ChiralMagnet,float> phases A (l1, l2) and B (l3, l4, update)",
-                             "launches_per_step": 2,
+                             "launches_per_step": launches / K, "words_per_site_and_step": words,
                              "algorithmic_bytes_per_step": bytes_step},
                 "cpu_baseline": cpu, "cpu_baseline_port": cpu_port,
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
@@ -770,7 +780,7 @@ def dat_field_dump(dev, F0, reps=3):
 
 
 def fused_fp64(dev, F0, steps=50):
-    """The same lattice with FP64 fields through the fused stage kernels (autotuned):
+    """The same lattice with FP64 fields through the fused phase kernels (autotuned):
     the precision-matched comparison with the plain FP64 form."""
     import torch
     from soliton_solver_b200.core.simulation import Simulation
@@ -789,11 +799,11 @@ def fused_fp64(dev, F0, steps=50):
     e1.record()
     torch.cuda.synchronize(dev)
     ms = e0.elapsed_time(e1) / steps
-    words = WORDS
+    words = words_per_step(E)
     gbs = words * 4 * 8 * XLEN * YLEN / (ms / 1e3) / 1e9
     out = {"value": XLEN * YLEN / (ms / 1e3) / 1e6, "unit": UNIT, "ms_per_step": ms, "steps": steps,
            "achieved_gbs": gbs, "bytes_per_point_update": words * 4 * 8, "finite": bool(torch.isfinite(E).all()),
-           "note": "FP64 fields, fused stage kernels, same lattice; CUDA events"}
+           "note": "FP64 fields, fused phase kernels, same lattice; CUDA events"}
     del sim
     torch.cuda.empty_cache()
     return out
