@@ -88,6 +88,7 @@ __global__ void __launch_bounds__((BatchShape<TH, R, PH, SMALL>::NT), (BatchShap
     A.l2 = A.out_l2 = (R*)I.buf[BB_L2];
     A.phi_out = PH == PH_E && !B.cur ? nullptr : (R*)I.buf[out];
     A.vel_out = (R*)I.buf[out + 1];
+    A.copy_phi = A.copy_vel = nullptr;
     A.force = nullptr;
     A.partial = I.partial;
     A.st = I.st;

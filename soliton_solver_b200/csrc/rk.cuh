@@ -45,6 +45,8 @@ struct StepArgs {
   R* out_l2;    // A
   R* phi_out;   // B: phi';  E: copy of phi (nullable)
   R* vel_out;   // B: V'
+  R* copy_phi;  // A, TMA staging (nullable): copies of phi and V for phase B to read
+  R* copy_vel;
   const double* force;  // FP64 fields (nullable): added to the gradient rows in every stage
   double* partial;      // one energy partial per tile (A, E)
   StepState* st;
@@ -344,6 +346,27 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
   }
 }
 
+// The tile's own phi and V from the staged raw buffers to copy_phi and copy_vel (TMA staging:
+// rows, row pitch and buffers are 16-byte multiples, so no vector straddles the lattice's edge).
+template <class TH, typename R, int TX, int TY, int NT>
+__device__ __forceinline__ void copy_tile(const StepArgs<R>& A, const R* B0, int x0, int y0) {
+  using TS = TileShape<TX, TY, NT>;
+  constexpr int VW = 16 / (int)sizeof(R), CH = TY / VW;
+  static_assert(TY % VW == 0 && TS::YOFF % VW == 0 && TS::HY % VW == 0 && TS::PLANE % VW == 0, "16-byte vectors");
+  for (int i = threadIdx.x; i < TX * CH; i += NT) {
+    const int lx = i / CH, c = (i % CH) * VW, gx = x0 + lx, gy = y0 + c;
+    if (gx >= A.G.X || gy >= A.G.Y) continue;
+    const R* t = B0 + (lx + 2) * TS::HY + TS::YOFF + c;
+    const long long g = (long long)gx * A.G.Y + gy;
+#pragma unroll
+    for (int a = 0; a < TH::NF; ++a) {
+      *reinterpret_cast<float4*>(A.copy_phi + a * A.G.N + g) = *reinterpret_cast<const float4*>(t + a * TS::PLANE);
+      *reinterpret_cast<float4*>(A.copy_vel + a * A.G.N + g) =
+          *reinterpret_cast<const float4*>(t + (TH::NF + a) * TS::PLANE);
+    }
+  }
+}
+
 // Expect and issue the TMA loads of one tile (one thread, barrier initialised).  Phase B
 // leaves V and l2 out of an arrested step, phase A leaves V out of a predicted one; phi and l1
 // are issued before the flag is read.
@@ -541,6 +564,12 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
       if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
       mbar_wait_bounded(&S.bar, 0, A.wait_cycles);
       return;
+    }
+    if constexpr (PH == PH_A) {
+      if (A.copy_phi) {
+        copy_tile<TH, R, TX, TY, NT>(A, B0, x0, y0);
+        __syncthreads();  // V is combined in place next
+      }
     }
     combine_tile<TH, R, TX, TY, NT, PH>(A.G, B0, arrest, C);
   } else {
