@@ -160,11 +160,13 @@ int ss_get_variant(const ss_handle *h, int mode);
  * counterpart (tuning control). */
 int ss_set_variant(ss_handle *h, int mode, int variant);
 /* Failure-detection hook.  Sets the bound (clock64 cycles, default 2e9) of every
- * device-side mbarrier wait of this handle's kernels; with inject != 0 the next
- * TMA-staged stage kernel's barrier expects 16 bytes more than its loads deliver,
- * so its bounded wait expires: the kernel records SS_ERR_TIMEOUT, waits the bound
- * again for its own copies and returns without computing.  No fault, trap or
- * unbounded spin is involved; after SS_ERR_TIMEOUT re-bind the handle. */
+ * device-side wait of this handle's kernels (16 times that for the cooperative step's grid
+ * barrier); with inject != 0 the next TMA-staged kernel's barrier expects 16 bytes more than
+ * its loads deliver, or the next cooperative step's one CTA more than it has, so the bounded
+ * wait expires: the kernel records SS_ERR_TIMEOUT, waits the bound again for its own copies
+ * and returns without computing.  No fault, trap or unbounded spin is involved.  Cooperative
+ * launches queued behind it fail likewise until a call has returned SS_ERR_TIMEOUT.  The field
+ * and velocity are then undefined: re-bind the handle or load them anew. */
 int ss_debug_wait_timeout(ss_handle *h, long long wait_cycles, int inject);
 
 /* One gradient evaluation of an arbitrary field buffer: energy_gradient (nullable)

@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <limits>
 #include <type_traits>
 #include <cstdarg>
 #include <cstdio>
@@ -136,7 +137,7 @@ struct ss_handle {
   float tune_ms[N_FLOW_MODES][2] = {};
   int fuse23 = 1;  // stages 2 and 3 in one kernel (TMA staging only)
   long long wait_cycles = WAIT_CYCLES;
-  mutable int inject_timeout = 0;  // test hook, consumed by the next flow launch
+  mutable int inject_timeout = 0;  // test hook, consumed by the next launch that waits
   cudaGraphExec_t graph = nullptr;  // captured n-step relaxation (ss_graph_create)
   const double* force = nullptr;    // FP64 flows: field added to the gradient rows (ss_set_forcing)
   // mapped page-locked staging: the energy and err trajectories of one ss_step chunk and the
@@ -498,7 +499,10 @@ struct Fused {
   }
   static int step_coop(ss_handle* h, int n, double prev, double* E_dev, double* err_dev, int* status_out) {
     StepArgs<R> A = step_args(h);
-    A.wait_cycles = 16 * h->wait_cycles;  // other work on the GPU may hold up a CTA of the grid
+    // other work on the GPU may hold up a CTA of the grid
+    A.wait_cycles = 16 * std::min(h->wait_cycles, std::numeric_limits<long long>::max() / 16);
+    A.tx_extra = h->inject_timeout;  // the grid barrier expects one CTA more than there are
+    h->inject_timeout = 0;
     CoopArgs<R> C;
     C.phi[0] = (R*)h->field;
     C.phi[1] = (R*)h->phi2;
@@ -541,7 +545,7 @@ struct Fused {
   // status_out (nullable, device-visible): the finish kernel copies the call's status there
   static int step(ss_handle* h, int n, double prev, double* E_dev, double* err_dev, int* status_out = nullptr) {
     if (n <= 0) return SS_OK;
-    if (h->coop && !h->inject_timeout) return step_coop(h, n, prev, E_dev, err_dev, status_out);
+    if (h->coop) return step_coop(h, n, prev, E_dev, err_dev, status_out);
     StepArgs<R> A = step_args(h);
     A.E_traj = E_dev;
     A.err_traj = err_dev;
@@ -890,10 +894,15 @@ int read_state(ss_handle* h, StepState* out) {
   return SS_OK;
 }
 
-// error of a nonzero device status (read by the caller), which is cleared on the device
+// error of a nonzero device status (read by the caller, with the stream idle), which is cleared on
+// the device together with the counters a kernel that gave up leaves behind
 int status_error(ss_handle* h, int status) {
-  const int zero = 0;
-  CK(cudaMemcpyAsync(&h->st->status, &zero, sizeof(int), cudaMemcpyHostToDevice, h->stream));
+  StepState s;
+  int rc = read_state(h, &s);
+  if (rc) return rc;
+  s.status = 0;
+  idle_counters(s);
+  CK(cudaMemcpyAsync(h->st, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (status == SS_ERR_TIMEOUT)
     return fail(SS_ERR_TIMEOUT, "a device-side wait timed out; re-bind the handle before further use");
@@ -1959,11 +1968,13 @@ int ss_batch_step(ss_batch* b, int n_steps, const double* prev_energy, double* e
   int worst = 0;
   for (size_t i = 0; i < nn; ++i) {
     if (hst[i].status) {
-      worst = hst[i].status;
-      const int zero = 0;
-      CK(cudaMemcpy(&b->d_st[i].status, &zero, sizeof(int), cudaMemcpyHostToDevice));
+      worst = std::max(worst, hst[i].status);
+      hst[i].status = 0;
+      idle_counters(hst[i]);
+      CK(cudaMemcpyAsync(&b->d_st[i], &hst[i], sizeof(StepState), cudaMemcpyHostToDevice, b->stream));
     }
   }
+  if (worst) CK(cudaStreamSynchronize(b->stream));
   if (worst == SS_ERR_TIMEOUT) return fail(SS_ERR_TIMEOUT, "a device-side wait timed out; re-bind the batch");
   if (worst) return fail(SS_ERR_NONFINITE, "a lattice's energy became non-finite");
   return SS_OK;

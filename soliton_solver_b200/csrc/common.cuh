@@ -69,6 +69,15 @@ struct StepState {
   unsigned long long err2[2];    // its err maxima of even and odd steps (ordered encoding)
 };
 
+// Record a failure (codes of ss_status): a timeout is not replaced by the non-finite sums it leaves.
+__device__ inline void raise_status(StepState* st, int code) { atomicMax(&st->status, code); }
+// What a call that gave up half-way left counted or maximised, back to the values between calls.
+inline void idle_counters(StepState& s) {
+  s.err_enc = s.err2[0] = s.err2[1] = 0;
+  s.ticket = s.bar = s.leave = 0;
+  s.l2_missing = 0;
+}
+
 // ---------------------------------------------------------------------------
 // ordered encoding of doubles for atomicMax (0 encodes below every value)
 // ---------------------------------------------------------------------------

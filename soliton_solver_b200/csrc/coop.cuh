@@ -25,9 +25,13 @@ struct CoopArgs {
   int* status_out;  // nullable, device-visible: the call's status
 };
 
-// Grid barrier of a cooperative launch: the count only grows within a launch and the last CTA
-// to leave resets it.  Bounded: returns false in every thread of the CTA when `limit` clock64
-// cycles pass first.
+// Grid barrier of a cooperative launch: the count only grows within a launch (by at most 4096
+// CTAs x 8193 barriers, below bit 31) and the last CTA to leave resets it.  Bounded: a CTA that
+// has waited `limit` clock64 cycles sets bit 31 in place of a count still below the target.  No
+// CTA can have passed that barrier then, so all of them see the mark and return false (in every
+// thread), here or, in launches queued behind, at the first barrier, until the host has reported
+// the timeout and put the state back (idle_counters).
+constexpr unsigned COOP_EXPIRED = 0x80000000u;
 __device__ __forceinline__ bool coop_barrier(StepState* st, unsigned target, long long limit) {
   __syncthreads();
   bool ok = true;
@@ -38,8 +42,12 @@ __device__ __forceinline__ bool coop_barrier(StepState* st, unsigned target, lon
     unsigned seen;
     for (;;) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&st->bar) : "memory");
+      if (seen & COOP_EXPIRED) {
+        ok = false;
+        break;
+      }
       if (seen >= target) break;
-      if (clock64() - t0 > limit) {
+      if (clock64() - t0 > limit && atomicCAS(&st->bar, seen, seen | COOP_EXPIRED) == seen) {
         ok = false;
         break;
       }
@@ -392,9 +400,9 @@ __global__ void __launch_bounds__(NT, (coop_min_ctas<TH, R, NT, SPLIT>())) coop_
   bool arrest = false, failed = false;
   auto sync_grid = [&]() {
     bar += gridDim.x;
-    if (!coop_barrier(st, bar, A.wait_cycles)) {
+    if (!coop_barrier(st, bar + A.tx_extra, A.wait_cycles)) {
       if (threadIdx.x == 0) {
-        atomicExch(&st->status, (int)ST_TIMEOUT);
+        raise_status(st, ST_TIMEOUT);
         if (C.status_out) *(volatile int*)C.status_out = (int)ST_TIMEOUT;
       }
       failed = true;
@@ -408,7 +416,7 @@ __global__ void __launch_bounds__(NT, (coop_min_ctas<TH, R, NT, SPLIT>())) coop_
     __syncthreads();
     const double En = sh_E;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-      if (!isfinite(En)) st->status = 3;
+      if (!isfinite(En)) raise_status(st, ST_NONFINITE);
       if (A.E_traj) A.E_traj[slot] = En;
       st->scalar = En;
     }

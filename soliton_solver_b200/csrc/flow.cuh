@@ -15,7 +15,7 @@ namespace ssb {
 // M_S3, M_S4 its phase B; M_ENERGY and M_S23 are kept for the pinning interface.
 enum FlowMode { M_GRAD = 0, M_S1 = 1, M_S2 = 2, M_S3 = 3, M_S4 = 4, M_ENERGY = 5, M_S23 = 6 };
 constexpr int N_FLOW_MODES = 7;
-enum { ST_TIMEOUT = 6 };
+enum { ST_NONFINITE = 3, ST_TIMEOUT = 6 };
 
 // Default bound of a device-side wait on an mbarrier (~1 s at 1.9 GHz).  On expiry
 // the kernel records ST_TIMEOUT, waits the same bound again for its copies in
@@ -410,7 +410,7 @@ __device__ __forceinline__ bool stage_tma(R* T, const CUtensorMap* map, uint64_t
   __syncthreads();
   const bool ok = __syncthreads_and(mbar_wait_bounded(bar, 0, limit));
   if (!ok) {
-    if (threadIdx.x == 0) atomicExch(&st->status, (int)ST_TIMEOUT);
+    if (threadIdx.x == 0) raise_status(st, ST_TIMEOUT);
     mbar_wait_bounded(bar, 0, limit);
   }
   return ok;
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(NT, 1) flow_kernel_pipe(const __grid_constant_
     const bool ok = __syncthreads_and(mbar_wait_bounded(&full[slot], parity, A.wait_cycles));
     if (!ok) {
       // record, then wait (bounded) for every load still in flight before leaving
-      if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
+      if (threadIdx.x == 0) raise_status(A.st, ST_TIMEOUT);
       for (int s = 0; s < STAGES; ++s) {
         const int kk = k + s;
         if (blockIdx.x + kk * gridDim.x < ntiles)
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(NT, (TH::NF <= 4 ? 3 : 2))
     if (threadIdx.x == 0) {
       st->scalars[q] = E;
       if (q == 0) st->scalar = E;
-      if (!isfinite(E)) st->status = 3;
+      if (!isfinite(E)) raise_status(st, ST_NONFINITE);
     }
   }
   if (threadIdx.x == 0) st->ticket = 0u;

@@ -428,7 +428,7 @@ __device__ __forceinline__ void step_reductions(const StepArgs<R>& A, StageShare
     const double E = fixed_order_sum<NT>(A.partial, nblk, S.sh_s, S.sh_c);
     if (threadIdx.x == 0) {
       st->scalar = E;
-      if (!isfinite(E)) st->status = 3;
+      if (!isfinite(E)) raise_status(st, ST_NONFINITE);
       if (A.E_traj && A.E_idx >= 0) A.E_traj[A.E_idx] = E;
       if (A.arrest_update) {
         const int arrest = (A.G.killkinen && E > st->E_last) ? 1 : 0;
@@ -561,7 +561,7 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
     if constexpr (PH == PH_A) arrest = A.predict && __ldcg(&A.st->streak) >= 2;
     const bool ok = __syncthreads_and(mbar_wait_bounded(&S.bar, 0, A.wait_cycles));
     if (!ok) {
-      if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
+      if (threadIdx.x == 0) raise_status(A.st, ST_TIMEOUT);
       mbar_wait_bounded(&S.bar, 0, A.wait_cycles);
       return;
     }
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__((PipeShape<TH, R>::NT), (PipeShape<TH, R>::CTA
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const bool ok = __syncthreads_and(mbar_wait_bounded(&full[slot], parity, A.wait_cycles));
     if (!ok) {  // record, then wait (bounded) for every load still in flight before leaving
-      if (threadIdx.x == 0) atomicExch(&A.st->status, (int)ST_TIMEOUT);
+      if (threadIdx.x == 0) raise_status(A.st, ST_TIMEOUT);
       for (int s = 0; s < SLOTS && t + s * (int)gridDim.x < ntiles; ++s) {
         mbar_wait_bounded(&full[slot], parity, A.wait_cycles);
         if (++slot == SLOTS) {
