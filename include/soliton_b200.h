@@ -139,7 +139,8 @@ int ss_step_async(ss_handle *h, int n_steps, double prev_energy, double *energy_
 /* Synchronise the bound stream and return the status the device-side checks set. */
 int ss_check_status(ss_handle *h);
 /* 1 when the bound Field/Velocity/workspace buffers are staged by TMA tensor maps
- * (row pitch and base 16-byte aligned), 0 when the plain-load path is used. */
+ * (row pitch and base 16-byte aligned), 0 when the plain-load path is used.  Field and output
+ * buffers need the alignment of their element type only. */
 int ss_tma_enabled(const ss_handle *h);
 /* Autotuner: times, on the bound buffers, the step's phase A (stages 1 and 2), the two
  * variants of its phase B (stages 3 and 4) and of the gradient (persistent CTAs walking

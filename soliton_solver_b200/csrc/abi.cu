@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <initializer_list>
 #include <limits>
 #include <type_traits>
 #include <cstdarg>
@@ -190,6 +191,14 @@ size_t layout(ss_handle* h, char* base) {
   return off;
 }
 
+// Interior tiles load and store y-adjacent site pairs of global buffers as one vector: rows of
+// even length in buffers (null: none) aligned to two elements of `es` bytes.
+int site_pairs(const Grid& G, size_t es, std::initializer_list<const void*> bufs) {
+  bool ok = G.Y % 2 == 0;
+  for (const void* p : bufs) ok = ok && (uintptr_t)p % (2 * es) == 0;
+  return ok ? 1 : 0;
+}
+
 // ---------------------------------------------------------------------------
 // parameter decoding (packed arrays of each theory's pack_device_params)
 // ---------------------------------------------------------------------------
@@ -218,6 +227,7 @@ int decode(ss_handle* h, int theory, const int32_t* p_i, int n_i, const double* 
     return fail(SS_ERR_ARG, "p_i[5]/p_i[6] (dim_grid/dim_fields) inconsistent with xlen*ylen*nf");
   G.killkinen = p_i[7] ? 1 : 0;
   G.unit_mag = p_i[9] ? 1 : 0;
+  G.pairs = site_pairs(G, 1, {});
   G.lsx = p_f[2];
   G.lsy = p_f[3];
   G.dA = p_f[4];
@@ -654,6 +664,7 @@ struct Fused {
     A.phi = (const R*)field;
     A.out_eg = (R*)eg;
     A.out_l = (R*)l_out;
+    A.G.pairs = site_pairs(h->G, sizeof(R), {eg, l_out});
     const bool tma = encode_tile_map(&A.tm_phi, field, sizeof(R), h->G.X, h->G.Y, TH::NF);
     return launch(h, A, tma);
   }
@@ -1031,6 +1042,7 @@ int ss_bind(ss_handle* h, void* field, void* velocity, void* workspace, size_t w
   h->ws = (char*)workspace;
   h->ws_bytes = workspace_bytes;
   h->stream = (cudaStream_t)stream;
+  h->G.pairs = site_pairs(h->G, h->elem, {field, velocity});
   layout(h, h->ws);
   StepState init;
   memset(&init, 0, sizeof(init));
@@ -1915,6 +1927,7 @@ int ss_batch_bind(ss_batch* b, void* const* fields, void* const* velocities, voi
     BatchInst& I = b->h_insts[i];
     if (!fields[i] || !velocities[i]) return fail(SS_ERR_ARG, "lattice %d: NULL field or velocity", i);
     I.G = b->inst[i].G;
+    I.G.pairs = site_pairs(I.G, b->elem, {fields[i], velocities[i]});
     I.P = b->inst[i].P;
     I.buf[0] = fields[i];
     I.buf[1] = velocities[i];

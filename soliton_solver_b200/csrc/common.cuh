@@ -21,6 +21,7 @@ struct Grid {
   double dA, dt;        // grid_volume, time_step     (p_f[4], p_f[5])
   int killkinen;        // arrest on energy increase  (p_i[7])
   int unit_mag;         // unit_magnetization         (p_i[9])
+  int pairs;            // y-adjacent site pairs of the launch's global buffers are pair-aligned (site_pairs)
   double ihx, ihy;      // 1/lsx, 1/lsy
   double ihx2, ihy2;    // 1/lsx^2, 1/lsy^2
   double ih2dA;         // 1/(2 dA)

@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(NT, (coop_min_ctas<TH, R, NT, SPLIT>())) coop_
   StepState* st = A.st;
   const int tiles_y = (G.Y + TY - 1) / TY;
   const int x0 = (blockIdx.x / tiles_y) * TX, y0 = (blockIdx.x % tiles_y) * TY;
-  const bool fast = (G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
+  const bool fast = G.pairs && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
                     y0 + TY - 1 <= G.Y - G.halo - 2;
   const int j = threadIdx.x % CT::PAIRS, lxg = (threadIdx.x % CT::PT) / CT::PAIRS;
   CoopChunks<NF, R, TX, TY, NT, VW> K;

@@ -319,8 +319,8 @@ __device__ __forceinline__ void flow_constraints(const Grid& G, const Jet<V, TH:
 }
 
 // The gradient hook on one staged tile.  Each thread owns y-adjacent site pairs; FAST: the
-// tile is interior (every derivative mask true, no halo site) and the lattice row length is
-// even, so pairs are aligned and need no lane masks.
+// tile is interior (every derivative mask true, no halo site) and the output buffers hold
+// aligned pairs (Grid::pairs), which need no lane masks.
 template <class TH, typename R, int TX, int TY, int NT, bool FAST>
 __device__ __forceinline__ void grad_tile(const FlowArgs<R>& A, const R* T, int x0, int y0) {
   using TS = TileShape<TX, TY, NT>;
@@ -389,7 +389,7 @@ struct StageShared {
 template <class TH, typename R, int TX, int TY, int NT>
 __device__ __forceinline__ void grad_any_tile(const FlowArgs<R>& A, const R* T, int x0, int y0) {
   const Grid& G = A.G;
-  if ((G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
+  if (G.pairs && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
       y0 + TY - 1 <= G.Y - G.halo - 2)
     grad_tile<TH, R, TX, TY, NT, true>(A, T, x0, y0);
   else

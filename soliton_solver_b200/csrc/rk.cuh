@@ -506,7 +506,7 @@ __device__ __forceinline__ void compute_tile(const StepArgs<R>& A, const R* B0, 
                                              bool arrest, double& e_acc, double& err_max) {
   constexpr int BUF = TH::NF * TileShape<TX, TY, NT>::PLANE;
   const Grid& G = A.G;
-  const bool fast = (G.Y % 2 == 0) && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
+  const bool fast = G.pairs && x0 >= G.halo + 1 && x0 + TX - 1 <= G.X - G.halo - 2 && y0 >= G.halo + 1 &&
                     y0 + TY - 1 <= G.Y - G.halo - 2;
   if constexpr (PH == PH_B) {
     const R* T3 = TMA ? B0 + 2 * BUF : B0;
