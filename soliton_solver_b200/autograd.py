@@ -31,6 +31,7 @@ from __future__ import annotations
 import itertools
 
 import torch
+from torch._C import _functorch
 
 _SOLVERS: dict = {}
 _KEYS = itertools.count(1)
@@ -143,7 +144,8 @@ def _setup(ctx, inputs, output):
 
 def _backward(ctx, grad_E):
     (field,) = ctx.saved_tensors
-    if not torch.is_grad_enabled():  # no graph of the backward itself: one pass
+    # one pass, unless the backward itself is recorded or several grad_E share one gradient (is_grads_batched)
+    if not torch.is_grad_enabled() and not _functorch.is_legacy_batchedtensor(grad_E):
         return energy_vjp_op(field, grad_E, ctx.key), None
     s = _SOLVERS[ctx.key]
     g = energy_gradient_op(field, ctx.key)
