@@ -33,6 +33,8 @@ import itertools
 import torch
 from torch._C import _functorch
 
+from .core.solver import _COUPLINGS
+
 _SOLVERS: dict = {}
 _KEYS = itertools.count(1)
 
@@ -178,7 +180,9 @@ def _partials(sim, solver, field, names):
             out = {k: out[k] for k in names}
         return out
     avail = {"baby_skyrme": ("kappa", "mpi"), "ginzburg_landau_superconductor": ("Lambda",)}.get(mod, ())
-    names = avail if names is None else names
+    names = list(avail if names is None else names)
+    for n in names:
+        _COUPLINGS[n]  # KeyError: not a coupling (solver.observables takes the energy and charges too)
     return solver.observables(field, names) if names else {}
 
 

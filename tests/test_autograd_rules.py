@@ -38,3 +38,13 @@ def test_batched_backward_evaluates_the_gradient_once():
     (g,) = torch.autograd.grad(ag.energy(x, s), x, grad_outputs=w, is_grads_batched=True)
     torch.testing.assert_close(g, DA * w[:, None] * x.detach(), rtol=1e-15, atol=0)
     assert s.calls == 1
+
+
+@pytest.mark.parametrize("theory", ["baby_skyrme", "ginzburg_landau_superconductor"])
+@pytest.mark.parametrize("name", ["energy", "skyrmion", "vortex", "nonsense"])
+def test_only_couplings_have_coupling_gradients(theory, name):
+    sim = types.SimpleNamespace(theory=types.SimpleNamespace(__name__=f"theories.{theory}"), solver=_Quadratic(),
+                                Field=torch.zeros(3))
+    with pytest.raises(KeyError):
+        ag.coupling_gradients(sim, ("kappa", name))
+    assert ag.coupling_gradients(sim, ()) == {}
