@@ -9,7 +9,8 @@ the masked boundary ring; ``tests/test_autograd.py`` states the tolerance.
 
 The native calls are registered as torch.library custom ops so they compose with
 torch's dispatcher (fake tensors, opcheck); solvers are passed by an integer key of
-``register()``:
+``register()``.  A solver's kernels run on the stream it was bound on: called on another
+one, the ops order the two streams by events, before and after.
 
   soliton_b200::energy(field, key) -> f64 scalar          ss_energy (differentiable)
   soliton_b200::energy_gradient(field, key) -> like field  ss_energy_gradient
@@ -49,10 +50,28 @@ def register(solver) -> int:
     return key
 
 
+def _fork(s, t):
+    """The solver's stream, made to wait for the current one's work (the inputs), or None where the
+    current stream is the solver's."""
+    if not t.is_cuda or torch._C._cuda_getCurrentRawStream(t.device.index) == s.bound_stream:
+        return None
+    side = torch.cuda.ExternalStream(s.bound_stream, t.device) if s.bound_stream else torch.cuda.default_stream(t.device)
+    side.wait_stream(torch.cuda.current_stream(t.device))
+    return side
+
+
+def _join(side, t):
+    """The current stream's next work (the results' readers, the buffers' next owners) after the solver's."""
+    if side is not None:
+        torch.cuda.current_stream(t.device).wait_stream(side)
+
+
 @torch.library.custom_op("soliton_b200::energy", mutates_args=())
 def energy_op(field: torch.Tensor, key: int) -> torch.Tensor:
     s = _SOLVERS[key]
-    return torch.full((), s.energy(field.contiguous()), dtype=torch.float64, device=field.device)
+    field = field.contiguous()
+    _fork(s, field)  # the call waits for its result
+    return torch.full((), s.energy(field), dtype=torch.float64, device=field.device)
 
 
 @energy_op.register_fake
@@ -63,7 +82,11 @@ def _(field, key):
 @torch.library.custom_op("soliton_b200::energy_gradient", mutates_args=())
 def energy_gradient_op(field: torch.Tensor, key: int) -> torch.Tensor:
     s = _SOLVERS[key]
-    return s.energy_gradient(field.contiguous())
+    field = field.contiguous()
+    side = _fork(s, field)
+    out = s.energy_gradient(field)
+    _join(side, field)
+    return out
 
 
 @energy_gradient_op.register_fake
@@ -74,7 +97,11 @@ def _(field, key):
 @torch.library.custom_op("soliton_b200::energy_vjp", mutates_args=())
 def energy_vjp_op(field: torch.Tensor, grad_E: torch.Tensor, key: int) -> torch.Tensor:
     s = _SOLVERS[key]
-    return s.energy_vjp(field.contiguous(), grad_E.to(torch.float64).contiguous())
+    field, grad_E = field.contiguous(), grad_E.to(torch.float64).contiguous()
+    side = _fork(s, field)
+    out = s.energy_vjp(field, grad_E)
+    _join(side, field)
+    return out
 
 
 @energy_vjp_op.register_fake
@@ -85,8 +112,11 @@ def _(field, grad_E, key):
 @torch.library.custom_op("soliton_b200::gradient", mutates_args=())
 def gradient_op(field: torch.Tensor, key: int) -> torch.Tensor:
     s = _SOLVERS[key]
+    field = field.contiguous()
     out = torch.empty_like(field)
-    s.gradient(field.contiguous(), out, None)
+    side = _fork(s, field)
+    s.gradient(field, out, None)
+    _join(side, field)
     return out
 
 
@@ -98,7 +128,9 @@ def _(field, key):
 @torch.library.custom_op("soliton_b200::charge", mutates_args=())
 def charge_op(field: torch.Tensor, key: int, which: str) -> torch.Tensor:
     s = _SOLVERS[key]
-    return torch.tensor(s.charge(field.contiguous(), which), dtype=torch.float64, device=field.device)
+    field = field.contiguous()
+    _fork(s, field)
+    return torch.tensor(s.charge(field, which), dtype=torch.float64, device=field.device)
 
 
 @charge_op.register_fake
@@ -109,7 +141,9 @@ def _(field, key, which):
 @torch.library.custom_op("soliton_b200::coupling_grad", mutates_args=())
 def coupling_grad_op(field: torch.Tensor, key: int, name: str) -> torch.Tensor:
     s = _SOLVERS[key]
-    return torch.tensor(s.coupling_grad(field.contiguous(), name), dtype=torch.float64, device=field.device)
+    field = field.contiguous()
+    _fork(s, field)
+    return torch.tensor(s.coupling_grad(field, name), dtype=torch.float64, device=field.device)
 
 
 @coupling_grad_op.register_fake
@@ -129,7 +163,9 @@ def flow_step_op(field: torch.Tensor, velocity: torch.Tensor, key: int, n_steps:
         s.bind(field, velocity)
     E = torch.empty(n_steps, dtype=torch.float64, device=field.device)
     err = torch.empty(n_steps, dtype=torch.float64, device=field.device)
+    side = _fork(s, field)
     s.step_async(n_steps, prev_energy, E, err)
+    _join(side, field)
     return E, err
 
 

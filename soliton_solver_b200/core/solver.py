@@ -80,9 +80,10 @@ class Solver:
         return int(torch.cuda.current_stream(self.device).cuda_stream)
 
     def _bind(self, field, velocity):
+        self.bound_stream = self._stream_handle()  # the stream the native calls run on
         with self._on_device():
             nat.check(self._lib.ss_bind(self._h, _ptr(field), _ptr(velocity), self.workspace.data_ptr(),
-                                        self.workspace.numel(), self._stream_handle()))
+                                        self.workspace.numel(), self.bound_stream))
         self.field, self.velocity = field, velocity
 
     def bind(self, field: torch.Tensor, velocity: torch.Tensor):
