@@ -142,6 +142,9 @@ int ss_check_status(ss_handle *h);
  * (row pitch and base 16-byte aligned), 0 when the plain-load path is used.  Field and output
  * buffers need the alignment of their element type only. */
 int ss_tma_enabled(const ss_handle *h);
+/* How the bound lattice steps: 0 two launches per step (or the plain form), 1 to 3 all steps of a
+ * call in one cooperative launch, in tiles of 8 x 32, 16 x 32 or 16 x 64 sites; -1 for NULL. */
+int ss_step_form(const ss_handle *h);
 /* Autotuner: times, on the bound buffers, the step's phase A (stages 1 and 2), the two
  * variants of its phase B (stages 3 and 4) and of the gradient (persistent CTAs walking
  * tiles through a shared-memory ring, or one tile per CTA) over `iters` launches and keeps

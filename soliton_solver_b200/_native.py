@@ -99,6 +99,7 @@ _SIG = {
     "ss_step": ([_P, _I, _D, _P, _P], _I),
     "ss_step_async": ([_P, _I, _D, _P, _P], _I),
     "ss_check_status": ([_P], _I),
+    "ss_step_form": ([_P], _I),
     "ss_tma_enabled": ([_P], _I),
     "ss_autotune": ([_P, _I, _P], _I),
     "ss_get_variant": ([_P, _I], _I),

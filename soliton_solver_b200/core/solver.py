@@ -149,6 +149,11 @@ class Solver:
         """True when the bound buffers are staged with TMA tensor maps."""
         return bool(self._lib.ss_tma_enabled(self._h))
 
+    @property
+    def step_form(self) -> int:
+        """0: two launches per step; 1 to 3: one cooperative launch per call (see ss_step_form)."""
+        return int(self._lib.ss_step_form(self._h))
+
     def autotune(self, iters: int = 5):
         """Pick the faster staging variants of the flow's kernels on the bound buffers.
 

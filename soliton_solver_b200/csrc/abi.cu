@@ -1072,6 +1072,8 @@ int ss_bind(ss_handle* h, void* field, void* velocity, void* workspace, size_t w
   return SS_OK;
 }
 
+int ss_step_form(const ss_handle* h) { return h ? h->coop : -1; }
+
 int ss_tma_enabled(const ss_handle* h) { return h && h->tma ? 1 : 0; }
 
 int ss_autotune(ss_handle* h, int iters, float* ms_out) {
