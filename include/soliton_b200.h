@@ -157,10 +157,10 @@ int ss_autotune(ss_handle *h, int iters, float *ms_out);
 int ss_get_variant(const ss_handle *h, int mode);
 /* Pin the staging variant of a mode instead of autotuning it: mode 0 (gradient) or 1..4
  * (RK stages; stages 3 and 4 run as one kernel, pinned by mode 4; stages 1 and 2 run as
- * one kernel with one form, so modes 1 and 2 are kept but change nothing, mode 1 sets the
- * energy observable's variant as well), variant 0 (one tile per CTA) or 1 (pipelined;
- * needs TMA-staged bound buffers and FP32 fields); mode 6 (0 or 1) is kept and changes
- * nothing.  For reproducible runs and for profiling a known kernel set.  No reference
+ * one kernel with one form, so modes 1 and 2 are kept but change nothing; mode 1 is
+ * reported for mode 5 as well), variant 0 (one tile per CTA) or 1 (pipelined; needs
+ * TMA-staged bound buffers and, for modes 0 to 2, FP32 fields); mode 6 (0 or 1) is kept and
+ * changes nothing.  A pinned step (any mode but 0) runs as two launches.  For reproducible runs and for profiling a known kernel set.  No reference
  * counterpart (tuning control). */
 int ss_set_variant(ss_handle *h, int mode, int variant);
 /* Failure-detection hook.  Sets the bound (clock64 cycles, default 2e9) of every

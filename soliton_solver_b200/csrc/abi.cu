@@ -371,8 +371,9 @@ struct Fused {
     CK(cudaGetLastError());
     return SS_OK;
   }
-  // whether a mode has a pipelined variant (phase A's, M_S1 and M_S2, is accepted and ignored)
-  static bool uses_pipe(int) { return sizeof(R) == 4; }
+  // whether a mode has a pipelined variant: the gradient's for FP32, phase B's (M_S3, M_S4) for both
+  // precisions; phase A's (M_S1 and M_S2) is accepted for FP32 and ignored
+  static bool uses_pipe(int mode) { return sizeof(R) == 4 || mode == M_S3 || mode == M_S4; }
 
   // tma: use the TMA-staged instantiations (A.tm_phi must describe A.phi)
   static int launch(const ss_handle* h, const FlowArgs<R>& A0, bool tma) {
@@ -1117,21 +1118,21 @@ int ss_set_variant(ss_handle* h, int mode, int variant) {
                 "stage 1", mode);
   if (variant != 0 && variant != 1) return fail(SS_ERR_ARG, "variant %d: 0 (one tile per CTA) or 1 (pipelined)", variant);
   if (h->precision == SS_PLAIN_FP64) return fail(SS_ERR_ARG, "the plain FP64 form has no staging variants");
-  if (mode != M_GRAD) {  // the step's launches were asked for
-    h->pinned = true;
-    h->coop = 0;
-  }
-  if (mode == M_S23) {  // 1: stages 2 and 3 in one kernel (used with TMA staging), 0: two kernels
-    h->fuse23 = variant;
-    return SS_OK;
-  }
-  if (variant == 1) {
+  if (variant == 1 && mode != M_S23) {
     if (!h->tma) return fail(SS_ERR_STATE, "the pipelined variant needs TMA-staged buffers (bind first; rows of 16-byte multiples)");
     const bool ok = dispatch(h, [&](auto* tag) -> int {
       using TH = std::remove_pointer_t<decltype(tag)>;
       return h->precision == SS_FP32 ? Fused<TH, float>::uses_pipe(mode) : Fused<TH, double>::uses_pipe(mode);
     }) != 0;
     if (!ok) return fail(SS_ERR_ARG, "no pipelined variant of mode %d for this theory and precision", mode);
+  }
+  if (mode != M_GRAD) {  // the step's launches were asked for
+    h->pinned = true;
+    h->coop = 0;
+  }
+  if (mode == M_S23) {  // kept for the caller, chooses nothing
+    h->fuse23 = variant;
+    return SS_OK;
   }
   h->use_pipe[mode] = variant;
   if (mode == M_S1) h->use_pipe[M_ENERGY] = variant;  // the energy pass reduces exactly like stage 1

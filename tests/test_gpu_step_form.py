@@ -67,3 +67,31 @@ def test_odd_counts_of_the_plain_two_launch_step(th, prev):
     for got in outs[1:]:
         for a, b in zip(got, outs[0]):
             np.testing.assert_array_equal(a, b)
+
+
+def test_fp64_second_phase_variants():
+    """Phase B has both variants in FP64 too: pinned to one tile per CTA and back, the same step up to the
+    compiler's contraction in the two kernels (1e-12 of max|phi|); a handle pinned to neither has variant 1."""
+    outs = []
+    for pins in ((), (0,), (0, 1)):
+        s = _solver("Abelian Higgs", "fp64", 600, 640)
+        assert s.step_form == 0 and s._lib.ss_get_variant(s._h, 4) == 1
+        for v in pins:
+            s.set_variant(4, v)
+            assert s._lib.ss_get_variant(s._h, 4) == v
+        s.step(5, 1e300)
+        outs.append(s.field)
+    assert torch.equal(outs[0], outs[2])
+    assert (outs[0] - outs[1]).abs().max() <= 1e-12 * outs[0].abs().max()
+
+
+def test_refused_variant_leaves_the_step_form():
+    s = _solver("Chiral magnet", "fp32", 64, 101)
+    assert s.step_form == 1 and not s.tma_enabled
+    with pytest.raises(Exception, match="TMA"):
+        s.set_variant(4, 1)
+    assert s.step_form == 1
+    s = _solver("Chiral magnet", "fp64", 64, 100)
+    with pytest.raises(ValueError, match="no pipelined variant"):
+        s.set_variant(1, 1)
+    assert s.step_form == 1
