@@ -480,6 +480,12 @@ struct Fused {
       if (capacity) *capacity = 0;
       return capacity ? SS_OK : fail(SS_ERR_ARG, "bad cooperative shape");
     } else {
+      // too many tiles by the kernel's bounds alone: the kernel is not loaded to ask for its occupancy
+      // (20 to 200 us for the first bind of a process whose lattice can never use it)
+      if (capacity && coop_tiles(h->G, S) > coop_ctas<TH, R, CX, CY, CN, COOP_SPLIT[S]>() * h->num_sms) {
+        *capacity = 0;
+        return SS_OK;
+      }
       auto k = coop_step_kernel<TH, R, CX, CY, CN, COOP_SPLIT[S], VW>;
       static unsigned long long done = 0;
       set_smem(k, CT::SMEM, done);

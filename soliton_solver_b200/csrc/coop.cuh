@@ -357,6 +357,15 @@ __host__ __device__ constexpr int coop_min_ctas() {
   return (sizeof(R) == 8 && TH::NF > 4 ? 256 : SPLIT && sizeof(R) == 4 && TH::NF <= 4 ? 768 : 512) / NT;
 }
 
+// The same as the kernel's residency: no more than that many CTAs, nor than fit an SM's shared memory
+// (228 KB; each CTA's arrays and 1 KB).
+template <class TH, typename R, int TX, int TY, int NT, bool SPLIT>
+__host__ __device__ constexpr int coop_ctas() {
+  const size_t per = CoopTile<TH, R, TX, TY, NT, SPLIT>::SMEM + sizeof(StageShared<NT>) + 128 + 1024;
+  const int fit = (int)(228 * 1024 / per), want = coop_min_ctas<TH, R, NT, SPLIT>();
+  return fit < want ? fit : want;
+}
+
 template <class TH, typename R, int TX, int TY, int NT, bool SPLIT, int VW>
 __global__ void __launch_bounds__(NT, (coop_min_ctas<TH, R, NT, SPLIT>())) coop_step_kernel(
     const __grid_constant__ StepArgs<R> A, const __grid_constant__ CoopArgs<R> C) {
