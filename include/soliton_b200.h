@@ -129,7 +129,8 @@ int ss_bind(ss_handle *h, void *field, void *velocity, void *workspace, size_t w
  * the energy the previous ss_step call left on the device.  Steps run in chunks of
  * 1024; a non-finite energy or a timed-out wait ends the call after the chunk in
  * which it happened (the trajectories up to there are written).  The first call
- * page-locks a 16 KB host staging buffer, held until ss_destroy. */
+ * takes a 17 KB page-locked staging block, held until ss_destroy (which keeps up to four of
+ * them for later handles). */
 int ss_step(ss_handle *h, int n_steps, double prev_energy, double *energy_traj, double *err_traj);
 /* As ss_step but without a host synchronisation: the trajectories go to device
  * arrays of n_steps doubles (nullable) and the status of the device-side checks is

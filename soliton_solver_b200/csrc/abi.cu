@@ -4,6 +4,7 @@
 #include <cmath>
 #include <initializer_list>
 #include <limits>
+#include <mutex>
 #include <type_traits>
 #include <cstdarg>
 #include <cstdio>
@@ -34,7 +35,7 @@ namespace {
 constexpr int TX = 16, TY = 64, NT = 256;  // fused tile: 16 x 64 sites, 256 threads
 constexpr int COOP_MAX_TILES = 4096;        // energy partials kept for the cooperative step
 constexpr int TRAJ_CAP = 1024;              // device trajectory slots used by ss_step
-constexpr size_t STAGE_TAIL = 64 + 192;      // bytes of ss_handle::host_stage behind the trajectories: status, state
+constexpr size_t STAGE_TAIL = 64 + 192;      // bytes of HostStage::host behind the trajectories: status, state
 constexpr size_t ALIGN = 256;
 // Tensor maps of a bound handle (halo boxes): phi and V of the caller's buffers and of the
 // workspace's pair in the tile shapes of phases A and B, l1 and l2 in phase B's
@@ -93,6 +94,58 @@ bool encode_tile_map(CUtensorMap* m, const void* ptr, size_t es, int X, int Y, i
 
 }  // namespace
 
+// Mapped page-locked staging of a handle: the energy and err trajectories of one ss_step chunk and
+// the status of the call, written by the kernels themselves, and behind them the step state as read
+// back by read_state.  Page-locking a block costs about 60 us and releasing one waits for the device,
+// so a destroyed handle's block is kept for the next handle: at most STAGE_KEEP blocks (17 KB each)
+// in the process, the others are released.
+struct HostStage {
+  double* host = nullptr;
+  double* dev = nullptr;  // its device address
+  bool busy = false;      // a launch or copy that writes it has not been waited for
+};
+
+namespace {
+constexpr size_t STAGE_KEEP = 4;
+std::mutex g_stage_mutex;
+HostStage g_stage_free[STAGE_KEEP];
+size_t g_stage_count = 0;
+
+cudaError_t stage_take(HostStage& s) {
+  {
+    std::lock_guard<std::mutex> lock(g_stage_mutex);
+    while (g_stage_count) {
+      const HostStage t = g_stage_free[--g_stage_count];
+      cudaPointerAttributes a;  // a device reset in between takes the blocks with it
+      if (cudaPointerGetAttributes(&a, t.host) == cudaSuccess && a.type == cudaMemoryTypeHost) {
+        s = t;
+        return cudaSuccess;
+      }
+      cudaGetLastError();
+    }
+  }
+  HostStage t;
+  cudaError_t e = cudaHostAlloc((void**)&t.host, 2 * TRAJ_CAP * sizeof(double) + STAGE_TAIL,
+                                cudaHostAllocMapped | cudaHostAllocPortable);
+  if (e == cudaSuccess && (e = cudaHostGetDevicePointer((void**)&t.dev, t.host, 0)) != cudaSuccess) cudaFreeHost(t.host);
+  if (e == cudaSuccess) s = t;
+  return e;
+}
+void stage_give(HostStage& s) {
+  if (!s.host) return;
+  if (!s.busy) {
+    std::lock_guard<std::mutex> lock(g_stage_mutex);
+    if (g_stage_count < STAGE_KEEP) {
+      g_stage_free[g_stage_count++] = s;
+      s = HostStage{};
+      return;
+    }
+  }
+  cudaFreeHost(s.host);  // waits for the device
+  s = HostStage{};
+}
+}  // namespace
+
 struct ss_handle {
   int theory = 0, precision = 0, nf = 0;
   double pf_raw[32] = {};  // the packed p_f as given (initial-condition kernels read it)
@@ -141,14 +194,10 @@ struct ss_handle {
   mutable int inject_timeout = 0;  // test hook, consumed by the next launch that waits
   cudaGraphExec_t graph = nullptr;  // captured n-step relaxation (ss_graph_create)
   const double* force = nullptr;    // FP64 flows: field added to the gradient rows (ss_set_forcing)
-  // mapped page-locked staging: the energy and err trajectories of one ss_step chunk and the
-  // status of the call, written by the kernels themselves, and behind them the step state as
-  // read back by read_state (allocated on first use; host_stage_dev is its device address)
-  double* host_stage = nullptr;
-  double* host_stage_dev = nullptr;
+  HostStage stage;  // taken on first use
   ~ss_handle() {
     if (graph) cudaGraphExecDestroy(graph);
-    if (host_stage) cudaFreeHost(host_stage);
+    stage_give(stage);
   }
 };
 
@@ -893,22 +942,16 @@ int coop_plan(const ss_handle* h) {
   return got;
 }
 
-// the handle's page-locked staging (mapped; allocated on first use)
 static_assert(sizeof(StepState) <= 192, "fits behind the staged status");
-int host_staging(ss_handle* h) {
-  if (h->host_stage) return SS_OK;
-  CK(cudaHostAlloc((void**)&h->host_stage, 2 * TRAJ_CAP * sizeof(double) + STAGE_TAIL, cudaHostAllocMapped));
-  CK(cudaHostGetDevicePointer((void**)&h->host_stage_dev, h->host_stage, 0));
-  return SS_OK;
-}
-
 int read_state(ss_handle* h, StepState* out) {
-  int rc = host_staging(h);  // page-locked: the copy needs no intermediate buffer
-  if (rc) return rc;
-  StepState* s = reinterpret_cast<StepState*>(h->host_stage + 2 * TRAJ_CAP + 8);
+  // page-locked: the copy needs no intermediate buffer; pageable where no block can be had
+  if (!h->stage.host && stage_take(h->stage) != cudaSuccess) cudaGetLastError();
+  StepState* s = h->stage.host ? reinterpret_cast<StepState*>(h->stage.host + 2 * TRAJ_CAP + 8) : out;
+  h->stage.busy = true;
   CK(cudaMemcpyAsync(s, h->st, sizeof(StepState), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  *out = *s;
+  h->stage.busy = false;
+  if (s != out) *out = *s;
   return SS_OK;
 }
 
@@ -1031,8 +1074,7 @@ int ss_workspace_bytes(const ss_handle* h, size_t* bytes) {
   if (!h || !bytes) return fail(SS_ERR_ARG, "NULL argument");
   ss_handle tmp = *h;
   tmp.graph = nullptr;  // the copy must not own the original's graph or staging
-  tmp.host_stage = nullptr;
-  tmp.host_stage_dev = nullptr;
+  tmp.stage = HostStage{};
   *bytes = layout(&tmp, nullptr);
   return SS_OK;
 }
@@ -1173,25 +1215,27 @@ int ss_step(ss_handle* h, int n_steps, double prev_energy, double* energy_traj, 
   if (n_steps == 0) return take_status(h);
   // each chunk's trajectories and status are written by the kernels into mapped
   // page-locked memory: one synchronisation per chunk and no copies
-  if ((rc = host_staging(h))) return rc;
-  double* hE = h->host_stage;
-  double* hErr = h->host_stage + TRAJ_CAP;
-  volatile int* hstatus = reinterpret_cast<volatile int*>(h->host_stage + 2 * TRAJ_CAP);
-  int* dstatus = reinterpret_cast<int*>(h->host_stage_dev + 2 * TRAJ_CAP);
+  if (!h->stage.host) CK(stage_take(h->stage));
+  double* hE = h->stage.host;
+  double* hErr = h->stage.host + TRAJ_CAP;
+  volatile int* hstatus = reinterpret_cast<volatile int*>(h->stage.host + 2 * TRAJ_CAP);
+  int* dstatus = reinterpret_cast<int*>(h->stage.dev + 2 * TRAJ_CAP);
   double prev = prev_energy;
   for (int done = 0; done < n_steps; done += TRAJ_CAP) {
     const int k = std::min(TRAJ_CAP, n_steps - done);
     *hstatus = -1;
+    h->stage.busy = true;
     rc = dispatch(h, [&](auto* tag) -> int {
       using TH = std::remove_pointer_t<decltype(tag)>;
-      double* dE = h->host_stage_dev;
-      double* dErr = h->host_stage_dev + TRAJ_CAP;
+      double* dE = h->stage.dev;
+      double* dErr = h->stage.dev + TRAJ_CAP;
       if (h->precision == SS_FP32) return Fused<TH, float>::step(h, k, prev, dE, dErr, dstatus);
       return Fused<TH, double>::step(h, k, prev, dE, dErr, dstatus);
     });
     if (rc) return rc;
     prev = NAN;
     CK(cudaStreamSynchronize(h->stream));
+    h->stage.busy = false;
     if (energy_traj) memcpy(energy_traj + done, hE, k * sizeof(double));
     if (err_traj) memcpy(err_traj + done, hErr, k * sizeof(double));
     const int status = *hstatus;
