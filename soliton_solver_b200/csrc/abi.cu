@@ -467,7 +467,7 @@ struct Fused {
     return StepMaps{h->tm[maps + 2 * pair], h->tm[maps + 2 * pair + 1], h->tm[TM_L], h->tm[TM_L + 1]};
   }
   template <bool TMA_, int PH>
-  static int launch_phase(const ss_handle* h, StepArgs<R>& A, const StepMaps* M = nullptr) {
+  static int launch_phase(const ss_handle* h, StepArgs<R>& A) {
     constexpr int NTP = StepShape<TH, R, PH>::NT;
     constexpr size_t smem = step_smem<TH, R, PH, TMA_>();
     auto k = step_kernel<TH, R, TMA_, PH>;
@@ -476,7 +476,7 @@ struct Fused {
     A.tx_extra = take_injection(h, TMA_);
     constexpr int TXP = StepShape<TH, R, PH>::TX;
     const int tiles = ((h->G.X + TXP - 1) / TXP) * ((h->G.Y + TY - 1) / TY);
-    k<<<tiles, NTP, smem, h->stream>>>(M ? *M : phase_maps(h, A, PH == PH_B ? TM_B : TM_A), A);
+    k<<<tiles, NTP, smem, h->stream>>>(phase_maps(h, A, PH == PH_B ? TM_B : TM_A), A);
     CK(cudaGetLastError());
     return SS_OK;
   }
@@ -491,11 +491,26 @@ struct Fused {
     CK(cudaGetLastError());
     return SS_OK;
   }
+  static int launch_energy(const ss_handle* h, StepArgs<R>& A, const CUtensorMap& map) {
+    using SH = EnergyPipe<TH, R>;
+    auto k = step_energy_pipe<TH, R>;
+    static unsigned long long done = 0;  // one per instantiation
+    set_smem(k, SH::SLOTS * SH::SLOT, done);
+    A.tx_extra = take_injection(h, true);
+    const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + SH::TY - 1) / SH::TY);
+    k<<<std::min(tiles, SH::CTAS * h->num_sms), SH::NT, SH::SLOTS * SH::SLOT, h->stream>>>(map, A);
+    CK(cudaGetLastError());
+    return SS_OK;
+  }
   template <int PH>
   static int launch_phase(const ss_handle* h, StepArgs<R>& A) {
     if (!h->tma) return launch_phase<false, PH>(h, A);
-    if (PH == PH_B && h->use_pipe[M_S4]) return launch_phase_pipe(h, A);
-    return launch_phase<true, PH>(h, A);
+    if constexpr (PH == PH_E) {
+      return launch_energy(h, A, phase_maps(h, A, TM_A).phi);
+    } else {
+      if (PH == PH_B && h->use_pipe[M_S4]) return launch_phase_pipe(h, A);
+      return launch_phase<true, PH>(h, A);
+    }
   }
 
   static StepArgs<R> step_args(const ss_handle* h) {
@@ -746,9 +761,9 @@ struct Fused {
       StepArgs<R> S = step_args(h);
       S.with_energy = 1;
       S.phi = (const R*)field;
-      StepMaps M{};
-      const bool tma = encode_tile_map(&M.phi, field, sizeof(R), h->G.X, h->G.Y, TH::NF, false, TXA, TY);
-      return tma ? launch_phase<true, PH_E>(h, S, &M) : launch_phase<false, PH_E>(h, S);
+      CUtensorMap map{};
+      const bool tma = encode_tile_map(&map, field, sizeof(R), h->G.X, h->G.Y, TH::NF, false, TXA, TY);
+      return tma ? launch_energy(h, S, map) : launch_phase<false, PH_E>(h, S);
     }
     ObsList L{};
     L.n = 1;

@@ -396,18 +396,18 @@ __device__ __forceinline__ void issue_step_tile(R* B0, const CUtensorMap* tm_phi
   }
 }
 
-// The reductions that close a phase: the tile's energy partial (A, E) or err (B); the last
-// tile of the lattice sums the partials in a fixed order, updates the arrest state and
-// writes the trajectory slots.
+// The reductions that close a phase: the tile's energy partial (A, E; stored by the caller's own
+// loop over tiles where nblk CTAs walk more: ntiles) or err (B); the last CTA of the lattice sums
+// the partials in a fixed order, updates the arrest state and writes the trajectory slots.
 template <int NT, typename R, int PH>
 __device__ __forceinline__ void step_reductions(const StepArgs<R>& A, StageShared<NT>& S, double e_acc, double err_max,
-                                                int tile, int nblk) {
+                                                int tile, int nblk, int ntiles = 0) {
   StepState* st = A.st;
   if (PH != PH_B && !A.with_energy) return;
   if constexpr (PH == PH_B) {
     const double bm = block_max<NT>(err_max, S.red);
     if (threadIdx.x == 0 && bm > -INFINITY) atomicMax(&st->err_enc, enc_max(bm));
-  } else {
+  } else if (!ntiles) {
     const double bs = block_sum_fixed<NT>(e_acc, S.red);
     if (threadIdx.x == 0) A.partial[tile] = bs;
   }
@@ -425,7 +425,7 @@ __device__ __forceinline__ void step_reductions(const StepArgs<R>& A, StageShare
       if (A.err_traj && A.err_idx >= 0) A.err_traj[A.err_idx] = err;
     }
   } else {
-    const double E = fixed_order_sum<NT>(A.partial, nblk, S.sh_s, S.sh_c);
+    const double E = fixed_order_sum<NT>(A.partial, ntiles ? ntiles : nblk, S.sh_s, S.sh_c);
     if (threadIdx.x == 0) {
       st->scalar = E;
       if (!isfinite(E)) raise_status(st, ST_NONFINITE);
@@ -677,6 +677,83 @@ __global__ void __launch_bounds__((PipeShape<TH, R>::NT), (PipeShape<TH, R>::CTA
     }
   }
   step_reductions<NT, R, PH_B>(A, S, e_acc, err_max, blockIdx.x, gridDim.x);
+}
+
+// Persistent phase E (TMA staging): the resident CTAs walk the tiles through a ring of staged
+// tiles, the next ones' loads in flight behind the current one's stencil.  Tiles, their partials
+// and the order of their sum are those of one tile per CTA: the same energy to the last bit.
+template <class TH, typename R>
+struct EnergyPipe : StepShape<TH, R, PH_E> {
+  using SH = StepShape<TH, R, PH_E>;
+  static constexpr size_t SLOT = tile_buf_bytes<R, TH::NF, SH::TX, SH::TY>();
+  static constexpr int FIT = (int)(216 * 1024 / SH::CTAS / SLOT), SLOTS = FIT > 4 ? 4 : FIT;
+  static_assert(SLOTS >= 2, "a load in flight behind the stencil");
+};
+template <class TH, typename R>
+__global__ void __launch_bounds__((EnergyPipe<TH, R>::NT), (EnergyPipe<TH, R>::CTAS))
+    step_energy_pipe(const __grid_constant__ CUtensorMap map, const __grid_constant__ StepArgs<R> A) {
+  using SH = EnergyPipe<TH, R>;
+  constexpr int TX = SH::TX, TY = SH::TY, NT = SH::NT, SLOTS = SH::SLOTS;
+  using TS = TileShape<TX, TY, NT>;
+  constexpr int BUF = TH::NF * TS::PLANE;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  R* ring = reinterpret_cast<R*>(smem_raw);
+  __shared__ StageShared<NT> S;
+  __shared__ __align__(8) uint64_t full[SLOTS];
+  const Grid& G = A.G;
+  const int tiles_y = (G.Y + TY - 1) / TY;
+  const int ntiles = ((G.X + TX - 1) / TX) * tiles_y;
+  auto issue = [&](int slot, int tile) {
+    mbar_expect_tx(&full[slot], (uint32_t)(sizeof(R) * BUF) + A.tx_extra);
+    tma_load_3d(ring + slot * BUF, &map, (tile % tiles_y) * TY - TS::YOFF, (tile / tiles_y) * TX - 2, 0, &full[slot]);
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < SLOTS; ++s) mbar_init(&full[s], 1);
+    for (int s = 0; s < SLOTS; ++s) {
+      const int t = blockIdx.x + s * gridDim.x;
+      if (t < ntiles) issue(s, t);
+    }
+  }
+  __syncthreads();
+  const int dq = gridDim.x / tiles_y, dr = gridDim.x % tiles_y;
+  int tx_i = blockIdx.x / tiles_y, ty_i = blockIdx.x % tiles_y;
+  int slot = 0;
+  uint32_t parity = 0;
+#pragma unroll 1
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const bool ok = __syncthreads_and(mbar_wait_bounded(&full[slot], parity, A.wait_cycles));
+    if (!ok) {  // record, then wait (bounded) for every load still in flight before leaving
+      if (threadIdx.x == 0) raise_status(A.st, ST_TIMEOUT);
+      for (int s = 0; s < SLOTS && t + s * (int)gridDim.x < ntiles; ++s) {
+        mbar_wait_bounded(&full[slot], parity, A.wait_cycles);
+        if (++slot == SLOTS) {
+          slot = 0;
+          parity ^= 1;
+        }
+      }
+      return;
+    }
+    double e_acc = 0.0, err_max = 0.0;
+    CentreL<typename PairOf<R>::type, 1, 1> none;
+    compute_tile<TH, R, TX, TY, NT, true, PH_E>(A, ring + slot * BUF, none, tx_i * TX, ty_i * TY, false, e_acc, err_max);
+    const double bs = block_sum_fixed<NT>(e_acc, S.red);  // its barriers: every thread is done with this slot
+    if (threadIdx.x == 0) {
+      A.partial[t] = bs;
+      const int nt = t + SLOTS * gridDim.x;
+      if (nt < ntiles) issue(slot, nt);
+    }
+    tx_i += dq;
+    ty_i += dr;
+    if (ty_i >= tiles_y) {
+      ty_i -= tiles_y;
+      ++tx_i;
+    }
+    if (++slot == SLOTS) {
+      slot = 0;
+      parity ^= 1;
+    }
+  }
+  step_reductions<NT, R, PH_E>(A, S, 0.0, 0.0, blockIdx.x, gridDim.x, ntiles);
 }
 
 template <class TH, typename R, bool TMA, int PH>
