@@ -27,6 +27,13 @@
 #include "adjoint.cuh"
 #include "text.cuh"
 #include "theories.cuh"
+#define SSB_INSTANCE extern
+#include "instances.cuh"
+
+namespace ssb {
+SSB_COOP_INSTANCES
+SSB_BATCH_INSTANCES
+}
 
 using namespace ssb;
 
