@@ -805,9 +805,12 @@ struct Fused {
       CK(cudaGetLastError());
       return SS_OK;
     };
-    static unsigned long long done_tma = 0, done_plain = 0;
-    return tma ? go(observe_kernel<TH, R, TX, TY, NT, true>, done_tma)
-               : go(observe_kernel<TH, R, TX, TY, NT, false>, done_plain);
+    static unsigned long long done[4] = {};  // one per instantiation
+    if (L.n == 1)
+      return tma ? go(observe_kernel<TH, R, TX, TY, NT, true, 1>, done[0])
+                 : go(observe_kernel<TH, R, TX, TY, NT, false, 1>, done[1]);
+    return tma ? go(observe_kernel<TH, R, TX, TY, NT, true, OBS_MAX>, done[2])
+               : go(observe_kernel<TH, R, TX, TY, NT, false, OBS_MAX>, done[3]);
   }
   static int density(ss_handle* h, const void* field, double* dens, bool reduce, int kind, int which) {
     ObsList L{};

@@ -509,15 +509,26 @@ struct ObsList {
 // derivatives) of the components they need, the theory's points on them, one fixed-order
 // compensated sum each (partial: n * gridDim.x slots, nullable) and, for n = 1, the density.
 // A thread owns four adjacent rows of one column and takes them two at a time, so that the
-// two rows' x neighbours are read and converted once.  Bound for FP32 fields by the
-// conversions (XU pipe: 16 per clock and SM) and FP64 arithmetic.
-template <class TH, typename R, int TX, int TY, int NT, bool TMA>
-__global__ void __launch_bounds__(NT, (TH::NF <= 4 ? 3 : 2))
+// two rows' x neighbours are read and converted once (six FP64 components would spill: one).
+// Bound for FP32 fields by the conversions (XU pipe: 16 per clock and SM), FP64 arithmetic and,
+// with one tile per CTA, the tiles' load latency.  NQ: 1, or OBS_MAX for several quantities.  One
+// quantity needs registers for its own sum only, and a CTA more per SM hides more of the loads; us,
+// OBS_MAX at three CTAs -> 1 at four: energy 4096^2 chiral 228 -> 189, baby Skyrme 205 -> 166, density
+// 1501 x 999 (plain loads) chiral 26.8 -> 22.7.  A ring of staged tiles under resident CTAs gave the
+// same (189, 160) and slower densities (174 against 187).
+template <class TH, typename R, int NQ>
+struct ObserveShape {
+  static constexpr bool WIDE = TH::NF > 4;
+  static constexpr int PER = NQ == 1 && WIDE && sizeof(R) == 8 ? 1 : 2;
+  static constexpr int CTAS = (WIDE ? 2 : 3) + (NQ == 1 ? 1 : 0);
+};
+template <class TH, typename R, int TX, int TY, int NT, bool TMA, int NQ>
+__global__ void __launch_bounds__(NT, (ObserveShape<TH, R, NQ>::CTAS))
     observe_kernel(const __grid_constant__ CUtensorMap map, const R* __restrict__ phi, double* density, double* partial,
                    StepState* st, const __grid_constant__ ObsList L, const __grid_constant__ Grid G,
                    const __grid_constant__ Phys P, long long wait_cycles, unsigned tx_extra) {
   using TS = TileShape<TX, TY, NT>;
-  constexpr int NF = TH::NF, ROWS = TX / (NT / TY), PER = 2;
+  constexpr int NF = TH::NF, ROWS = TX / (NT / TY), PER = ObserveShape<TH, R, NQ>::PER;
   static_assert(NT % TY == 0 && ROWS % PER == 0, "column mapping");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   R* tile = reinterpret_cast<R*>(smem_raw);
@@ -533,7 +544,7 @@ __global__ void __launch_bounds__(NT, (TH::NF <= 4 ? 3 : 2))
   }
   const double ihx = G.ihx, ihy = G.ihy;
   const int ly = threadIdx.x % TY, gy = y0 + ly;
-  double acc[OBS_MAX] = {0.0, 0.0, 0.0, 0.0};
+  double acc[NQ] = {};
 #pragma unroll 1
   for (int s = 0; s < ROWS; s += PER) {
     const int lx = (threadIdx.x / TY) * ROWS + s;
@@ -567,19 +578,21 @@ __global__ void __launch_bounds__(NT, (TH::NF <= 4 ? 3 : 2))
       const int gx = x0 + lx + p;
       if (gx >= G.X) break;
 #pragma unroll
-      for (int q = 0; q < OBS_MAX; ++q) {
-        if (q >= L.n) break;
+      for (int q = 0; q < NQ; ++q) {
+        if (NQ > 1 && q >= L.n) break;
         const double v = L.kind[q] == D_ENERGY   ? TH::energy(J[p], P, G.dA)
                          : L.kind[q] == D_CHARGE ? TH::charge(J[p], P, L.which[q], G.dA)
                                                  : TH::coupling(J[p], P, L.which[q], G.dA);
         if (q == 0 && density) density[(long long)gx * G.Y + gy] = v;
-        acc[q] += v;
+        acc[q] = __dadd_rn(acc[q], v);  // no contraction: both NQ round alike
       }
     }
   }
   if (!partial) return;
   for (int q = 0; q < L.n; ++q) {
-    const double bs = block_sum_fixed<NT>(q == 0 ? acc[0] : q == 1 ? acc[1] : q == 2 ? acc[2] : acc[3], S.red);
+    double a = acc[0];
+    if constexpr (NQ > 1) a = q == 0 ? a : q == 1 ? acc[1] : q == 2 ? acc[2] : acc[3];
+    const double bs = block_sum_fixed<NT>(a, S.red);
     if (threadIdx.x == 0) partial[(long long)q * gridDim.x + blockIdx.x] = bs;
   }
   if (threadIdx.x == 0) {
