@@ -475,15 +475,14 @@ struct Fused {
   }
   template <bool TMA_, int PH>
   static int launch_phase(const ss_handle* h, StepArgs<R>& A) {
-    constexpr int NTP = StepShape<TH, R, PH>::NT;
+    using SH = StepShape<TH, R, PH, TMA_>;
     constexpr size_t smem = step_smem<TH, R, PH, TMA_>();
     auto k = step_kernel<TH, R, TMA_, PH>;
     static unsigned long long done = 0;  // one per instantiation
     set_smem(k, smem, done);
     A.tx_extra = take_injection(h, TMA_);
-    constexpr int TXP = StepShape<TH, R, PH>::TX;
-    const int tiles = ((h->G.X + TXP - 1) / TXP) * ((h->G.Y + TY - 1) / TY);
-    k<<<tiles, NTP, smem, h->stream>>>(phase_maps(h, A, PH == PH_B ? TM_B : TM_A), A);
+    const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + TY - 1) / TY);
+    k<<<tiles, SH::NT, smem, h->stream>>>(phase_maps(h, A, PH == PH_B ? TM_B : TM_A), A);
     CK(cudaGetLastError());
     return SS_OK;
   }
@@ -612,11 +611,11 @@ struct Fused {
 
   static int launch_a2(const ss_handle* h, const StepArgs<R>& A) {
     constexpr size_t smem = step_smem<TH, R, PH_A, false>();
-    constexpr int CX = StepShape<TH, R, PH_A>::TX;
-    const long long tiles = (long long)((h->G.X + CX - 1) / CX) * ((h->G.Y + TY - 1) / TY);
+    using SH = StepShape<TH, R, PH_A, false>;
+    const long long tiles = (long long)((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + TY - 1) / TY);
     auto go = [&](auto k, unsigned long long& done) -> int {
       set_smem(k, smem, done);
-      k<<<(int)std::min<long long>(tiles, 2 * h->num_sms), StepShape<TH, R, PH_A>::NT, smem, h->stream>>>(A);
+      k<<<(int)std::min<long long>(tiles, 2 * h->num_sms), SH::NT, smem, h->stream>>>(A);
       CK(cudaGetLastError());
       return SS_OK;
     };

@@ -70,16 +70,18 @@ struct StepArgs {
 // for the phase A of the other FP32 theories with up to four components and for the baby
 // Skyrme phase B, else 128 (at most 48 bytes of spills); the s+id model's FP64 stencils take
 // up to 254 and one CTA.
-// Phase B stages four halo buffers: 16 rows where two CTAs' buffers fit an SM (FP32, up to
-// four components), else 8.
-template <class TH, typename R, int PH>
+// Phase B stages four halo buffers by TMA: 16 rows where two CTAs' buffers fit an SM (FP32, up to
+// four components), else 8.  Plain loads stage two (one in E), which fit at 16 rows throughout, and
+// fewer halo rows count there: every element is a load of its own.
+template <class TH, typename R, int PH, bool TMA = true>
 struct StepShape {
   static constexpr int TY = 64, NT = 256;
   static constexpr int BYTES = (int)sizeof(R) * TH::NF;  // per site
   static constexpr bool F32 = sizeof(R) == 4;
-  static constexpr int TX = BYTES <= (PH == PH_B ? 16 : 32) ? 16 : 8;
-  static constexpr int CTAS = TH::NF > 4                       ? (F32 ? 2 : 1)
-                              : !F32                           ? 2
+  static constexpr int TX = !TMA || BYTES <= (PH == PH_B ? 16 : 32) ? 16 : 8;
+  static constexpr int PLAIN_E = PH == PH_E && !TMA ? 1 : 0;  // FP64: one buffer and few registers
+  static constexpr int CTAS = TH::NF > 4                       ? (F32 ? 2 : 1 + PLAIN_E)
+                              : !F32                           ? 2 + PLAIN_E
                               : PH == PH_B                     ? (TH::NF <= 3 ? 3 : 2)
                               : PH == PH_E || TH::S1_CTAS == 4 ? 4
                                                                : 3;
@@ -91,7 +93,8 @@ __host__ __device__ constexpr int step_buffers() {
 }
 template <class TH, typename R, int PH, bool TMA>
 __host__ __device__ constexpr size_t step_smem() {
-  return step_buffers<PH, TMA>() * tile_buf_bytes<R, TH::NF, StepShape<TH, R, PH>::TX, StepShape<TH, R, PH>::TY>();
+  using SH = StepShape<TH, R, PH, TMA>;
+  return step_buffers<PH, TMA>() * tile_buf_bytes<R, TH::NF, SH::TX, SH::TY>();
 }
 
 // The flow's gradient rows of a site pair from the staged field T: jets, theory, forcing,
@@ -757,9 +760,9 @@ __global__ void __launch_bounds__((EnergyPipe<TH, R>::NT), (EnergyPipe<TH, R>::C
 }
 
 template <class TH, typename R, bool TMA, int PH>
-__global__ void __launch_bounds__((StepShape<TH, R, PH>::NT), (StepShape<TH, R, PH>::CTAS))
+__global__ void __launch_bounds__((StepShape<TH, R, PH, TMA>::NT), (StepShape<TH, R, PH, TMA>::CTAS))
     step_kernel(const __grid_constant__ StepMaps M, const __grid_constant__ StepArgs<R> A) {
-  using SH = StepShape<TH, R, PH>;
+  using SH = StepShape<TH, R, PH, TMA>;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ StageShared<SH::NT> S;
   step_tile<TH, R, SH::TX, SH::TY, SH::NT, TMA, PH>(A, &M.phi, &M.vel, &M.l1, &M.l2, blockIdx.x, gridDim.x,
@@ -770,8 +773,8 @@ __global__ void __launch_bounds__((StepShape<TH, R, PH>::NT), (StepShape<TH, R, 
 // resident grid walks the tiles with plain loads (it runs once in a while, and an idle launch
 // must cost no more than its CTAs' start: 28 us with one CTA per tile at 4096^2).
 template <class TH, typename R, bool FUSED_T2>
-__global__ void __launch_bounds__((StepShape<TH, R, PH_A>::NT)) step_a2_kernel(const __grid_constant__ StepArgs<R> A) {
-  using SH = StepShape<TH, R, PH_A>;
+__global__ void __launch_bounds__((StepShape<TH, R, PH_A, false>::NT)) step_a2_kernel(const __grid_constant__ StepArgs<R> A) {
+  using SH = StepShape<TH, R, PH_A, false>;
   constexpr int TX = SH::TX, TY = SH::TY, NT = SH::NT, NF = TH::NF;
   if (__ldcg(&A.st->l2_missing) == 0) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
