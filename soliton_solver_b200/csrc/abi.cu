@@ -637,10 +637,10 @@ struct Fused {
     A.E_traj = E_dev;
     A.err_traj = err_dev;
     int rc, cur = 0;
-    // An odd count would end in the other pair.  With TMA staging its first phase A copies phi and
-    // V there on the way, so that phase B writes the caller's buffers and nothing is copied back.
-    // 4096^2 chiral magnet FP32, one-step call: phase A 244 -> 266 us, phase E 165 -> 122, finish 137 -> 6.
-    const bool land = h->tma && (n & 1);
+    // An odd count would end in the other pair.  Its first phase A copies phi and V there on the
+    // way, so that phase B writes the caller's buffers and nothing is copied back.  4096^2 chiral
+    // magnet FP32, one-step call: phase A 244 -> 266 us, phase E 165 -> 122, finish 137 -> 6.
+    const bool land = n & 1;
     for (int s = 0; s < n; ++s, cur ^= 1) {
       A.copy_phi = land && s == 0 ? (R*)h->phi2 : nullptr;
       A.copy_vel = land && s == 0 ? (R*)h->vel2 : nullptr;
@@ -664,16 +664,14 @@ struct Fused {
       set_input(h, A, cur);
       if ((rc = launch_phase<PH_B>(h, A))) return rc;
     }
-    // trailing energy of the final field and its arrest test; phi back to the caller's buffer
+    // trailing energy of the final field (cur is 0: the caller's) and its arrest test
     A.predict = 0;
     A.with_energy = A.arrest_update = 1;
     A.E_idx = n - 1;
-    A.phi_out = cur ? (R*)h->field : nullptr;
-    set_input(h, A, cur);
+    set_input(h, A, 0);
     if ((rc = launch_phase<PH_E>(h, A))) return rc;
     const long long nfN = (long long)h->nf * h->G.N;
-    step_finish_kernel<R><<<grid_1d(nfN), 256, 0, h->stream>>>((R*)h->vel, cur ? (const R*)h->vel2 : nullptr, nfN,
-                                                               h->st, status_out);
+    step_finish_kernel<R><<<grid_1d(nfN), 256, 0, h->stream>>>((R*)h->vel, nfN, h->st, status_out);
     CK(cudaGetLastError());
     return SS_OK;
   }
@@ -1843,7 +1841,10 @@ struct Batched {
       B.init_state = s == 0;
       B.prev_energy = (s == 0 && use_prev) ? b->d_prev : nullptr;
       B.E_idx = s - 1;
+      B.copy = s == 0 && (n & 1);  // as for a single lattice: the count ends in the caller's buffers
       if ((rc = launch<PH_A>(b, B))) return rc;
+      if (B.copy) B.cur = 1;
+      B.copy = 0;
       B.init_state = 0;
       B.prev_energy = nullptr;
       B.err_idx = s;
@@ -1852,7 +1853,7 @@ struct Batched {
     B.with_energy = B.arrest_update = 1;
     B.E_idx = n - 1;
     if ((rc = launch<PH_E>(b, B))) return rc;
-    batch_finish_kernel<R, TH::NF><<<dim3(64, b->n), 256, 0, b->stream>>>(b->d_insts, B.cur);
+    batch_finish_kernel<R, TH::NF><<<dim3(64, b->n), 256, 0, b->stream>>>(b->d_insts);
     CK(cudaGetLastError());
     return SS_OK;
   }

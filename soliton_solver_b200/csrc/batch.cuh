@@ -31,7 +31,8 @@ struct BatchInst {
 };
 
 struct BatchStep {
-  int cur;  // the pair that holds phi and V: 0 the caller's, 1 the workspace's
+  int cur;   // the pair that holds phi and V: 0 the caller's, 1 the workspace's
+  int copy;  // A: phi and V to the workspace's pair (first step of an odd count)
   int with_energy, arrest_update, init_state;
   int E_idx, err_idx;
   const double* prev_energy;  // device, one per lattice (NaN keeps E_last); read with init_state
@@ -86,9 +87,10 @@ __global__ void __launch_bounds__((BatchShape<TH, R, PH, SMALL>::NT), (BatchShap
     A.vel = (const R*)I.buf[in + 1];
     A.l1 = A.out_l1 = (R*)I.buf[BB_L1];
     A.l2 = A.out_l2 = (R*)I.buf[BB_L2];
-    A.phi_out = PH == PH_E && !B.cur ? nullptr : (R*)I.buf[out];
+    A.phi_out = (R*)I.buf[out];
     A.vel_out = (R*)I.buf[out + 1];
-    A.copy_phi = A.copy_vel = nullptr;
+    A.copy_phi = B.copy ? (R*)I.buf[BB_PHI2] : nullptr;
+    A.copy_vel = B.copy ? (R*)I.buf[BB_VEL2] : nullptr;
     A.force = nullptr;
     A.partial = I.partial;
     A.st = I.st;
@@ -109,17 +111,15 @@ __global__ void __launch_bounds__((BatchShape<TH, R, PH, SMALL>::NT), (BatchShap
 }
 
 // Apply each lattice's pending arrest (V = 0), left by the trailing energy pass, at the
-// end of a call, or copy V out of the workspace's pair (cur = 1).  grid.y = lattice.
+// end of a call.  grid.y = lattice.
 template <typename R, int NF>
-__global__ void batch_finish_kernel(const BatchInst* __restrict__ insts, int cur) {
+__global__ void batch_finish_kernel(const BatchInst* __restrict__ insts) {
   const BatchInst& I = insts[blockIdx.y];
-  const bool arrest = I.st->arrest != 0;
-  if (!arrest && !cur) return;
+  if (!I.st->arrest) return;
   R* dv = (R*)I.buf[BB_VEL];
-  const R* src = (const R*)I.buf[BB_VEL2];
   const long long n = (long long)NF * I.G.N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dv[i] = arrest ? (R)0 : src[i];
+    dv[i] = (R)0;
 }
 
 }  // namespace ssb

@@ -12,9 +12,8 @@
 //   phase A  reads phi, V          writes l1, l2     (+ the energy of phi)
 //   phase B  reads phi, V, l1, l2  writes phi', V'   (+ err)
 // 10 words per site and step, two launches.  Phase B reads the neighbours of phi and V, so
-// steps alternate between the caller's buffers and a pair in the workspace; after an odd
-// number of steps the trailing energy pass (phase E), which reads phi anyway, copies phi
-// back and the finish kernel copies V.
+// steps alternate between the caller's buffers and a pair in the workspace; an odd number of
+// steps starts in that pair: the first phase A, which reads phi and V anyway, copies them there.
 // The energy of a step's result is computed by the next step's phase A.  The arrest it
 // decides (V = 0) is applied by phase B: V = 0 means T2 = T1, so l2 = l1 and phase B takes
 // l1 for l2 (and loads neither V nor l2); phase A's l2, computed before the decision, is
@@ -43,9 +42,9 @@ struct StepArgs {
   const R* l2;  // B
   R* out_l1;    // A
   R* out_l2;    // A
-  R* phi_out;   // B: phi';  E: copy of phi (nullable)
+  R* phi_out;   // B: phi'
   R* vel_out;   // B: V'
-  R* copy_phi;  // A, TMA staging (nullable): copies of phi and V for phase B to read
+  R* copy_phi;  // A (nullable): copies of phi and V for phase B to read
   R* copy_vel;
   const double* force;  // FP64 fields (nullable): added to the gradient rows in every stage
   double* partial;      // one energy partial per tile (A, E)
@@ -147,8 +146,7 @@ __device__ __forceinline__ double pair_energy(const Jet<V, TH::NF>& J, const Phy
   }
 }
 
-// Phase A (l1, l2 and the energy; skip: no l2), A2 (l2) or E (the energy, and a copy of phi) of
-// a staged tile.
+// Phase A (l1, l2 and the energy; skip: no l2), A2 (l2) or E (the energy) of a staged tile.
 template <class TH, typename R, int TX, int TY, int NT, bool FAST, int PH>
 __device__ __forceinline__ void first_half(const StepArgs<R>& A, const R* T1, const R* T2, int x0, int y0,
                                            bool skip, double* e_acc) {
@@ -184,10 +182,6 @@ __device__ __forceinline__ void first_half(const StepArgs<R>& A, const R* T1, co
     if constexpr (PH == PH_E) {
       tile_jet<TH, V, R, TS::HY, TS::PLANE, FAST>(T1, toff, kc, m0, m1, J);
       e_sum += pair_energy<TH, V, R>(J, A.P, v1, chk);
-      if (A.phi_out) {
-#pragma unroll
-        for (int a = 0; a < NF; ++a) gstore<V, R>(A.phi_out + a * N + sidx, J.f[a], FAST, v1);
-      }
     } else {
       V g[NF];
       if constexpr (PH == PH_A) {
@@ -301,8 +295,8 @@ __device__ __forceinline__ void second_half(const StepArgs<R>& A, const R* T3, c
 
 // Plain-load staging of a phase (row pitch not a multiple of 16 bytes): T1 = phi and T2 (A),
 // T1 (E) or T3 and T4 (B; an arrested step takes V = 0 and l1 for l2) into D0 and D1.  Every
-// thread issues the loads of one component plane before it combines them.  FUSED_T2: T2 rounded
-// as in TMA-staged tiles.
+// thread issues the loads of one component plane before it combines them; the tile's own phi and
+// V also go to copy_phi and copy_vel (A, where set).  FUSED_T2: T2 rounded as in TMA-staged tiles.
 template <int NF, typename R, int TX, int TY, int NT, int PH, bool FUSED_T2 = false>
 __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int x0, int y0, bool arrest) {
   using TS = TileShape<TX, TY, NT>;
@@ -310,7 +304,7 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
   const Grid& G = A.G;
   const R dt = (R)G.dt;
   long long off[KM];
-  bool ok[KM];
+  bool ok[KM], own[PH == PH_A ? KM : 1];
 #pragma unroll
   for (int k = 0; k < KM; ++k) {
     const int i = threadIdx.x + k * NT;
@@ -318,6 +312,7 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
     const int gx = x0 - 2 + r, gy = y0 - TS::YOFF + c;
     ok[k] = i < TS::PLANE && gx >= 0 && gx < G.X && gy >= 0 && gy < G.Y;
     off[k] = (long long)gx * G.Y + gy;
+    if constexpr (PH == PH_A) own[k] = ok[k] && r >= 2 && r < TX + 2 && c >= TS::YOFF && c < TS::YOFF + TY;
   }
 #pragma unroll 1
   for (int a = 0; a < NF; ++a) {
@@ -342,6 +337,12 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
         D1[a * TS::PLANE + i] = vfma(dt, vfma((R)0.5, l2, v[k]), p[k]);
       } else {
         D0[a * TS::PLANE + i] = p[k];
+        if constexpr (PH == PH_A) {
+          if (A.copy_phi && own[k]) {
+            A.copy_phi[base + off[k]] = p[k];
+            A.copy_vel[base + off[k]] = v[k];
+          }
+        }
         if constexpr (PH == PH_A)
           D1[a * TS::PLANE + i] = FUSED_T2 ? vfma(grid_k<R>(G, GK_HDT), v[k], p[k]) : stage_t2<R>(p[k], v[k], dt);
       }
@@ -791,16 +792,14 @@ __global__ void __launch_bounds__((StepShape<TH, R, PH_A, false>::NT)) step_a2_k
   }
 }
 
-// End of a call: a pending arrest left by the trailing energy pass (V = 0), the copy of V out
-// of the workspace after an odd number of steps (src non-null), and the call's status to
-// status_out (nullable; e.g. mapped host memory).
+// End of a call: a pending arrest left by the trailing energy pass (V = 0) and the call's status
+// to status_out (nullable; e.g. mapped host memory).
 template <typename R>
-__global__ void step_finish_kernel(R* vel, const R* src, long long n, const StepState* st, int* status_out) {
+__global__ void step_finish_kernel(R* vel, long long n, const StepState* st, int* status_out) {
   if (status_out && blockIdx.x == 0 && threadIdx.x == 0) *(volatile int*)status_out = st->status;
-  const bool arrest = st->arrest != 0;
-  if (!arrest && !src) return;
+  if (!st->arrest) return;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    vel[i] = arrest ? (R)0 : src[i];
+    vel[i] = (R)0;
 }
 
 }  // namespace ssb
