@@ -46,7 +46,9 @@ template <class TH, typename R, int PH, bool SMALL>
 struct BatchShape {
   using SH = StepShape<TH, R, PH>;
   static constexpr int TX = SMALL ? 8 : SH::TX, TY = SMALL ? 32 : SH::TY, NT = SMALL ? 128 : SH::NT;
-  static constexpr int CTAS = SMALL ? (TH::NF > 4 ? 4 : PH == PH_B ? 5 : 6) : SH::CTAS;
+  // (FP64 phase E stages one buffer and needs few registers: one CTA more, as with plain rows)
+  static constexpr int CTAS = SMALL ? (TH::NF > 4 ? 4 : PH == PH_B ? 5 : 6)
+                                    : SH::CTAS + (PH == PH_E && sizeof(R) == 8 ? 1 : 0);
 };
 
 template <class TH, typename R, bool SMALL, bool TMA, int PH>
