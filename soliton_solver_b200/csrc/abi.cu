@@ -193,8 +193,11 @@ struct ss_handle {
   bool tma = false;
   int num_sms = 148;
   // per flow mode: 1 = persistent pipelined kernel, 0 = one tile per CTA (autotuned).  The
-  // gradient's (0) and phase B's (3, 4) are read; 1, 2, 5 and fuse23 are kept as pinned
-  int use_pipe[N_FLOW_MODES] = {1, 1, 1, 1, 1, 1, 0};
+  // gradient's (0) and phase B's (3, 4) are read; 1, 2, 5 and fuse23 are kept as pinned.  The
+  // gradient starts with one tile per CTA: us FP32 2048^2, pipelined -> one tile, chiral magnet 43 ->
+  // 33, baby Skyrme 48 -> 33, Abelian Higgs 47 -> 33, s+id 77 -> 62; 1024^2 13.5 -> 10.5, 14.5 -> 12.4,
+  // 14.5 -> 10.5, 22.7 -> 18.6.
+  int use_pipe[N_FLOW_MODES] = {0, 1, 1, 1, 1, 1, 0};
   float tune_ms[N_FLOW_MODES][2] = {};
   int fuse23 = 1;  // stages 2 and 3 in one kernel (TMA staging only)
   long long wait_cycles = WAIT_CYCLES;

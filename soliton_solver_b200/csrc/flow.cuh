@@ -416,9 +416,20 @@ __device__ __forceinline__ bool stage_tma(R* T, const CUtensorMap* map, uint64_t
   return ok;
 }
 
+// CTAs per SM of the gradient hook, one tile per CTA: its tiles' load latency is hidden by the other
+// CTAs only.  us at 2048^2 (plain rows 1501 x 999), registers unbounded -> bounded for the CTAs below:
+// FP64 chiral magnet 65 -> 56 (33 -> 31), Abelian Higgs 68 -> 56 (33 -> 29), baby Skyrme 66 -> 66 (41 ->
+// 31; three CTAs 35), s+id 176 -> 115 (74 -> 64; three CTAs spill: 236); s+id FP32 69 -> 62 (37 -> 33).
+// FP32 stencils of up to four components take 56 to 66 registers unbounded: four CTAs.
+template <class TH, typename R>
+__host__ __device__ constexpr int grad_ctas() {
+  if (sizeof(R) == 4) return TH::NF > 4 ? 3 : 4;
+  return TH::NF == 4 ? 3 : 2;
+}
+
 // The gradient hook, one tile per CTA.
 template <class TH, typename R, int TX, int TY, int NT, bool TMA>
-__global__ void __launch_bounds__(NT) flow_kernel(const __grid_constant__ FlowArgs<R> A) {
+__global__ void __launch_bounds__(NT, (grad_ctas<TH, R>())) flow_kernel(const __grid_constant__ FlowArgs<R> A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t bar;
   R* T = reinterpret_cast<R*>(smem_raw);
