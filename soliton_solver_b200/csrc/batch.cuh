@@ -45,7 +45,9 @@ struct BatchStep {
 template <class TH, typename R, int PH, bool SMALL>
 struct BatchShape {
   using SH = StepShape<TH, R, PH>;
-  static constexpr int TX = SMALL ? 8 : SH::TX, TY = SMALL ? 32 : SH::TY, NT = SMALL ? 128 : SH::NT;
+  // six FP64 components run phase A at one CTA per SM: 16 rows, so that fewer loads are waited for
+  static constexpr bool TALL = PH != PH_B && sizeof(R) == 8 && TH::NF > 4;
+  static constexpr int TX = SMALL ? 8 : TALL ? 16 : SH::TX, TY = SMALL ? 32 : SH::TY, NT = SMALL ? 128 : SH::NT;
   // (FP64 phase E stages one buffer and needs few registers: one CTA more, as with plain rows)
   static constexpr int CTAS = SMALL ? (TH::NF > 4 ? 4 : PH == PH_B ? 5 : 6)
                                     : SH::CTAS + (PH == PH_E && sizeof(R) == 8 ? 1 : 0);
