@@ -84,14 +84,13 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // 3-D map over component planes (dims y, x, component) whose box is one staged
 // tile: (TY + 8) x (TX + 4) x NF.  Fails (-> plain loads) when the buffer or its
 // row pitch is not 16-byte aligned.
-bool encode_tile_map(CUtensorMap* m, const void* ptr, size_t es, int X, int Y, int NF, bool centre = false,
-                     int tx = TX, int ty = TY) {
+bool encode_tile_map(CUtensorMap* m, const void* ptr, size_t es, int X, int Y, int NF, int tx = TX, int ty = TY) {
   if (!ptr || ((uintptr_t)ptr) % 16 || ((size_t)Y * es) % 16) return false;
   auto fn = encode_fn();
   if (!fn) return false;
   cuuint64_t dims[3] = {(cuuint64_t)Y, (cuuint64_t)X, (cuuint64_t)NF};
   cuuint64_t strides[2] = {(cuuint64_t)Y * es, (cuuint64_t)X * Y * es};
-  cuuint32_t box[3] = {(cuuint32_t)(centre ? ty : ty + 8), (cuuint32_t)(centre ? tx : tx + 4), (cuuint32_t)NF};
+  cuuint32_t box[3] = {(cuuint32_t)(ty + 8), (cuuint32_t)(tx + 4), (cuuint32_t)NF};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(m, es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
                   const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -245,7 +244,7 @@ size_t layout(ss_handle* h, char* base) {
     h->l[2] = h->l[3] = nullptr;
     h->phi2 = take(field_bytes);
     h->vel2 = take(field_bytes);
-    take(field_bytes);  // five field-sized buffers, the size callers know (scratch of the exact gradient)
+    take(field_bytes);  // unused: callers know the workspace as five field-sized buffers at least
   }
   return off;
 }
@@ -493,10 +492,10 @@ struct Fused {
     using SH = PipeShape<TH, R>;
     auto k = step_kernel_pipe<TH, R>;
     static unsigned long long done = 0;  // one per instantiation
-    set_smem(k, SH::SLOTS * SH::SLOT, done);
+    set_smem(k, SH::SMEM, done);
     A.tx_extra = take_injection(h, true);
     const int tiles = ((h->G.X + SH::TX - 1) / SH::TX) * ((h->G.Y + SH::TY - 1) / SH::TY);
-    k<<<std::min(tiles, SH::CTAS * h->num_sms), SH::NT, SH::SLOTS * SH::SLOT, h->stream>>>(phase_maps(h, A, TM_B), A);
+    k<<<std::min(tiles, SH::CTAS * h->num_sms), SH::NT, SH::SMEM, h->stream>>>(phase_maps(h, A, TM_B), A);
     CK(cudaGetLastError());
     return SS_OK;
   }
@@ -769,7 +768,7 @@ struct Fused {
       S.with_energy = 1;
       S.phi = (const R*)field;
       CUtensorMap map{};
-      const bool tma = encode_tile_map(&map, field, sizeof(R), h->G.X, h->G.Y, TH::NF, false, TXA, TY);
+      const bool tma = encode_tile_map(&map, field, sizeof(R), h->G.X, h->G.Y, TH::NF, TXA, TY);
       return tma ? launch_energy(h, S, map) : launch_phase<false, PH_E>(h, S);
     }
     ObsList L{};
@@ -948,10 +947,17 @@ void step_shape(const ss_handle* h, int& txa, int& txb) {
 
 // Whether (and in which tile shape) the handle's steps run cooperatively: 1 + shape, or 0.
 // The first shape whose tiles are all resident: wherever one fits, the cooperative step was
-// the faster (us per step, two launches -> cooperative: chiral magnet FP32 150 x 200 19.6 ->
-// 7.1, 321 x 256 19.6 -> 10.5, 384 x 400 26.6 -> 15.5, 512 x 560 27.4 -> 18.9; FP64 240 x 256
-// 24.7 -> 11.1, 321 x 256 28.6 -> 20.8; s+id FP32 240 x 256 22.7 -> 11.3), and of two shapes
-// that fit the smaller tile (10.5 against 12.9 and 12.7 at 321 x 256).
+// the faster.  us per step, two launches -> cooperative, by shape:
+//                    8 x 32                      16 x 32                      16 x 64
+//   FP32 chiral      320 x 320 25.1 -> 11.5      420 x 500 31.0 -> 16.9       512 x 560 30.8 -> 18.9
+//        baby        320 x 320 26.3 -> 11.7      544 x 544 32.5 -> 20.1
+//        Higgs       320 x 320 21.0 -> 11.4      420 x 500 27.2 -> 16.6       512 x 560 27.2 -> 19.6
+//        s+id        256 x 256 24.2 -> 12.1      333 x 400 29.1 -> 20.8
+//   FP64 chiral      256 x 256 30.0 -> 11.7                                   333 x 400 32.9 -> 22.2
+//        baby        256 x 256 29.3 -> 11.9      333 x 400 31.6 -> 21.5
+//        Higgs       256 x 256 25.2 -> 11.8                                   333 x 400 27.9 -> 20.3
+//        s+id        128 x 128 27.2 -> 11.4      256 x 256 28.5 -> 27.1
+// Of two shapes that fit the smaller tile (10.5 against 12.9 and 12.7, FP32 chiral 321 x 256).
 int coop_plan(const ss_handle* h) {
   if (h->pinned) return 0;
   int dev = 0, ok = 0;
@@ -1131,10 +1137,10 @@ int ss_bind(ss_handle* h, void* field, void* velocity, void* workspace, size_t w
     step_shape(h, txa, txb);
     bool ok = true;
     for (int i = 0; i < 4 && ok; ++i)
-      ok = encode_tile_map(&h->tm[TM_A + i], pairs[i], h->elem, h->G.X, h->G.Y, h->nf, false, txa, TY) &&
-           encode_tile_map(&h->tm[TM_B + i], pairs[i], h->elem, h->G.X, h->G.Y, h->nf, false, txb, TY);
+      ok = encode_tile_map(&h->tm[TM_A + i], pairs[i], h->elem, h->G.X, h->G.Y, h->nf, txa, TY) &&
+           encode_tile_map(&h->tm[TM_B + i], pairs[i], h->elem, h->G.X, h->G.Y, h->nf, txb, TY);
     for (int i = 0; i < 2 && ok; ++i)
-      ok = encode_tile_map(&h->tm[TM_L + i], h->l[i], h->elem, h->G.X, h->G.Y, h->nf, false, txb, TY);
+      ok = encode_tile_map(&h->tm[TM_L + i], h->l[i], h->elem, h->G.X, h->G.Y, h->nf, txb, TY);
     h->tma = ok;
   }
   h->coop = 0;
@@ -1208,7 +1214,7 @@ int ss_set_variant(ss_handle* h, int mode, int variant) {
     return SS_OK;
   }
   h->use_pipe[mode] = variant;
-  if (mode == M_S1) h->use_pipe[M_ENERGY] = variant;  // the energy pass reduces exactly like stage 1
+  if (mode == M_S1) h->use_pipe[M_ENERGY] = variant;  // reported only
   return SS_OK;
 }
 
@@ -1514,7 +1520,8 @@ int ss_observables(ss_handle* h, const void* field, int n, const int* kinds, con
     if (kinds[i] == SS_OBS_COUPLING && !theory_has_coupling(h->theory, which[i]))
       return fail(SS_ERR_ARG, "coupling %d not defined for theory %d", which[i], h->theory);
     if (h->precision != SS_FP32 && kinds[i] == SS_OBS_ENERGY) {
-      // the flow's own FP64 energy (ss_energy): equal to the last step's to the last bit
+      // the flow's own FP64 energy (ss_energy): the two-launch step's to the last bit, a cooperative
+      // step's to rounding (other tiles)
       if ((rc = ss_energy(h, field, out + i))) return rc;
       continue;
     }
@@ -1902,7 +1909,7 @@ bool batch_encode(ss_batch* b, int i) {
   const int sh = b->shape[i];
   bool ok = true;
   for (int k = 0; k < BT_COUNT && ok; ++k)
-    ok = encode_tile_map(&I.tm[k], I.buf[BATCH_TM_BUF[k]], b->elem, I.G.X, I.G.Y, b->nf, false,
+    ok = encode_tile_map(&I.tm[k], I.buf[BATCH_TM_BUF[k]], b->elem, I.G.X, I.G.Y, b->nf,
                          batch_tx(b, sh, k >= BT_B ? 1 : 0), BSHAPE_TY[sh]);
   return ok;
 }
@@ -2159,7 +2166,7 @@ int ss_batch_autotune(ss_batch* b, int iters, float* ms_out) {
   if (ms_out)
     for (int i = 0; i < b->n; ++i)
       for (int sh = 0; sh < N_BATCH_SHAPES; ++sh) ms_out[2 * i + sh] = ms[cls[i] * N_BATCH_SHAPES + sh];
-  // the timing steps ran the stages with every state update off; only the ticket and
+  // the timing steps ran the phases with every state update off; only the ticket and
   // err slots they reset were touched
   return SS_OK;
 }

@@ -57,9 +57,9 @@ __device__ __forceinline__ S phys_k(const Phys& P, int i) {
 // Device-side state of one lattice's flow (lives in the caller's workspace).
 struct StepState {
   double E_last;                 // energy the next arrest test compares against
-  unsigned long long err_enc;    // running signed max of the stage-4 gradient (ordered encoding)
+  unsigned long long err_enc;    // running signed max of phase B's second gradient (ordered encoding)
   unsigned int ticket;           // last-block-done counter, reset by the last block
-  int arrest;                    // 1: treat the velocity as zero in this step's stages 2-4
+  int arrest;                    // 1: phase B takes the velocity as zero and l1 for l2
   int status;                    // 0 ok, SS_ERR_NONFINITE on a non-finite reduction
   int streak;                    // arrested steps in a row (saddle flows: predicts the next)
   double scalar;                 // result slot of single reductions (energy / charge / coupling)
@@ -265,7 +265,7 @@ __device__ inline void two_sum_add(double& s, double& c, double s2, double c2) {
 // then the NT (sum, error) pairs meet in a fixed xor tree (warps, then warp 0 over the
 // warps' pairs).  The tree is a chain of log2(NT) dependent TwoSums: one thread adding
 // the NT pairs in turn was a serial chain of 256 of them and most of a small lattice's
-// energy pass (320^2 FP32: stage 1 with its energy 12.6 us, with the tree 8.3 us; without energy 5.3 us).
+// energy pass (320^2 FP32, a gradient kernel with its energy: serial 12.6 us, tree 8.3, without the energy 5.3).
 template <int NT>
 __device__ inline double fixed_order_sum(const double* partial, int nb, double* sh_s, double* sh_c) {
   constexpr int NW = NT / 32;

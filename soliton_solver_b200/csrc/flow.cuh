@@ -253,7 +253,7 @@ struct ScaledValue<float> {
 
 // FP64 energy of an FP32 site pair from the jets the gradient stencil already built
 // (f, dx, dy after masking): the theory's energy point evaluated in FP64 on the
-// converted jets, so a flow stage pays no second stencil for its energy.  The jets
+// converted jets, so phase A pays no second stencil for its energy.  The jets
 // carry FP32 rounding (~1e-7 relative per site), the precision the flow's gradient
 // has.  `chk` folds v * 0 of every jet value (Inf/NaN -> NaN, see ScaledValue).
 template <class TH, typename V, int NF>

@@ -67,8 +67,8 @@ struct StepArgs {
 // Tile rows, threads and resident CTAs per SM of each phase (tiles are TX x 64 sites, a
 // warp owns rows).  Registers follow from the CTAs: 64 for the chiral magnet's phase A, 80
 // for the phase A of the other FP32 theories with up to four components and for the baby
-// Skyrme phase B, else 128 (at most 48 bytes of spills); the s+id model's FP64 stencils take
-// up to 254 and one CTA.
+// Skyrme phase B, else 128 (at most 52 bytes of spills; in the batched kernels up to 188, FP64 baby
+// Skyrme's phase B); the s+id model's FP64 stencils take up to 255 and one CTA.
 // Phase B stages four halo buffers by TMA: 16 rows where two CTAs' buffers fit an SM (FP32, up to
 // four components), else 8.  Plain loads stage two (one in E), which fit at 16 rows throughout, and
 // fewer halo rows count there: every element is a load of its own.
@@ -597,8 +597,7 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
 template <class TH, typename R>
 struct PipeShape : StepShape<TH, R, PH_B> {
   using SH = StepShape<TH, R, PH_B>;
-  static constexpr size_t SLOT = 4 * tile_buf_bytes<R, TH::NF, SH::TX, SH::TY>();
-  static constexpr int SLOTS = 1;
+  static constexpr size_t SMEM = 4 * tile_buf_bytes<R, TH::NF, SH::TX, SH::TY>();
 };
 
 template <class TH, typename R>
@@ -606,79 +605,60 @@ __global__ void __launch_bounds__((PipeShape<TH, R>::NT), (PipeShape<TH, R>::CTA
     step_kernel_pipe(const __grid_constant__ StepMaps M, const __grid_constant__ StepArgs<R> A) {
   using SH = PipeShape<TH, R>;
   using V = typename PairOf<R>::type;
-  constexpr int TX = SH::TX, TY = SH::TY, NT = SH::NT, NF = TH::NF, SLOTS = SH::SLOTS;
+  constexpr int TX = SH::TX, TY = SH::TY, NT = SH::NT, NF = TH::NF;
   using TS = TileShape<TX, TY, NT>;
-  constexpr int BUF = NF * TS::PLANE, SLOT = 4 * BUF;
+  constexpr int BUF = NF * TS::PLANE;
   constexpr int PASSES = TX / (NT / (TY / 2));
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  R* ring = reinterpret_cast<R*>(smem_raw);
+  R* B0 = reinterpret_cast<R*>(smem_raw);
   __shared__ StageShared<NT> S;
-  __shared__ __align__(8) uint64_t full[SLOTS];
   const Grid& G = A.G;
   const int tiles_y = (G.Y + TY - 1) / TY;
   const int ntiles = ((G.X + TX - 1) / TX) * tiles_y;
   const bool arrest = __ldcg(&A.st->arrest) != 0;
   constexpr uint32_t bytes = (uint32_t)(sizeof(R) * BUF);
   const uint32_t tx = bytes * (arrest ? 2 : 4) + A.tx_extra;
-  auto issue = [&](int slot, int tile) {
-    R* b = ring + slot * SLOT;
+  auto issue = [&](int tile) {
     const int c0 = (tile % tiles_y) * TY - TS::YOFF, c1 = (tile / tiles_y) * TX - 2;
-    mbar_expect_tx(&full[slot], tx);
-    tma_load_3d(b, &M.phi, c0, c1, 0, &full[slot]);
-    tma_load_3d(b + 2 * BUF, &M.l1, c0, c1, 0, &full[slot]);
+    mbar_expect_tx(&S.bar, tx);
+    tma_load_3d(B0, &M.phi, c0, c1, 0, &S.bar);
+    tma_load_3d(B0 + 2 * BUF, &M.l1, c0, c1, 0, &S.bar);
     if (!arrest) {
-      tma_load_3d(b + BUF, &M.vel, c0, c1, 0, &full[slot]);
-      tma_load_3d(b + 3 * BUF, &M.l2, c0, c1, 0, &full[slot]);
+      tma_load_3d(B0 + BUF, &M.vel, c0, c1, 0, &S.bar);
+      tma_load_3d(B0 + 3 * BUF, &M.l2, c0, c1, 0, &S.bar);
     }
   };
   if (threadIdx.x == 0) {
-    for (int s = 0; s < SLOTS; ++s) mbar_init(&full[s], 1);
-    for (int s = 0; s < SLOTS; ++s) {
-      const int t = blockIdx.x + s * gridDim.x;
-      if (t < ntiles) issue(s, t);
-    }
+    mbar_init(&S.bar, 1);
+    if (blockIdx.x < ntiles) issue(blockIdx.x);
   }
   __syncthreads();
   double e_acc = 0.0, err_max = -INFINITY;
   const int dq = gridDim.x / tiles_y, dr = gridDim.x % tiles_y;
   int tx_i = blockIdx.x / tiles_y, ty_i = blockIdx.x % tiles_y;
-  int slot = 0;
   uint32_t parity = 0;
 #pragma unroll 1
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const bool ok = __syncthreads_and(mbar_wait_bounded(&full[slot], parity, A.wait_cycles));
-    if (!ok) {  // record, then wait (bounded) for every load still in flight before leaving
+    const bool ok = __syncthreads_and(mbar_wait_bounded(&S.bar, parity, A.wait_cycles));
+    if (!ok) {  // record, then wait (bounded) for the loads still in flight before leaving
       if (threadIdx.x == 0) raise_status(A.st, ST_TIMEOUT);
-      for (int s = 0; s < SLOTS && t + s * (int)gridDim.x < ntiles; ++s) {
-        mbar_wait_bounded(&full[slot], parity, A.wait_cycles);
-        if (++slot == SLOTS) {
-          slot = 0;
-          parity ^= 1;
-        }
-      }
+      mbar_wait_bounded(&S.bar, parity, A.wait_cycles);
       return;
     }
-    R* B0 = ring + slot * SLOT;
     CentreL<V, NF, PASSES> C;
     combine_tile<TH, R, TX, TY, NT, PH_B>(G, B0, arrest, C);
     compute_tile<TH, R, TX, TY, NT, true, PH_B>(A, B0, C, tx_i * TX, ty_i * TY, arrest, e_acc, err_max);
-    // order this tile's in-place writes before the next bulk copy into the slot
+    // order this tile's in-place writes before the next bulk copies into its buffers
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();  // every thread is done with this slot
-    if (threadIdx.x == 0) {
-      const int nt = t + SLOTS * gridDim.x;
-      if (nt < ntiles) issue(slot, nt);
-    }
+    __syncthreads();  // every thread is done with them
+    if (threadIdx.x == 0 && t + (int)gridDim.x < ntiles) issue(t + gridDim.x);
     tx_i += dq;
     ty_i += dr;
     if (ty_i >= tiles_y) {
       ty_i -= tiles_y;
       ++tx_i;
     }
-    if (++slot == SLOTS) {
-      slot = 0;
-      parity ^= 1;
-    }
+    parity ^= 1;
   }
   step_reductions<NT, R, PH_B>(A, S, e_acc, err_max, blockIdx.x, gridDim.x);
 }
