@@ -949,14 +949,14 @@ void step_shape(const ss_handle* h, int& txa, int& txb) {
 // The first shape whose tiles are all resident: wherever one fits, the cooperative step was
 // the faster.  us per step, two launches -> cooperative, by shape:
 //                    8 x 32                      16 x 32                      16 x 64
-//   FP32 chiral      320 x 320 25.1 -> 11.5      420 x 500 31.0 -> 16.9       512 x 560 30.8 -> 18.9
-//        baby        320 x 320 26.3 -> 11.7      544 x 544 32.5 -> 20.1
-//        Higgs       320 x 320 21.0 -> 11.4      420 x 500 27.2 -> 16.6       512 x 560 27.2 -> 19.6
-//        s+id        256 x 256 24.2 -> 12.1      333 x 400 29.1 -> 20.8
-//   FP64 chiral      256 x 256 30.0 -> 11.7                                   333 x 400 32.9 -> 22.2
-//        baby        256 x 256 29.3 -> 11.9      333 x 400 31.6 -> 21.5
-//        Higgs       256 x 256 25.2 -> 11.8                                   333 x 400 27.9 -> 20.3
-//        s+id        128 x 128 27.2 -> 11.4      256 x 256 28.5 -> 27.1
+//   FP32 chiral      320 x 320 25.1 -> 11.6      420 x 500 31.1 -> 16.1       512 x 560 30.8 -> 18.9
+//        baby        320 x 320 26.2 -> 11.6      544 x 544 33.9 -> 20.4
+//        Higgs       320 x 320 20.9 -> 11.4      420 x 500 27.1 -> 15.5       512 x 560 27.2 -> 19.6
+//        s+id        256 x 256 24.3 -> 12.1      333 x 400 29.1 -> 20.3
+//   FP64 chiral      256 x 256 29.4 -> 11.7                                   333 x 400 32.9 -> 20.1
+//        baby        256 x 256 29.7 -> 11.9      333 x 400 31.8 -> 21.0
+//        Higgs       256 x 256 25.1 -> 11.8                                   333 x 400 27.9 -> 20.0
+//        s+id        128 x 128 27.2 -> 11.4      256 x 256 28.1 -> 27.0
 // Of two shapes that fit the smaller tile (10.5 against 12.9 and 12.7, FP32 chiral 321 x 256).
 int coop_plan(const ss_handle* h) {
   if (h->pinned) return 0;

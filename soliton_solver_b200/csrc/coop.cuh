@@ -353,23 +353,20 @@ __device__ __forceinline__ void coop_compute(const StepArgs<R>& A, unsigned char
 }
 
 // CTAs per SM the kernel is built for: 128 registers per thread, 80 with one FP32 stencil per
-// thread; the s+id model's FP64 stencils take 255.
-template <class TH, typename R, int NT, bool SPLIT>
-__host__ __device__ constexpr int coop_min_ctas() {
-  return (sizeof(R) == 8 && TH::NF > 4 ? 256 : SPLIT && sizeof(R) == 4 && TH::NF <= 4 ? 768 : 512) / NT;
-}
-
-// The same as the kernel's residency: no more than that many CTAs, nor than fit an SM's shared memory
-// (228 KB; each CTA's arrays and 1 KB).
+// thread, 255 for the s+id model's FP64 stencils; no more than fit an SM's shared memory (228 KB; each
+// CTA's arrays and 1 KB), which leaves the larger tiles more registers: us per step, bounded by threads
+// alone -> so, FP64 chiral magnet 333 x 400 22.2 -> 20.1, baby Skyrme 21.5 -> 21.0, FP32 Higgs
+// 420 x 500 16.6 -> 15.5, chiral magnet 16.9 -> 16.1, s+id 333 x 400 20.8 -> 20.3.
 template <class TH, typename R, int TX, int TY, int NT, bool SPLIT>
 __host__ __device__ constexpr int coop_ctas() {
   const size_t per = CoopTile<TH, R, TX, TY, NT, SPLIT>::SMEM + sizeof(StageShared<NT>) + 128 + 1024;
-  const int fit = (int)(228 * 1024 / per), want = coop_min_ctas<TH, R, NT, SPLIT>();
+  const int fit = (int)(228 * 1024 / per);
+  const int want = (sizeof(R) == 8 && TH::NF > 4 ? 256 : SPLIT && sizeof(R) == 4 && TH::NF <= 4 ? 768 : 512) / NT;
   return fit < want ? fit : want;
 }
 
 template <class TH, typename R, int TX, int TY, int NT, bool SPLIT, int VW>
-__global__ void __launch_bounds__(NT, (coop_min_ctas<TH, R, NT, SPLIT>())) coop_step_kernel(
+__global__ void __launch_bounds__(NT, (coop_ctas<TH, R, TX, TY, NT, SPLIT>())) coop_step_kernel(
     const __grid_constant__ StepArgs<R> A, const __grid_constant__ CoopArgs<R> C) {
   using CT = CoopTile<TH, R, TX, TY, NT, SPLIT>;
   using V = typename PairOf<R>::type;
