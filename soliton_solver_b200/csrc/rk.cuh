@@ -590,7 +590,7 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
 // Persistent phase B (TMA staging): the resident CTAs walk the tiles b, b + gridDim.x, ...
 // through one staged tile each, so that a CTA's set-up is paid once and its SM's other CTAs
 // compute while it waits for a tile.  us, one tile per CTA -> persistent: 4096^2 chiral magnet
-// FP32 441 -> 361 (HBM floor 246; issue-bound), 2048^2 baby Skyrme FP32 118 -> 95, 1024^2
+// FP32 441 -> 361 (HBM floor 246; 46% issue, waits on loads at 16 warps per SM), 2048^2 baby Skyrme FP32 118 -> 95, 1024^2
 // Abelian Higgs FP64 79 -> 66, 1024^2 s+id FP32 64 -> 53.  A ring of two tiles under one
 // 512-thread CTA per SM took 391 us (chiral), 112 us (baby Skyrme).  Phase A gains nothing
 // (four CTAs per SM already hide its waits: 241 against 244 us) and stays one tile per CTA.
