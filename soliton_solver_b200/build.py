@@ -22,7 +22,10 @@ CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIBDIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIBDIR, "libsoliton_b200.so")
-SOURCES = ["abi.cu", "coop.cu", "batch.cu"]
+SOURCES = ["abi.cu", "coop.cu", "batch.cu", "plain.cu"]
+# --split-compile generates other code.  The FP32 step of plain rows gains by it (ten steps of 2000 x 1999,
+# chiral magnet 2864 against 3215 us, Higgs 3378 against 3606); gradients and densities lose up to 14%
+UNIT_FLAGS = {"plain.cu": ["--split-compile=0"]}
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -55,11 +58,9 @@ def build(force: bool = False, verbose: bool = False, ptxas_verbose: bool = Fals
               "-cudart", "shared", "-I", INCLUDE, "-I", CSRC]
     if ptxas_verbose:
         common += ["-Xptxas", "-v"]
-    # the translation units side by side (--split-compile would use the cores too, but its code for the
-    # gradient and density kernels is up to 10% slower)
     with tempfile.TemporaryDirectory(dir=LIBDIR) as tmp:
         objects = [os.path.join(tmp, s + ".o") for s in SOURCES]
-        cmds = [[*common, "-c", "-o", o, os.path.join(CSRC, s)] for s, o in zip(SOURCES, objects)]
+        cmds = [[*common, *UNIT_FLAGS.get(s, []), "-c", "-o", o, os.path.join(CSRC, s)] for s, o in zip(SOURCES, objects)]
         with concurrent.futures.ThreadPoolExecutor(len(cmds)) as pool:
             list(pool.map(lambda c: _run(c, verbose, ptxas_verbose), cmds))
         out = os.path.join(tmp, "lib.so")

@@ -33,6 +33,7 @@
 namespace ssb {
 SSB_COOP_INSTANCES
 SSB_BATCH_INSTANCES
+SSB_PLAIN_INSTANCES
 }
 
 using namespace ssb;

@@ -1,4 +1,4 @@
-// instances.cuh -- the kernels compiled in translation units of their own (coop.cu, batch.cu), so
+// instances.cuh -- the kernels compiled in translation units of their own (coop.cu, batch.cu, plain.cu), so
 // that the library's parts compile side by side.  SSB_INSTANCE is `extern` where they are only
 // launched (abi.cu) and empty in the unit that holds them.
 #pragma once
@@ -38,3 +38,10 @@
   SSB_BATCH_PHASES(TH, float, true, true) SSB_BATCH_PHASES(TH, double, false, true)         \
   SSB_BATCH_PHASES(TH, double, false, false)
 #define SSB_BATCH_INSTANCES SSB_FOR_THEORIES(SSB_BATCH_ALL)
+
+// the FP32 step of plain rows
+#define SSB_PLAIN(TH, PH)                                               \
+  SSB_INSTANCE template __global__ void step_kernel<TH, float, false, PH>( \
+      const __grid_constant__ StepMaps, const __grid_constant__ StepArgs<float>);
+#define SSB_PLAIN_ALL(TH) SSB_PLAIN(TH, PH_A) SSB_PLAIN(TH, PH_B) SSB_PLAIN(TH, PH_E)
+#define SSB_PLAIN_INSTANCES SSB_FOR_THEORIES(SSB_PLAIN_ALL)

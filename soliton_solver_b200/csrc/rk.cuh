@@ -77,7 +77,7 @@ struct StepShape {
   static constexpr int TY = 64, NT = 256;
   static constexpr int BYTES = (int)sizeof(R) * TH::NF;  // per site
   static constexpr bool F32 = sizeof(R) == 4;
-  static constexpr int TX = !TMA || BYTES <= (PH == PH_B ? 16 : 32) ? 16 : 8;
+  static constexpr int TX = (!TMA && !F32) || BYTES <= (PH == PH_B ? 16 : 32) ? 16 : 8;
   static constexpr int PLAIN_E = PH == PH_E && !TMA ? 1 : 0;  // FP64: one buffer and few registers
   static constexpr int CTAS = TH::NF > 4                       ? (F32 ? 2 : 1 + PLAIN_E)
                               : !F32                           ? 2 + PLAIN_E
@@ -295,8 +295,8 @@ __device__ __forceinline__ void second_half(const StepArgs<R>& A, const R* T3, c
 
 // Plain-load staging of a phase (row pitch not a multiple of 16 bytes): T1 = phi and T2 (A),
 // T1 (E) or T3 and T4 (B; an arrested step takes V = 0 and l1 for l2) into D0 and D1.  Every
-// thread issues the loads of one component plane before it combines them; the tile's own phi and
-// V also go to copy_phi and copy_vel (A, where set).  FUSED_T2: T2 rounded as in TMA-staged tiles.
+// thread issues the loads of one component plane before it combines them.  FUSED_T2: T2 rounded
+// as in TMA-staged tiles.
 template <int NF, typename R, int TX, int TY, int NT, int PH, bool FUSED_T2 = false>
 __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int x0, int y0, bool arrest) {
   using TS = TileShape<TX, TY, NT>;
@@ -304,7 +304,7 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
   const Grid& G = A.G;
   const R dt = (R)G.dt;
   long long off[KM];
-  bool ok[KM], own[PH == PH_A ? KM : 1];
+  bool ok[KM];
 #pragma unroll
   for (int k = 0; k < KM; ++k) {
     const int i = threadIdx.x + k * NT;
@@ -312,7 +312,6 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
     const int gx = x0 - 2 + r, gy = y0 - TS::YOFF + c;
     ok[k] = i < TS::PLANE && gx >= 0 && gx < G.X && gy >= 0 && gy < G.Y;
     off[k] = (long long)gx * G.Y + gy;
-    if constexpr (PH == PH_A) own[k] = ok[k] && r >= 2 && r < TX + 2 && c >= TS::YOFF && c < TS::YOFF + TY;
   }
 #pragma unroll 1
   for (int a = 0; a < NF; ++a) {
@@ -337,12 +336,6 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
         D1[a * TS::PLANE + i] = vfma(dt, vfma((R)0.5, l2, v[k]), p[k]);
       } else {
         D0[a * TS::PLANE + i] = p[k];
-        if constexpr (PH == PH_A) {
-          if (A.copy_phi && own[k]) {
-            A.copy_phi[base + off[k]] = p[k];
-            A.copy_vel[base + off[k]] = v[k];
-          }
-        }
         if constexpr (PH == PH_A)
           D1[a * TS::PLANE + i] = FUSED_T2 ? vfma(grid_k<R>(G, GK_HDT), v[k], p[k]) : stage_t2<R>(p[k], v[k], dt);
       }
@@ -367,6 +360,22 @@ __device__ __forceinline__ void copy_tile(const StepArgs<R>& A, const R* B0, int
       *reinterpret_cast<float4*>(A.copy_phi + a * A.G.N + g) = *reinterpret_cast<const float4*>(t + a * TS::PLANE);
       *reinterpret_cast<float4*>(A.copy_vel + a * A.G.N + g) =
           *reinterpret_cast<const float4*>(t + (TH::NF + a) * TS::PLANE);
+    }
+  }
+}
+
+// The same after plain staging: phi from the staged tile, V once more from global memory.
+template <class TH, typename R, int TX, int TY, int NT>
+__device__ __noinline__ void copy_tile_plain(const StepArgs<R>& A, const R* D0, int x0, int y0) {
+  using TS = TileShape<TX, TY, NT>;
+  for (int i = threadIdx.x; i < TX * TY; i += NT) {
+    const int lx = i / TY, c = i % TY, gx = x0 + lx, gy = y0 + c;
+    if (gx >= A.G.X || gy >= A.G.Y) continue;
+    const long long g = (long long)gx * A.G.Y + gy;
+#pragma unroll
+    for (int a = 0; a < TH::NF; ++a) {
+      A.copy_phi[a * A.G.N + g] = D0[a * TS::PLANE + (lx + 2) * TS::HY + TS::YOFF + c];
+      A.copy_vel[a * A.G.N + g] = A.vel[a * A.G.N + g];
     }
   }
 }
@@ -580,7 +589,10 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
     if constexpr (PH == PH_B) arrest = __ldcg(&A.st->arrest) != 0;
     stage_step_plain<NF, R, TX, TY, NT, PH>(B0, B0 + BUF, A, x0, y0, arrest);
     __syncthreads();
-    if constexpr (PH == PH_A) arrest = A.predict && __ldcg(&A.st->streak) >= 2;
+    if constexpr (PH == PH_A) {
+      if (A.copy_phi) copy_tile_plain<TH, R, TX, TY, NT>(A, B0, x0, y0);
+      arrest = A.predict && __ldcg(&A.st->streak) >= 2;
+    }
   }
   double e_acc = 0.0, err_max = -INFINITY;
   compute_tile<TH, R, TX, TY, NT, TMA, PH>(A, B0, C, x0, y0, arrest, e_acc, err_max);
