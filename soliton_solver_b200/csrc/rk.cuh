@@ -70,8 +70,8 @@ struct StepArgs {
 // Skyrme phase B, else 128 (at most 52 bytes of spills; in the batched kernels up to 188, FP64 baby
 // Skyrme's phase B); the s+id model's FP64 stencils take up to 255 and one CTA.
 // Phase B stages four halo buffers by TMA: 16 rows where two CTAs' buffers fit an SM (FP32, up to
-// four components), else 8.  Plain loads stage two (one in E), which fit at 16 rows throughout, and
-// fewer halo rows count there: every element is a load of its own.
+// four components), else 8.  Plain loads stage two (one in E), which fit at 16 rows in FP64 too, and fewer
+// halo rows count there: every element is a load of its own.
 template <class TH, typename R, int PH, bool TMA = true>
 struct StepShape {
   static constexpr int TY = 64, NT = 256;
@@ -304,7 +304,8 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
   const Grid& G = A.G;
   const R dt = (R)G.dt;
   long long off[KM];
-  bool ok[KM];
+  constexpr bool COPY = PH == PH_A && sizeof(R) == 8;  // FP64: phi and V to copy_phi and copy_vel on the way
+  bool ok[KM], own[COPY ? KM : 1];
 #pragma unroll
   for (int k = 0; k < KM; ++k) {
     const int i = threadIdx.x + k * NT;
@@ -312,6 +313,7 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
     const int gx = x0 - 2 + r, gy = y0 - TS::YOFF + c;
     ok[k] = i < TS::PLANE && gx >= 0 && gx < G.X && gy >= 0 && gy < G.Y;
     off[k] = (long long)gx * G.Y + gy;
+    if constexpr (COPY) own[k] = ok[k] && r >= 2 && r < TX + 2 && c >= TS::YOFF && c < TS::YOFF + TY;
   }
 #pragma unroll 1
   for (int a = 0; a < NF; ++a) {
@@ -336,6 +338,12 @@ __device__ inline void stage_step_plain(R* D0, R* D1, const StepArgs<R>& A, int 
         D1[a * TS::PLANE + i] = vfma(dt, vfma((R)0.5, l2, v[k]), p[k]);
       } else {
         D0[a * TS::PLANE + i] = p[k];
+        if constexpr (COPY) {
+          if (A.copy_phi && own[k]) {
+            A.copy_phi[base + off[k]] = p[k];
+            A.copy_vel[base + off[k]] = v[k];
+          }
+        }
         if constexpr (PH == PH_A)
           D1[a * TS::PLANE + i] = FUSED_T2 ? vfma(grid_k<R>(G, GK_HDT), v[k], p[k]) : stage_t2<R>(p[k], v[k], dt);
       }
@@ -364,7 +372,8 @@ __device__ __forceinline__ void copy_tile(const StepArgs<R>& A, const R* B0, int
   }
 }
 
-// The same after plain staging: phi from the staged tile, V once more from global memory.
+// The same after plain staging in FP32: phi from the staged tile, V once more from global memory (copied on
+// the way as in FP64, the staging loop of every step was 2% slower).
 template <class TH, typename R, int TX, int TY, int NT>
 __device__ __noinline__ void copy_tile_plain(const StepArgs<R>& A, const R* D0, int x0, int y0) {
   using TS = TileShape<TX, TY, NT>;
@@ -590,7 +599,9 @@ __device__ __forceinline__ void step_tile(const StepArgs<R>& A, const CUtensorMa
     stage_step_plain<NF, R, TX, TY, NT, PH>(B0, B0 + BUF, A, x0, y0, arrest);
     __syncthreads();
     if constexpr (PH == PH_A) {
-      if (A.copy_phi) copy_tile_plain<TH, R, TX, TY, NT>(A, B0, x0, y0);
+      if constexpr (sizeof(R) == 4) {
+        if (A.copy_phi) copy_tile_plain<TH, R, TX, TY, NT>(A, B0, x0, y0);
+      }
       arrest = A.predict && __ldcg(&A.st->streak) >= 2;
     }
   }
